@@ -12,9 +12,9 @@
 // C rows of one (walker, electron). Pair streams depend on r only through d_ij and are carried as
 // Taylor triples (f, df/dd, d2f/dd2); el-ion streams depend only on r_i and carry (value, three
 // gradients, Laplacian) in r_i. This form is the precision anchor of the mixed form (and the FP64
-// GPU rerun of its accuracy checks); it is not tuned for speed: the FP64 pipe of this part issues
-// at a small fraction of the FP32 rate.
-#include "net.cuh"
+// GPU rerun of its accuracy checks). The FP64 pipe of this part issues at a small fraction of the
+// FP32 rate, so the GEMMs run as exact digit products on the tensor cores (fp64_gemm.cu).
+#include "fp64_gemm.cuh"
 #include <algorithm>
 
 namespace dw {
@@ -31,97 +31,6 @@ __device__ __forceinline__ int valid_walkers(const Run64& q) {
     return q.nvalid ? min(q.B, max(0, *q.nvalid)) : q.B;
 }
 __device__ __forceinline__ double softplus_d(double x) { return fmax(x, 0.0) + log1p(exp(-fabs(x))); }
-
-// ------------------------------------------------------------------ GEMM
-// C[m, n] = sum_k A[m, k] W[k, n] (+ bias[n] on channel-0 rows, + rowbias[(walker, channel), n]),
-// A and C FP64, W the FP32 weights (converted exactly). Batched over blockIdx.z with strides sA /
-// sC (batch index = walker when rows_per_walker == 0). 64 x 64 tiles, 16-deep K slices, 256
-// threads with a 4 x 4 patch each (rows tr + 16 i, columns tc + 16 j: a warp's shared reads of
-// W are 16 consecutive doubles, those of A two broadcasts).
-struct Epi64 {
-    const float* bias = nullptr;
-    const double* rowbias = nullptr;
-    int ldrb = 0;
-    int rows_per_walker = 0;    // rows of one walker (0: batch index is the walker)
-};
-__global__ void __launch_bounds__(256)
-k64_gemm(const double* __restrict__ A, int lda, int64_t sA, const float* __restrict__ W, int ldw,
-         double* __restrict__ Cm, int ldc, int64_t sC, int M, int N, int K, Epi64 e, Run64 q) {
-    constexpr int BM = 64, BN = 64, BK = 16;
-    const int bz = blockIdx.z;
-    const int nv = valid_walkers(q);
-    const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
-    if (e.rows_per_walker == 0) {
-        if (bz >= nv) return;
-    } else if ((int64_t)m0 >= (int64_t)nv * e.rows_per_walker) {
-        return;
-    }
-    A += bz * sA;
-    Cm += bz * sC;
-    __shared__ double As[BK][BM + 1];
-    __shared__ double Ws[BK][BN];
-    const int tid = threadIdx.x, tr = tid / 16, tc = tid % 16;
-    double acc[4][4];
-    #pragma unroll
-    for (int i = 0; i < 4; ++i)
-        #pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = 0.0;
-    for (int k0 = 0; k0 < K; k0 += BK) {
-        #pragma unroll
-        for (int u = 0; u < (BM * BK) / 256; ++u) {
-            const int idx = tid + u * 256, rr = idx / BK, kk = idx % BK;
-            const int gm = m0 + rr, gk = k0 + kk;
-            As[kk][rr] = (gm < M && gk < K) ? A[(int64_t)gm * lda + gk] : 0.0;
-        }
-        #pragma unroll
-        for (int u = 0; u < (BK * BN) / 256; ++u) {
-            const int idx = tid + u * 256, kk = idx / BN, cc = idx % BN;
-            const int gk = k0 + kk, gn = n0 + cc;
-            Ws[kk][cc] = (gk < K && gn < N) ? (double)W[(int64_t)gk * ldw + gn] : 0.0;
-        }
-        __syncthreads();
-        #pragma unroll
-        for (int kk = 0; kk < BK; ++kk) {
-            double a[4], w[4];
-            #pragma unroll
-            for (int i = 0; i < 4; ++i) a[i] = As[kk][tr + 16 * i];
-            #pragma unroll
-            for (int j = 0; j < 4; ++j) w[j] = Ws[kk][tc + 16 * j];
-            #pragma unroll
-            for (int i = 0; i < 4; ++i)
-                #pragma unroll
-                for (int j = 0; j < 4; ++j) acc[i][j] = fma(a[i], w[j], acc[i][j]);
-        }
-        __syncthreads();
-    }
-    #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const int m = m0 + tr + 16 * i;
-        if (m >= M) continue;
-        const int t = m % q.C;
-        const double* rb = nullptr;
-        if (e.rowbias && e.rows_per_walker > 0)
-            rb = e.rowbias + ((int64_t)(m / e.rows_per_walker) * q.C + t) * e.ldrb;
-        #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int n = n0 + tc + 16 * j;
-            if (n >= N) continue;
-            double v = acc[i][j];
-            if (e.bias && t == 0) v += (double)e.bias[n];
-            if (rb) v += rb[n];
-            Cm[(int64_t)m * ldc + n] = v;
-        }
-    }
-}
-
-static void gemm64(const double* A, int lda, int64_t sA, const float* W, int ldw, double* C, int ldc, int64_t sC,
-                   int M, int N, int K, const Epi64& e, int batch, const Run64& q, cudaStream_t s) {
-    dim3 grid((N + 63) / 64, (M + 63) / 64, batch);
-    timer_begin("fp64_gemm", s);
-    k64_gemm<<<grid, 256, 0, s>>>(A, lda, sA, W, ldw, C, ldc, sC, M, N, K, e, q);
-    timer_end("fp64_gemm", s, 2.0 * M * N * K * batch, 0.0);
-    count_launch();
-}
 
 // ------------------------------------------------------------------ elementwise tanh over channels
 // Y = tanh(Z) for the C channel rows of each (walker, electron): value tanh(z0); gradient rows
@@ -328,9 +237,11 @@ __global__ void k64_ei_streams(const float* __restrict__ r, const float* __restr
 // conv_ee[i] = sum_j w_ij * h_map_j (ferminet_embedding.py:152-169, self-pair included) with the
 // product rule over the channels: w_ij depends on r only through d_ij (gradient u = (r_i - r_j) /
 // d_ij along r_i, -u along r_j; |grad d|^2 = 2, Lap d = 4 / d). Thread per (channel, column) of one
-// (walker, electron) block; writes columns [col0, col0 + 32) of the layer input.
-__global__ void k64_conv_ee(const float* __restrict__ r, const double* __restrict__ WPl, const double* __restrict__ HM,
-                            Run64 q, double* __restrict__ X, int ldx, int col0) {
+// (walker, electron) block; writes columns [col0, col0 + 32) of the layer input. Columns [col0 + 32,
+// col0 + 32 + eiw) take conv_ei of the level: value, electron i's own gradient rows and the
+// Laplacian, zero elsewhere.
+__global__ void k64_conv(const float* __restrict__ r, const double* __restrict__ WPl, const double* __restrict__ HM,
+                         const double* __restrict__ CEl, int eiw, Run64 q, double* __restrict__ X, int ldx, int col0) {
     const Dims& d = q.d;
     const int i = blockIdx.x % d.n;
     const int64_t b = blockIdx.x / d.n;
@@ -380,46 +291,15 @@ __global__ void k64_conv_ee(const float* __restrict__ r, const double* __restric
         }
         X[(((b * n + i) * C) + t) * (int64_t)ldx + col0 + col] = v;
     }
-}
-
-// conv_ei of one level expanded to the channels: value, electron i's own gradient rows and the
-// Laplacian; zero elsewhere. Columns [col0, col0 + width).
-__global__ void k64_conv_ei(const double* __restrict__ CEl, Run64 q, int width, double* __restrict__ X, int ldx,
-                            int col0) {
-    const Dims& d = q.d;
-    const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const int col = (int)(idx % width);
-    const int64_t row = idx / width;
-    const int t = (int)(row % q.C);
-    const int64_t be = row / q.C;
-    const int i = (int)(be % d.n);
-    const int64_t b = be / d.n;
-    if (b >= valid_walkers(q)) return;
-    const double* ce = CEl + be * 5 * 32 + col;
-    double v = 0.0;
-    if (t == 0) v = ce[0];
-    else if (t == q.C - 1) v = ce[4 * 32];
-    else if ((t - 1) / 3 == i) v = ce[(1 + (t - 1) % 3) * 32];
-    X[row * ldx + col0 + col] = v;
-}
-
-// Spin means of the h columns per (walker, channel): M[(b, t)] = [mean over up electrons,
-// mean over down electrons] (SymmetricFeatures, ferminet_embedding.py:52-94).
-__global__ void k64_spin_means(const double* __restrict__ X, int ldx, int hw, Run64 q, double* __restrict__ M) {
-    const Dims& d = q.d;
-    const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const int col = (int)(idx % hw);
-    const int64_t bt = idx / hw;
-    const int t = (int)(bt % q.C);
-    const int64_t b = bt / q.C;
-    if (b >= valid_walkers(q)) return;
-    double su = 0.0, sd = 0.0;
-    for (int i = 0; i < d.n; ++i) {
-        const double x = X[((b * d.n + i) * q.C + t) * (int64_t)ldx + col];
-        if (i < d.nu) su += x; else sd += x;
+    const double* ce = CEl + (b * n + i) * 5 * 32;
+    for (int e = threadIdx.x; e < C * eiw; e += blockDim.x) {
+        const int t = e / eiw, col = e % eiw;
+        double v = 0.0;
+        if (t == 0) v = ce[col];
+        else if (t == C - 1) v = ce[4 * 32 + col];
+        else if ((t - 1) / 3 == i) v = ce[(1 + (t - 1) % 3) * 32 + col];
+        X[(((b * n + i) * C) + t) * (int64_t)ldx + col0 + 32 + col] = v;
     }
-    M[bt * 2 * hw + col] = su / d.nu;
-    M[bt * 2 * hw + hw + col] = sd / d.nd;
 }
 
 // ------------------------------------------------------------------ envelope orbitals
@@ -626,11 +506,14 @@ struct Plan64 {
     int Bc, C;
     double* him;
     double *XA, *XB, *Zt, *HM, *M, *WB, *WP, *CE, *BF, *MO, *logdet, *sign, *Ainv, *g, *lapdet, *J1, *J2, *jas;
+    Digits act, mean;              // digit planes of the activation rows and of the spin-mean rows
+    Weight64 w[kMaxW64];           // h_map[4], mean rows[4], main rows[4], backflow[2], Jastrow[2] (w.w set per call)
     size_t bytes;
 };
 static const int kXW64 = 320;    // layer 1..3 input [h (256) | conv_ee (32) | conv_ei (32)]
 
-static Plan64 carve64(const Dims& d, int C, int Bc, void* ws) {
+// Buffers of a chunk of Bc walkers; without `digits` only those that the chunk size is chosen by.
+static Plan64 carve64(const Dims& d, int C, int Bc, void* ws, bool digits = true) {
     Carver c(ws, (size_t)-1);
     Plan64 p;
     p.Bc = Bc; p.C = C;
@@ -659,29 +542,44 @@ static Plan64 carve64(const Dims& d, int C, int Bc, void* ws) {
     p.J1 = c.take<double>(rows * d.J0);
     p.J2 = c.take<double>(rows * d.J1);
     p.jas = c.take<double>((int64_t)Bc * C);
+    if (digits) {
+        auto take = [&](int64_t r, int K) {
+            const int Kp = pad_k64(K);
+            __nv_bfloat16* dig = c.take<__nv_bfloat16>((size_t)kDig * r * Kp);
+            return Digits{dig, c.take<int>(r), r, Kp};
+        };
+        p.act = take(rows, std::max(kXW64, w0));
+        p.mean = take((int64_t)Bc * C, 2 * std::max(d.D, d.hw[0]));
+        const int J[2] = {d.J0, d.J1}, JK[2] = {d.D, d.J0};
+        for (int k = 0; k < kMaxW64; ++k) {
+            const int l = k % 4;
+            const int K = k < 4 ? d.hw[l] : k < 8 ? 2 * d.hw[l] : k < 12 ? d.hw[l] + d.E + d.eiw[l] : k < 14 ? d.D : JK[k - 14];
+            const int N = k < 4 ? d.E : k < 12 ? d.D : k < 14 ? d.KN : J[k - 14];
+            p.w[k] = Weight64{nullptr, N, K, N, take(N, K)};
+        }
+    }
     p.bytes = c.used;
     return p;
 }
 
-static const size_t kChunkBudget64 = (size_t)6 << 30;
+static const size_t kChunkBudget64 = (size_t)6 << 30;    // without the digit planes (about half as much again)
 
 static int choose_chunk64(const Dims& d, int C, int B, size_t budget) {
-    const size_t one = carve64(d, C, 1, nullptr).bytes, two = carve64(d, C, 2, nullptr).bytes;
+    const size_t one = carve64(d, C, 1, nullptr, false).bytes, two = carve64(d, C, 2, nullptr, false).bytes;
     const size_t per = std::max<size_t>(two > one ? two - one : one, 1);
     const size_t fixed = one > per ? one - per : 0;
     const size_t avail = budget > fixed ? budget - fixed : per;
-    // batched GEMMs put the walker on grid.z (at most 65535)
     int bc = std::min((int)std::min<size_t>(std::max<size_t>(1, avail / per), 32768), B);
-    while (bc > 1 && carve64(d, C, bc, nullptr).bytes > budget) bc -= std::max(1, bc / 32);
+    while (bc > 1 && carve64(d, C, bc, nullptr, false).bytes > budget) bc -= std::max(1, bc / 32);
     return bc;
 }
 
 static inline unsigned blocks_for(int64_t n, int tpb) { return (unsigned)((n + tpb - 1) / tpb); }
 
 // The FP64 forward (value or tangent) of one chunk of walkers.
-static int run_chunk64(const Plan64& p, const Dims& d0, int Bc, const float* P, const ParamLayout& L, const float* main_w[4],
-                       const float* mean_w[4], const float* r, const float* R, const int32_t* Z, const int32_t* seg,
-                       const int* nvalid, float* lp, float* phase, float* E, float* grad, cudaStream_t s) {
+static int run_chunk64(const Plan64& p, const Dims& d0, int Bc, const float* P, const ParamLayout& L, const float* r,
+                       const float* R, const int32_t* Z, const int32_t* seg, const int* nvalid, float* lp, float* phase,
+                       float* E, float* grad, cudaStream_t s) {
     Dims d = d0;
     d.seg = seg;
     Run64 q;
@@ -690,6 +588,11 @@ static int run_chunk64(const Plan64& p, const Dims& d0, int Bc, const float* P, 
     const int64_t rows = (int64_t)Bc * n * C;
     const bool tang = C > 1;
     const int w0 = d.hw[0] + d.E + d.eiw[0];
+    const Rows64 all = plain_rows(Bc, n * C, nvalid), chan = plain_rows(Bc, C, nvalid);
+    // digit planes of the first K columns, reusing the plan's buffer at that width
+    auto planes = [](Digits x, int K) { x.Kp = pad_k64(K); return x; };
+    auto gemm = [&](const double* A, int lda, const Digits& da, const Weight64& w, double* Cm, int ldc, const Rows64& rr,
+                    const Epi64& e) { return gemm64_tc(A, lda, da, w, Cm, ldc, rr, C, e, s); };
     // layer-0 input [features | conv_ee | conv_ei] in XB (free until layer 1 writes it)
     timer_begin("fp64_streams", s);
     k64_features<<<blocks_for(rows * d.N, 256), 256, 0, s>>>(r, R, Z, q, p.XB, w0);
@@ -705,38 +608,46 @@ static int run_chunk64(const Plan64& p, const Dims& d0, int Bc, const float* P, 
         double* xout = (l % 2 == 0) ? p.XA : p.XB;
         const int hw = d.hw[l];
         // h_map = tanh(h W + b) -> HM
-        Epi64 em; em.bias = P + L.h_map_b[l]; em.rows_per_walker = n * C;
-        gemm64(xin, ldin, 0, P + L.h_map_w[l], d.E, p.Zt, d.E, 0, (int)rows, d.E, hw, em, 1, q, s);
+        Epi64 em; em.bias = P + L.h_map_b[l];
+        const Digits dh = planes(p.act, hw);
+        slice_rows64(xin, ldin, hw, all, dh, s);
+        DW_CHECK(gemm(xin, ldin, dh, p.w[l], p.Zt, d.E, all, em));
         jet_tanh(p.Zt, d.E, d.E, q, p.HM, 32, s);
         // convolutions into columns [hw, hw + E + eiw)
         timer_begin("fp64_conv", s);
-        k64_conv_ee<<<(unsigned)((int64_t)Bc * n), 128, 0, s>>>(r, p.WP + (int64_t)l * Bc * n * n * 96, p.HM, q, xin,
-                                                                 ldin, hw);
+        k64_conv<<<(unsigned)((int64_t)Bc * n), 128, 0, s>>>(r, p.WP + (int64_t)l * Bc * n * n * 96, p.HM,
+                                                              p.CE + (int64_t)l * Bc * n * 5 * 32, d.eiw[l], q, xin, ldin,
+                                                              hw);
         timer_end("fp64_conv", s, 0.0, 0.0);
         count_launch();
-        k64_conv_ei<<<blocks_for(rows * d.eiw[l], 256), 256, 0, s>>>(p.CE + (int64_t)l * Bc * n * 5 * 32, q, d.eiw[l],
-                                                                      xin, ldin, hw + d.E);
-        count_launch();
         // spin means and their per-(walker, channel) product with the mean rows (+ the layer bias)
-        k64_spin_means<<<blocks_for((int64_t)Bc * C * hw, 256), 256, 0, s>>>(xin, ldin, hw, q, p.M);
-        count_launch();
-        Epi64 eb; eb.bias = P + L.h_el_b[l]; eb.rows_per_walker = C;
-        gemm64(p.M, 2 * hw, 0, mean_w[l], d.D, p.WB, d.D, 0, Bc * C, d.D, 2 * hw, eb, 1, q, s);
+        const Digits dm = planes(p.mean, 2 * hw);
+        spin_means64(xin, ldin, hw, n, d.nu, C, chan, p.M, dm, s);
+        Epi64 eb; eb.bias = P + L.h_el_b[l];
+        DW_CHECK(gemm(p.M, 2 * hw, dm, p.w[4 + l], p.WB, d.D, chan, eb));
         // h_el = tanh([h | conv_ee | conv_ei] W_main + mean term) (ferminet_embedding.py:233-241)
-        Epi64 e3; e3.rowbias = p.WB; e3.ldrb = d.D; e3.rows_per_walker = n * C;
-        gemm64(xin, ldin, 0, main_w[l], d.D, p.Zt, d.D, 0, (int)rows, d.D, hw + d.E + d.eiw[l], e3, 1, q, s);
+        Epi64 e3; e3.rowbias = p.WB; e3.ldrb = d.D;
+        const Digits dx = planes(p.act, p.w[8 + l].K);
+        slice_rows64(xin, ldin, p.w[8 + l].K, all, dx, s);
+        DW_CHECK(gemm(xin, ldin, dx, p.w[8 + l], p.Zt, d.D, all, e3));
         jet_tanh(p.Zt, d.D, d.D, q, xout, kXW64, s);
         xin = xout;
         ldin = kXW64;
     }
     const double* H = xin;
-    // backflow per spin (envelope_orbitals.py:46-75): the electrons of one spin are nu * C
-    // consecutive rows of each walker
+    // The final embedding's digit rows ordered by spin, then walker: backflow of each spin's rows
+    // (envelope_orbitals.py:46-75), and the Jastrow layer over both groups.
+    Rows64 spins = all;
+    spins.ngroups = 2;
+    spins.g[0] = RowGroup{0, d.nu * C, (int64_t)n * C, 0};
+    spins.g[1] = RowGroup{(int64_t)Bc * d.nu * C, d.nd * C, (int64_t)n * C, (int64_t)d.nu * C};
+    const Digits dH = planes(p.act, d.D);
+    slice_rows64(H, kXW64, d.D, spins, dH, s);
     for (int spin = 0; spin < 2; ++spin) {
-        const int i0 = spin == 0 ? 0 : d.nu, ns = spin == 0 ? d.nu : d.nd;
-        Epi64 e0;
-        gemm64(H + (int64_t)i0 * C * kXW64, kXW64, (int64_t)n * C * kXW64, P + (spin == 0 ? L.bf_up : L.bf_dn), d.KN,
-               p.BF + (int64_t)i0 * C * d.KN, d.KN, (int64_t)n * C * d.KN, ns * C, d.KN, d.D, e0, Bc, q, s);
+        Rows64 one = spins;
+        one.ngroups = 1;
+        one.g[0] = spins.g[spin];
+        DW_CHECK(gemm(H, kXW64, dH, p.w[12 + spin], p.BF, d.KN, one, Epi64()));
     }
     timer_begin("fp64_envelope", s);
     k64_envelope_mo<<<blocks_for((int64_t)Bc * d.K * n * n, 128), 128, 0, s>>>(r, R, Z, P, L, q, p.BF, d.KN, p.MO);
@@ -758,11 +669,13 @@ static int run_chunk64(const Plan64& p, const Dims& d0, int Bc, const float* P, 
         count_launch();
     }
     // Jastrow MLP([64, 64, 1]) on the final embedding (wavefunction.py:42-60)
-    Epi64 j0; j0.bias = P + L.jas_b[0]; j0.rows_per_walker = n * C;
-    gemm64(H, kXW64, 0, P + L.jas_w[0], d.J0, p.Zt, d.J0, 0, (int)rows, d.J0, d.D, j0, 1, q, s);
+    Epi64 j0; j0.bias = P + L.jas_b[0];
+    DW_CHECK(gemm(H, kXW64, dH, p.w[14], p.Zt, d.J0, spins, j0));
     jet_tanh(p.Zt, d.J0, d.J0, q, p.J1, d.J0, s);
-    Epi64 j1; j1.bias = P + L.jas_b[1]; j1.rows_per_walker = n * C;
-    gemm64(p.J1, d.J0, 0, P + L.jas_w[1], d.J1, p.Zt, d.J1, 0, (int)rows, d.J1, d.J0, j1, 1, q, s);
+    Epi64 j1; j1.bias = P + L.jas_b[1];
+    const Digits dj = planes(p.act, d.J0);
+    slice_rows64(p.J1, d.J0, d.J0, all, dj, s);
+    DW_CHECK(gemm(p.J1, d.J0, dj, p.w[15], p.Zt, d.J1, all, j1));
     jet_tanh(p.Zt, d.J1, d.J1, q, p.J2, d.J1, s);
     k64_jastrow_out<<<blocks_for((int64_t)Bc * C * 32, 256), 256, 0, s>>>(p.J2, d.J1, P + L.jas_w[2], q, p.jas);
     count_launch();
@@ -835,12 +748,22 @@ int fp64_forward_all(const DwArch* a, const float* P, const void* prepared, cons
     if (nvalid && bc < B) return DW_ERR_ARG;       // a device-side walker count needs one chunk
     Plan64 p = carve64(d, C, bc, ws);
     if (p.bytes > ws_bytes) return DW_ERR_WORKSPACE;
+    for (int l = 0; l < 4; ++l) {
+        p.w[l].w = P + L.h_map_w[l];
+        p.w[4 + l].w = mean_w[l];
+        p.w[8 + l].w = main_w[l];
+    }
+    p.w[12].w = P + L.bf_up;
+    p.w[13].w = P + L.bf_dn;
+    p.w[14].w = P + L.jas_w[0];
+    p.w[15].w = P + L.jas_w[1];
+    slice_weights64(p.w, kMaxW64, nvalid, s);
     const int total = nseg * 4 * d.N * 32;
     k64_ion_maps<<<(total + 255) / 256, 256, 0, s>>>(P, L, d, Z, p.him);
     count_launch();
     for (int b0 = 0; b0 < B; b0 += bc) {
         const int nb = std::min(bc, B - b0);
-        DW_CHECK(run_chunk64(p, d, nb, P, L, main_w, mean_w, r + (int64_t)b0 * d.n * 3, R, Z, seg ? seg + b0 : nullptr,
+        DW_CHECK(run_chunk64(p, d, nb, P, L, r + (int64_t)b0 * d.n * 3, R, Z, seg ? seg + b0 : nullptr,
                              nvalid, lp + b0, phase ? phase + b0 : nullptr, E ? E + b0 : nullptr,
                              grad ? grad + (int64_t)b0 * 3 * d.n : nullptr, s));
     }

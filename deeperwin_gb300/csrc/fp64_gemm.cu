@@ -1,0 +1,514 @@
+// FP64 matrix product on the BF16 tensor cores, by splitting both operands into small integers
+// (K. Ozaki, T. Ogita, S. Oishi, S. Rump, "Error-free transformations of matrix multiplication by
+// using fast routines of matrix multiplication and its applications", Numer. Algorithms 59, 2012; on
+// tensor cores: D. Mukunoki et al., "DGEMM using tensor cores, and its accurate and reproducible
+// versions", ISC 2020).
+//
+// Each row of A and each column of W is scaled by a power of two so that its largest magnitude is
+// below one, rounded to 62 fractional bits and written as nine signed 7-bit digits,
+//   a = 2^Ea sum_i d_i 2^(-6 - 7 i),  d_0 in [-64, 64], d_i in [-64, 63].
+// A digit is exact in BF16, a product of two digits is below 2^12, and the sum of the up to nine
+// products with i + j = s over K <= 512 columns stays below 2^24 (for s = 8 and K = 512 the bound is
+// 2^24.2, reached only if every digit were extreme; a rounding there is 2^-56 of the last digit), so
+// the FP32 accumulators in TMEM hold every digit sum exactly, in any order. The 45 products with
+// i + j <= 8 give the result to about 2^-61 sqrt(K) max|a| max|w|, below the rounding error of an
+// FP64 sum; the nine sums are combined in integers and rounded to FP64 once. FP32 weights are
+// represented exactly down to 2^-38 of their column's maximum.
+//
+// Why: FP64 issues at about two lanes per clock and SM here (1.2 TFLOP/s), the BF16 tensor cores at
+// about 1500 times that, so even 45 products per multiplication are far cheaper: the 16 GEMMs of a
+// C2H4-shaped local energy (16 electrons, 32 determinants, 64 walkers) took 46.0 ms on the FP64 pipe
+// (64 x 64 tiles, 0.97 TFLOP/s) and take 4.6 ms here; a single tile of the FP64 loop took longer than
+// the smallest launch of this kernel, so no size keeps it.
+//
+// Rows and columns whose scale is not an ordinary one (infinities, NaN, below 2^-922) are computed
+// from the original FP64 values in the epilogue.
+#include "fp64_gemm.cuh"
+#include "gemm_tc.cuh"
+#include <algorithm>
+
+namespace dw {
+
+namespace {
+
+constexpr int BM = 128, BN = 48, BK = 32;            // rows, columns, K-columns of a pipeline stage
+constexpr int kStages = 2;
+constexpr int kEpi = 8;                              // epilogue warps: two per TMEM lane quarter
+constexpr int kThreads64 = 64 + 32 * kEpi;
+constexpr int kABytes = BM * BK * 2, kBBytes = BN * BK * 2;      // one digit plane of a stage
+constexpr int kStageBytes = kDig * (kABytes + kBBytes);          // 101,376
+constexpr int kSmem64 = 1024 + kStages * kStageBytes + 256;
+constexpr int kFlagged = 0x7fffffff;                 // exponent of a row that the digits do not represent
+
+__device__ __forceinline__ int valid_of(const Rows64& r) { return r.nvalid ? min(r.B, max(0, *r.nvalid)) : r.B; }
+
+// Biased exponent field of x.
+__device__ __forceinline__ int exp_field(double x) { return (__double2hiint(x) >> 20) & 0x7ff; }
+// Exponent of a row from the largest exponent field: values are below 2^E.
+__device__ __forceinline__ int row_exponent(int emax) {
+    if (emax == 0) return 0;                          // zeros (and subnormals, see below)
+    return emax == 0x7ff || emax < 100 ? kFlagged : emax - 1022;
+}
+// x 2^(62 - E) rounded to an integer (E = emax - 1022), |result| <= 2^62.
+__device__ __forceinline__ long long to_fixed(double x, int emax) {
+    const long long bits = __double_as_longlong(x);
+    const int e = (int)(bits >> 52) & 0x7ff;
+    unsigned long long m = (bits & 0xfffffffffffffll) | (1ll << 52);
+    const int sh = emax - e - 9;                      // right shift of the 53-bit significand
+    if (e == 0 || sh > 54) return 0;
+    m = sh <= 0 ? m << -sh : (m + (1ull << (sh - 1))) >> sh;
+    return bits < 0 ? -(long long)m : (long long)m;
+}
+// Next digit from the low end: d in [-64, 63], x <- (x - d) / 128.
+__device__ __forceinline__ int low_digit(long long& x) {
+    const int d = (((int)x & 127) ^ 64) - 64;
+    x = (x - d) >> 7;
+    return d;
+}
+__device__ __forceinline__ uint32_t pack_digits(int a, int b) {
+    const __nv_bfloat162 h = __floats2bfloat162_rn((float)a, (float)b);
+    return *reinterpret_cast<const uint32_t*>(&h);
+}
+
+// One row held by a warp (columns 64 u + 2 lane, + 1): common exponent and digit planes.
+__device__ __forceinline__ void slice_row(const double2 (&x)[kMaxK64 / 64], int emax, bool nonzero, int64_t m,
+                                          const Digits& d) {
+    const int lane = threadIdx.x & 31, Kp = d.Kp;
+    emax = __reduce_max_sync(0xffffffffu, emax);
+    int E = row_exponent(emax);
+    if (emax == 0 && __any_sync(0xffffffffu, nonzero)) E = kFlagged;    // only subnormals
+    if (lane == 0) d.ex[m] = E;
+    __nv_bfloat16* o = d.dig + m * Kp;
+    const int64_t plane = d.rows * Kp;
+    #pragma unroll
+    for (int u = 0; u < kMaxK64 / 64; ++u) {
+        const int c = u * 64 + 2 * lane;
+        if (c >= Kp) continue;
+        long long f0 = 0, f1 = 0;
+        if (E != kFlagged) { f0 = to_fixed(x[u].x, emax); f1 = to_fixed(x[u].y, emax); }
+        #pragma unroll
+        for (int i = kDig - 1; i >= 0; --i) {
+            const int d0 = i ? low_digit(f0) : (int)f0, d1 = i ? low_digit(f1) : (int)f1;
+            *reinterpret_cast<uint32_t*>(o + i * plane + c) = pack_digits(d0, d1);
+        }
+    }
+}
+
+// Warp per row: the largest exponent, then the digits of two neighbouring columns per lane and step.
+// HBM-bound: 8 K bytes read, 18 Kp written per row.
+__global__ void __launch_bounds__(256)
+k64_slice_rows(const double* __restrict__ A, int lda, int K, Rows64 rows, Digits d) {
+    const int nv = valid_of(rows), lane = threadIdx.x & 31;
+    const int64_t w = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const int gi = rows.ngroups > 1 && w >= (int64_t)rows.B * rows.g[0].rpw ? 1 : 0;
+    const RowGroup& g = rows.g[gi];
+    const int64_t k = gi ? w - (int64_t)rows.B * rows.g[0].rpw : w;    // row within the group
+    const int64_t b = k / g.rpw;
+    if (b >= nv) return;
+    const int64_t m = g.base + k;
+    const double* src = A + (b * g.out_rpw + g.out_off + k % g.rpw) * lda;
+    double2 x[kMaxK64 / 64];
+    int emax = 0;
+    bool sub = false;
+    #pragma unroll
+    for (int u = 0; u < kMaxK64 / 64; ++u) {
+        const int c = u * 64 + 2 * lane;
+        x[u] = make_double2(0.0, 0.0);
+        if (c < K) x[u].x = src[c];
+        if (c + 1 < K) x[u].y = src[c + 1];
+        emax = max(emax, max(exp_field(x[u].x), exp_field(x[u].y)));
+        sub |= x[u].x != 0.0 || x[u].y != 0.0;
+    }
+    slice_row(x, emax, sub, m, d);
+}
+
+// Spin means of the hw columns of X per (walker, channel), M[(b, t)] = [mean over up electrons, mean
+// over down electrons] (SymmetricFeatures, ferminet_embedding.py:52-94), and their digit planes; warp
+// per row of M.
+__global__ void __launch_bounds__(256)
+k64_spin_means(const double* __restrict__ X, int ldx, int hw, int n, int nu, int C, Rows64 rows, double* __restrict__ M,
+               Digits d) {
+    const int64_t bt = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const int64_t b = bt / C;
+    if (b >= valid_of(rows)) return;
+    const int t = (int)(bt % C), lane = threadIdx.x & 31;
+    double2 x[kMaxK64 / 64];
+    int emax = 0;
+    bool sub = false;
+    #pragma unroll
+    for (int u = 0; u < kMaxK64 / 64; ++u) {
+        double v[2] = {0.0, 0.0};
+        #pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            const int c = u * 64 + 2 * lane + k;
+            if (c >= 2 * hw) continue;
+            const int i0 = c < hw ? 0 : nu, i1 = c < hw ? nu : n, col = c < hw ? c : c - hw;
+            double acc = 0.0;
+            for (int i = i0; i < i1; ++i) acc += X[((b * n + i) * C + t) * (int64_t)ldx + col];
+            v[k] = acc / (i1 - i0);
+            M[bt * 2 * hw + c] = v[k];
+            emax = max(emax, exp_field(v[k]));
+            sub |= v[k] != 0.0;
+        }
+        x[u] = make_double2(v[0], v[1]);
+    }
+    slice_row(x, emax, sub, bt, d);
+}
+
+struct WeightTable {
+    Weight64 w[kMaxW64];
+    int first[kMaxW64 + 1];                           // first block of each matrix (32 columns per block)
+    int count;
+    const int* nvalid;
+};
+
+// Block per 32 columns of a weight matrix: column exponents, then digits by 64-row tiles transposed
+// through shared memory so that a warp writes consecutive K.
+__global__ void __launch_bounds__(256) k64_slice_weights(WeightTable t) {
+    if (t.nvalid && *t.nvalid <= 0) return;
+    int mi = 0;
+    while (mi + 1 < t.count && (int)blockIdx.x >= t.first[mi + 1]) ++mi;
+    const Weight64& w = t.w[mi];
+    const int n0 = ((int)blockIdx.x - t.first[mi]) * 32, tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+    __shared__ float tile[64][33];
+    __shared__ int emax_s[8][32], sub_s[8][32];
+    int emax = 0, sub = 0;
+    if (n0 + tx < w.N)
+        for (int k = ty; k < w.K; k += 8) {
+            const float x = w.w[(int64_t)k * w.ldw + n0 + tx];
+            emax = max(emax, exp_field((double)x));
+            sub |= x != 0.f;
+        }
+    emax_s[ty][tx] = emax;
+    sub_s[ty][tx] = sub;
+    __syncthreads();
+    if (ty == 0) {
+        for (int k = 1; k < 8; ++k) { emax = max(emax, emax_s[k][tx]); sub |= sub_s[k][tx]; }
+        emax_s[0][tx] = emax;
+        if (n0 + tx < w.N) w.d.ex[n0 + tx] = emax == 0 && sub ? kFlagged : row_exponent(emax);
+    }
+    const int64_t plane = w.d.rows * w.d.Kp;
+    for (int k0 = 0; k0 < w.d.Kp; k0 += 64) {
+        __syncthreads();
+        for (int k = ty; k < 64; k += 8)
+            tile[k][tx] = k0 + k < w.K && n0 + tx < w.N ? w.w[(int64_t)(k0 + k) * w.ldw + n0 + tx] : 0.f;
+        __syncthreads();
+        const int k = k0 + 2 * tx;
+        for (int n = ty; n < 32; n += 8) {
+            if (n0 + n >= w.N || k >= w.d.Kp) continue;
+            const int em = emax_s[0][n];
+            const bool ok = row_exponent(em) != kFlagged;
+            long long f0 = ok ? to_fixed((double)tile[2 * tx][n], em) : 0, f1 = ok ? to_fixed((double)tile[2 * tx + 1][n], em) : 0;
+            __nv_bfloat16* o = w.d.dig + (int64_t)(n0 + n) * w.d.Kp + k;
+            #pragma unroll
+            for (int i = kDig - 1; i >= 0; --i) {
+                const int d0 = i ? low_digit(f0) : (int)f0, d1 = i ? low_digit(f1) : (int)f1;
+                *reinterpret_cast<uint32_t*>(o + i * plane) = pack_digits(d0, d1);
+            }
+        }
+    }
+}
+
+struct Args64 {
+    const double* A; int lda;
+    const float* W; int ldw;
+    double* C; int ldc;
+    const int* ea; const int* ew;
+    Rows64 rows;
+    Epi64 e;
+    int N, K, channels, ntn;
+    int* error;                    // set when a bounded wait ran out
+};
+
+__device__ __forceinline__ void tmem_ld8(uint32_t taddr, float* v) {
+    uint32_t r[8];
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+                 : "r"(taddr));
+    #pragma unroll
+    for (int j = 0; j < 8; ++j) v[j] = __uint_as_float(r[j]);
+}
+
+// 2^scale sum_s acc_s 2^(56 - 7 s), rounded to the nearest double. |sum| < 2^79.
+__device__ __forceinline__ double combine_digits(const float* acc, int stride, int scale) {
+    long long hi = 0, lo = 0;
+    #pragma unroll
+    for (int s = 0; s < 4; ++s) hi = (hi << 7) + (long long)(int)acc[s * stride];
+    #pragma unroll
+    for (int s = 4; s < kDig; ++s) lo = (lo << 7) + (long long)(int)acc[s * stride];
+    hi += lo >> 35;                                   // value = hi 2^35 + lo, 0 <= lo < 2^35
+    lo &= (1ll << 35) - 1;
+    const bool neg = hi < 0;
+    if (neg) {
+        hi = -hi;
+        if (lo) { hi -= 1; lo = (1ll << 35) - lo; }
+    }
+    // significand with its top bit at 63, value = m 2^(e - 63)
+    unsigned long long m;
+    int e;
+    if (hi == 0) {
+        if (lo == 0) return 0.0;
+        const int z = __clzll(lo);
+        m = (unsigned long long)lo << z;
+        e = 63 - z;
+    } else {
+        const int z = __clzll(hi);                    // hi < 2^45: z >= 19
+        m = (unsigned long long)hi << z;
+        m |= z >= 35 ? (unsigned long long)lo << (z - 35) : (unsigned long long)lo >> (35 - z);
+        e = 98 - z;
+    }
+    unsigned long long q = m >> 11;                   // 53 bits, round to nearest even
+    const unsigned rem = (unsigned)m & 0x7ffu;
+    q += rem > 0x400u || (rem == 0x400u && (q & 1u));
+    q += (unsigned long long)(e + scale + 1022) << 52;
+    return __longlong_as_double((long long)(q | (neg ? 1ull << 63 : 0ull)));
+}
+
+// Persistent: one CTA per SM loops over 128 x 48 output tiles. Warp 0 loads the nine digit planes of
+// 32 K-columns of both operands per stage (two TMA copies, 101 KB, two stages), warp 1 issues the 90
+// MMAs of a stage into nine TMEM accumulators (432 columns), eight warps combine and store them. Bound
+// by the MMAs' shared-memory reads of A (N = 48: 32 clocks of reads for 24 of products); nine
+// accumulators leave no room for a second set, so the epilogue (about a fifth) is not overlapped.
+__global__ void __launch_bounds__(kThreads64, 1)
+k64_gemm_tc(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, Args64 a) {
+    const int nv = valid_of(a.rows);
+    int64_t tiles_of[2] = {0, 0};
+    for (int g = 0; g < a.rows.ngroups; ++g) tiles_of[g] = ((int64_t)nv * a.rows.g[g].rpw + BM - 1) / BM * a.ntn;
+    const int64_t n_tiles = tiles_of[0] + tiles_of[1];
+    if ((int64_t)blockIdx.x >= n_tiles) return;       // before any barrier or TMEM allocation
+    extern __shared__ __align__(1024) uint8_t smem_raw[];
+    uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+    uint64_t* full = reinterpret_cast<uint64_t*>(smem + kStages * kStageBytes);
+    uint64_t* empty = full + kStages;
+    uint64_t* tfull = empty + kStages;
+    uint64_t* tempty = tfull + 1;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tempty + 1);
+    __shared__ int s_err, s_epi_err;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int nk = (a.K + BK - 1) / BK;
+    if (threadIdx.x == 0) {
+        s_err = 0;
+        s_epi_err = 0;
+        for (int s = 0; s < kStages; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
+        mbar_init(tfull, 1);
+        mbar_init(tempty, kEpi);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        fence_async_smem();
+    }
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_u32(tmem_slot)) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = *tmem_slot;
+    // tile -> row group, first row within the group, first column
+    auto locate = [&](int64_t tile, int& g, int64_t& k0, int& n0) {
+        g = tile >= tiles_of[0] ? 1 : 0;
+        const int64_t u = g ? tile - tiles_of[0] : tile;
+        k0 = u / a.ntn * BM;
+        n0 = (int)(u % a.ntn) * BN;
+    };
+
+    if (warp == 0) {
+        if (lane == 0) {
+            uint32_t cnt = 0, issued[kStages] = {0, 0};
+            bool err = false;
+            for (int64_t tile = blockIdx.x; tile < n_tiles && !err; tile += gridDim.x) {
+                int g, n0;
+                int64_t k0;
+                locate(tile, g, k0, n0);
+                const int row = (int)(a.rows.g[g].base + k0);
+                for (int kt = 0; kt < nk; ++kt, ++cnt) {
+                    const int s = cnt % kStages;
+                    const uint32_t use = cnt / kStages;
+                    if (use > 0 && !mbar_wait(&empty[s], (use - 1) & 1)) { err = true; break; }
+                    mbar_expect_tx(&full[s], kStageBytes);
+                    uint8_t* st = smem + s * kStageBytes;
+                    tma_load_3d(st, &tmA, &full[s], kt * BK, row, 0);
+                    tma_load_3d(st + kDig * kABytes, &tmB, &full[s], kt * BK, n0, 0);
+                    issued[s] = use + 1;
+                }
+            }
+            if (err) {
+                atomicExch(&s_err, 1);
+                for (int s = 0; s < kStages; ++s)
+                    if (issued[s]) mbar_wait(&full[s], (issued[s] - 1) & 1);
+            }
+        }
+    } else if (warp == 1) {
+        if (lane == 0) {
+            const uint32_t idesc = idesc_bf16(BN);
+            uint32_t cnt = 0, it = 0;
+            bool err = false;
+            for (int64_t tile = blockIdx.x; tile < n_tiles && !err; tile += gridDim.x, ++it) {
+                if (!mbar_wait(tempty, (it & 1) ^ 1)) { err = true; break; }
+                tc_fence_after();
+                for (int kt = 0; kt < nk; ++kt, ++cnt) {
+                    const int s = cnt % kStages;
+                    if (!mbar_wait(&full[s], (cnt / kStages) & 1)) { err = true; break; }
+                    tc_fence_after();
+                    const uint64_t da = smem_desc_sw64(smem + s * kStageBytes);
+                    const uint64_t db = smem_desc_sw64(smem + s * kStageBytes + kDig * kABytes);
+                    for (int kk = 0; kk < BK / 16; ++kk) {
+                        #pragma unroll
+                        for (int i = 0; i < kDig; ++i) {
+                            #pragma unroll
+                            for (int j = 0; j < kDig - i; ++j)
+                                umma_bf16(tmem + (i + j) * BN, da + (uint64_t)((i * kABytes + kk * 32) >> 4),
+                                          db + (uint64_t)((j * kBBytes + kk * 32) >> 4), idesc, (kt | kk | i) ? 1u : 0u);
+                        }
+                    }
+                    umma_commit(&empty[s]);
+                }
+                umma_commit(tfull);
+            }
+            if (err) atomicExch(&s_err, 1);
+        }
+    } else {
+        const int q = warp & 3, h = (warp - 2) >> 2;          // TMEM lane quarter, column half
+        uint32_t it = 0;
+        for (int64_t tile = blockIdx.x; tile < n_tiles; tile += gridDim.x, ++it) {
+            int g, n0;
+            int64_t k0;
+            locate(tile, g, k0, n0);
+            const RowGroup& rg = a.rows.g[g];
+            const int64_t k = k0 + q * 32 + lane;             // row within the group
+            const bool live = k < (int64_t)nv * rg.rpw;
+            const int64_t b = live ? k / rg.rpw : 0;
+            const int64_t row = b * rg.out_rpw + rg.out_off + (live ? k % rg.rpw : 0);
+            const int t = (int)(row % a.channels);
+            const int ea = live ? a.ea[rg.base + k] : 0;
+            const double* rb = a.e.rowbias ? a.e.rowbias + (b * a.channels + t) * a.e.ldrb : nullptr;
+            const bool ready = mbar_wait(tfull, it & 1);
+            if (!ready && lane == 0) s_epi_err = 1;
+            asm volatile("bar.sync 1, %0;" ::"n"(32 * kEpi) : "memory");   // all epilogue warps agree
+            if (*(volatile int*)&s_epi_err) { if (lane == 0) atomicExch(&s_err, 1); break; }
+            tc_fence_after();
+            for (int c0 = h * 8; c0 < BN; c0 += 16) {
+                if (n0 + c0 >= a.N) break;
+                float acc[kDig * 8];
+                #pragma unroll
+                for (int s = 0; s < kDig; ++s) tmem_ld8(tmem + s * BN + ((uint32_t)(q * 32) << 16) + c0, acc + s * 8);
+                tmem_wait_ld();
+                if (live) {
+                    #pragma unroll
+                    for (int j = 0; j < 8; j += 2) {
+                        double v[2];
+                        #pragma unroll
+                        for (int u = 0; u < 2; ++u) {
+                            const int n = min(n0 + c0 + j + u, a.N - 1);
+                            const int ew = a.ew[n];
+                            const int scale = ea + ew - 68;
+                            if (ea == kFlagged || ew == kFlagged || scale < -900 || scale > 900) {
+                                double x = 0.0;
+                                for (int kk = 0; kk < a.K; ++kk)
+                                    x = fma(a.A[row * a.lda + kk], (double)a.W[(int64_t)kk * a.ldw + n], x);
+                                v[u] = x;
+                            } else {
+                                v[u] = combine_digits(acc + j + u, 8, scale);
+                            }
+                            if (a.e.bias && t == 0) v[u] += (double)a.e.bias[n];
+                            if (rb) v[u] += rb[n];
+                        }
+                        const int n = n0 + c0 + j;
+                        double* o = a.C + row * a.ldc + n;
+                        if (n + 1 < a.N && !(a.ldc & 1)) *reinterpret_cast<double2*>(o) = make_double2(v[0], v[1]);
+                        else {
+                            if (n < a.N) o[0] = v[0];
+                            if (n + 1 < a.N) o[1] = v[1];
+                        }
+                    }
+                }
+                __syncwarp();
+            }
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(tempty);
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (s_err && threadIdx.x == 0) atomicExch(a.error, 1);
+    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem) : "memory");
+}
+
+}  // namespace
+
+void slice_rows64(const double* A, int lda, int K, const Rows64& rows, const Digits& d, cudaStream_t s) {
+    int64_t n = 0;
+    for (int g = 0; g < rows.ngroups; ++g) n += (int64_t)rows.B * rows.g[g].rpw;
+    k64_slice_rows<<<(unsigned)((n + 7) / 8), 256, 0, s>>>(A, lda, K, rows, d);
+    count_launch();
+}
+
+void spin_means64(const double* X, int ldx, int hw, int n, int nu, int C, const Rows64& rows, double* M, const Digits& d,
+                  cudaStream_t s) {
+    k64_spin_means<<<(unsigned)(((int64_t)rows.B * C + 7) / 8), 256, 0, s>>>(X, ldx, hw, n, nu, C, rows, M, d);
+    count_launch();
+}
+
+void slice_weights64(const Weight64* w, int count, const int* nvalid, cudaStream_t s) {
+    WeightTable t;
+    t.count = count;
+    t.nvalid = nvalid;
+    t.first[0] = 0;
+    for (int k = 0; k < count; ++k) {
+        t.w[k] = w[k];
+        t.first[k + 1] = t.first[k] + (w[k].N + 31) / 32;
+    }
+    k64_slice_weights<<<t.first[count], 256, 0, s>>>(t);
+    count_launch();
+}
+
+int gemm64_tc(const double* A, int lda, const Digits& da, const Weight64& w, double* C, int ldc, const Rows64& rows,
+              int channels, const Epi64& e, cudaStream_t s) {
+    if (w.K > kMaxK64 || da.Kp < w.K || w.d.Kp < w.K) return DW_ERR_ARG;
+    CUtensorMap ma, mb;
+    DW_CHECK(make_map3(&ma, da.dig, kDig, (int)da.rows, da.Kp, da.Kp, da.rows * da.Kp, BK, BM, kDig, false));
+    DW_CHECK(make_map3(&mb, w.d.dig, kDig, w.N, w.d.Kp, w.d.Kp, w.d.rows * w.d.Kp, BK, BN, kDig, false));
+    Args64 a;
+    a.A = A; a.lda = lda; a.W = w.w; a.ldw = w.ldw; a.C = C; a.ldc = ldc;
+    a.ea = da.ex; a.ew = w.d.ex;
+    a.rows = rows; a.e = e;
+    a.N = w.N; a.K = w.K; a.channels = channels;
+    a.ntn = (w.N + BN - 1) / BN;
+    a.error = tc_error_flag();
+    if (!a.error) return DW_ERR_CUDA;
+    int64_t tiles = 0;
+    for (int g = 0; g < rows.ngroups; ++g) tiles += ((int64_t)rows.B * rows.g[g].rpw + BM - 1) / BM * a.ntn;
+    DW_CHECK_CUDA(cudaFuncSetAttribute(k64_gemm_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem64));
+    timer_begin("fp64_gemm", s);
+    k64_gemm_tc<<<(unsigned)std::min<int64_t>(tiles, num_sms()), kThreads64, kSmem64, s>>>(ma, mb, a);
+    timer_end("fp64_gemm", s, 0.0, 0.0);
+    count_launch();
+    DW_CHECK_CUDA(cudaGetLastError());
+    return DW_OK;
+}
+
+}  // namespace dw
+
+extern "C" {
+
+// Test hook: C [M, N] = A [M, K] (row stride lda) @ W [K, N] (FP32, row stride ldw) by the digit products; ws
+// holds the digit planes (dw_debug_gemm_fp64_bytes).
+size_t dw_debug_gemm_fp64_bytes(int M, int N, int K) {
+    return ((size_t)M + N) * dw::kDig * dw::pad_k64(K) * 2 + ((size_t)M + N) * 4 + 4 * 256;
+}
+int dw_debug_gemm_fp64(const double* A, int lda, const float* W, int ldw, double* C, int M, int N, int K, void* ws,
+                       void* stream) {
+    using namespace dw;
+    if (!tc_available()) return DW_ERR_UNSUPPORTED;
+    if (!A || !W || !C || !ws || M <= 0 || N <= 0 || K <= 0 || K > kMaxK64) return DW_ERR_ARG;
+    cudaStream_t s = (cudaStream_t)stream;
+    Carver c(ws, (size_t)-1);
+    Digits da{c.take<__nv_bfloat16>((size_t)kDig * M * pad_k64(K)), c.take<int>(M), M, pad_k64(K)};
+    Weight64 w{W, ldw, K, N, {c.take<__nv_bfloat16>((size_t)kDig * N * pad_k64(K)), c.take<int>(N), N, pad_k64(K)}};
+    const Rows64 rows = plain_rows(M, 1, nullptr);
+    slice_rows64(A, lda, K, rows, da, s);
+    slice_weights64(&w, 1, nullptr, s);
+    return gemm64_tc(A, lda, da, w, C, N, rows, 1, Epi64(), s);
+}
+
+}  // extern "C"

@@ -1,10 +1,19 @@
 // Persistent tcgen05 tensor-core GEMM (TMA loads, TMEM accumulators, TMA stores).
 #pragma once
 #include "net.cuh"
+#include "tc_ptx.cuh"
 
 namespace dw {
 
 bool tc_available();
+int num_sms();
+int* tc_error_flag();      // device address of the error flag of the tensor-core kernels (null on failure)
+
+// Tensor maps of K-major tiles (swizzle = box_cols * element size: 128 or 64 bytes).
+int make_map(CUtensorMap* map, const void* base, int64_t rows, int cols, int64_t ld, int box_cols, int box_rows,
+             bool f32);
+int make_map3(CUtensorMap* map, const void* base, int64_t nw, int rows, int cols, int64_t ld, int64_t wstride,
+              int box_cols, int box_rows, int box_w, bool f32);
 
 // C[M, N] = epilogue(A[M, K] @ W[N, K]^T).
 // np = 1: A and W are BF16; np = 2: split-BF16 (A is [hi | lo] rows of logical width lda, W = W0 + W1).
