@@ -172,7 +172,7 @@ static Plan<Act> carve_plan(const Dims& d, int Bc, void* ws) {
     int pc = d.Tp > 1 ? 3 : 1, ec = d.Tp > 1 ? 5 : 1;
     p.WP = c.take<float>((int64_t)4 * Bc * d.n * d.n * pc * 32);
     p.HE = c.take<float>((int64_t)4 * Bc * d.n * d.N * ec * 32);
-    p.BF = c.take<float>(rows * round_up(2 * d.KN, 4));   // row pitch padded to 16 bytes (TMA stores)
+    p.BF = c.take<float>(rows * round_up(2 * d.KN, 4));   // row pitch padded to 16 bytes (TMA stores of value rows)
     p.MO = c.take<float>((int64_t)Bc * d.K * d.T * d.n * d.n);
     p.logdet = c.take<double>((int64_t)Bc * d.K);
     p.sign = c.take<double>((int64_t)Bc * d.K);
@@ -226,24 +226,26 @@ template <> struct MM<float> {
         return DW_OK;
     }
 };
+// All electrons of the M / (n T) walkers of a tangent pass.
+static inline JetRows jet_rows(int M, const Dims& d) { return JetRows{M / (d.n * d.T), d.n, d.T, d.n, 0}; }
 template <class Act> struct MMTC {
     static constexpr int np = ActIO<Act>::kParts;
     static constexpr int out_act = np == 2 ? 2 : 1;
     static int mm(const Act* A, int lda, const WRef& W, float* C, int ldc, int M, int N, int K, const GemmEpi& e,
                   cudaStream_t s) {
-        return gemm_tc(np, 0, A, lda, W.hi, W.lo, C, ldc, M, N, K, e, 0, 0, s);
+        return gemm_tc(np, 0, A, lda, W.hi, W.lo, C, ldc, M, N, K, e, s);
     }
     static int mm(const Act* A, int lda, const WRef& W, Act* C, int ldc, int M, int N, int K, const GemmEpi& e,
                   cudaStream_t s) {
-        return gemm_tc(np, out_act, A, lda, W.hi, W.lo, C, ldc, M, N, K, e, 0, 0, s);
+        return gemm_tc(np, out_act, A, lda, W.hi, W.lo, C, ldc, M, N, K, e, s);
     }
     static int mm_fl(const Act* A, int lda, const WRef& W, float* C, int ldc, int M, int N, int K, const GemmEpi& e,
                      const Dims& d, float*, cudaStream_t s) {
-        return gemm_tc(np, 0, A, lda, W.hi, W.lo, C, ldc, M, N, K, e, 1, 3 * d.n, s);
+        return gemm_jet(np, 0, 1, A, lda, W.hi, W.lo, C, ldc, jet_rows(M, d), N, K, e, s);
     }
     static int mm_fl(const Act* A, int lda, const WRef& W, Act* C, int ldc, int M, int N, int K, const GemmEpi& e,
                      const Dims& d, float*, cudaStream_t s) {
-        return gemm_tc(np, out_act, A, lda, W.hi, W.lo, C, ldc, M, N, K, e, 1, 3 * d.n, s);
+        return gemm_jet(np, out_act, 1, A, lda, W.hi, W.lo, C, ldc, jet_rows(M, d), N, K, e, s);
     }
 };
 template <> struct MM<__nv_bfloat16> : MMTC<__nv_bfloat16> {};
@@ -251,9 +253,6 @@ template <> struct MM<Split> : MMTC<Split> {};
 
 // Runs `stmt` between per-tag timer events (no-ops unless dw_timer_enable(1)).
 #define DW_TIMED(tag, stmt) do { timer_begin(tag, s); stmt; timer_end(tag, s, 0.0, 0.0); } while (0)
-
-// Element offset of row `row` in a logical-width-ld activation buffer of type Act.
-template <class Act> static inline int64_t act_off(int64_t row, int ld) { return row * ld * ActIO<Act>::kParts; }
 
 // The forward (value or tangent) of one chunk of walkers.
 template <class Act>
@@ -308,8 +307,7 @@ static int run_chunk(const Plan<Act>& p, int Bc, int precision, const float* P, 
         WRef wm = wref(pre.main[l], d.D, &pre.main_bf[0][0], l);
         if (tang) {
             // algorithmic work of this launch: 2 M N K over the T = 3n + 2 channel rows of each
-            // electron (not the Tp - T zero padding rows the launch also moves) and the unpadded K,
-            // A and C streamed once
+            // electron and the unpadded K, A and C streamed once
             const double kreal = hw + d.E + d.eiw[l];
             const double rows_alg = (double)Bc * d.n * d.T;
             const double flops = 2.0 * rows_alg * d.D * kreal;
@@ -328,26 +326,19 @@ static int run_chunk(const Plan<Act>& p, int Bc, int precision, const float* P, 
     }
     const Act* H = xin;   // final embedding, logical row width kXW
     // backflow (envelope_orbitals.py:46-75). Tensor-core tangent passes: one GEMM per spin over
-    // that spin's electron rows of every walker (walker-block tensor maps), so each row gets only
-    // its own spin's KN columns. Otherwise every row times [W_up | W_dn] and the envelope kernel
-    // takes the half that matches the electron's spin.
+    // that spin's electron rows of every walker, so each row gets only its own spin's KN columns.
+    // Otherwise every row times [W_up | W_dn] and the envelope kernel takes the half that matches
+    // the electron's spin.
     int ldbf = round_up(2 * d.KN, 4), spin_cols = d.KN;
-    const bool per_spin = tang && pt >= 1 && (d.nu * d.Tp) % 32 == 0 && (d.nd * d.Tp) % 32 == 0 && d.KN % 4 == 0;
-    if (per_spin) {
+    if (tang && pt >= 1) {
         ldbf = d.KN;
         spin_cols = 0;
         timer_begin("backflow_gemm", s);
         for (int spin = 0; spin < 2; ++spin) {
-            const int i0 = spin == 0 ? 0 : d.nu, ns = spin == 0 ? d.nu : d.nd;
-            WalkerBlocks wb;
-            wb.nw = Bc;
-            wb.rows = ns * d.Tp;
-            wb.a_wstride = (int64_t)d.n * d.Tp * kXW * ActIO<Act>::kParts;
-            wb.c_wstride = (int64_t)d.n * d.Tp * d.KN;
+            const JetRows jr{Bc, d.n, d.T, spin == 0 ? d.nu : d.nd, spin == 0 ? 0 : d.nu};
             const int64_t wrow = (int64_t)spin * d.KN * d.D;           // W_up / W_dn rows of the K-major copy
-            DW_CHECK(gemm_tc_wb(pt, H + act_off<Act>((int64_t)i0 * d.Tp, kXW), kXW, pre.bf_bf[0] + wrow,
-                                pt >= 2 ? pre.bf_bf[1] + wrow : nullptr, p.BF + (int64_t)i0 * d.Tp * d.KN, d.KN, wb,
-                                d.KN, d.D, s));
+            DW_CHECK(gemm_jet(pt, 0, 0, H, kXW, pre.bf_bf[0] + wrow, pt >= 2 ? pre.bf_bf[1] + wrow : nullptr, p.BF, d.KN,
+                              jr, d.KN, d.D, GemmEpi(), s));
         }
         timer_end("backflow_gemm", s, 0.0, 0.0);
     } else {
@@ -454,7 +445,7 @@ static int forward_all(const DwArch* a, int precision, const float* P, const voi
     Dims d = make_dims(a, tang);
     if (nseg < 1 || nseg > kMaxSeg || (nseg > 1 && !seg)) return DW_ERR_ARG;
     // the fused forward-Laplacian epilogue keeps one electron's channels inside a 128-row tile
-    if (tang && !std::is_same<Act, float>::value && d.Tp > 128) return DW_ERR_ARCH;
+    if (tang && !std::is_same<Act, float>::value && d.T > 128) return DW_ERR_ARCH;
     ParamLayout L;
     make_layout(a, &L);
     Prepared pre = carve_prepared(a, precision, const_cast<void*>(prepared));

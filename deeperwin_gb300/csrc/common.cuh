@@ -59,7 +59,7 @@ struct Dims {
     int kw[4];     // row width of the per-electron layer input [h | conv_ee | conv_ei] padded to 64
     int KN;        // n_dets * n_el
     int T;         // channels: 1 (value) or 3n + 2 (value, 3n gradients, Laplacian)
-    int Tp;        // padded channel count (power of two >= T)
+    int Tp;        // channel rows per electron in memory (= T)
     int lap;       // index of the Laplacian channel (T-1) or -1
     // Packed launches: walker b of this launch belongs to geometry segment seg[b] (R, Z and the
     // ion maps are per segment; ions with Z = 0 are padding and contribute nothing).

@@ -220,15 +220,6 @@ struct Args64 {
     int* error;                    // set when a bounded wait ran out
 };
 
-__device__ __forceinline__ void tmem_ld8(uint32_t taddr, float* v) {
-    uint32_t r[8];
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
-                 : "r"(taddr));
-    #pragma unroll
-    for (int j = 0; j < 8; ++j) v[j] = __uint_as_float(r[j]);
-}
-
 // 2^scale sum_s acc_s 2^(56 - 7 s), rounded to the nearest double. |sum| < 2^79.
 __device__ __forceinline__ double combine_digits(const float* acc, int stride, int scale) {
     long long hi = 0, lo = 0;

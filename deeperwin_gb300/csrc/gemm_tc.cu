@@ -10,10 +10,8 @@
 // * Shared-memory ring of S stages (128-byte swizzled K-major tiles), two TMEM accumulators
 //   so the epilogue of tile i overlaps the main loop of tile i + 1, one CTA per SM looping
 //   over output tiles.
-// * Epilogue: value-channel bias, per-(walker, channel) row bias, and either tanh on value
-//   rows or the forward-Laplacian tanh across the Tp channel rows of each electron
-//   (y = tanh z; y_t = (1 - y^2) z_t; y_lap = (1 - y^2) z_lap - 2 y (1 - y^2) sum_t z_t^2).
-//   Results are written to swizzled shared-memory staging tiles (two per warp, so the staging
+// * Epilogue: value-channel bias, per-(walker, channel) row bias and tanh on value rows (the tangent
+//   passes' layers are in gemm_jet.cu). Results are written to swizzled shared-memory staging tiles (two per warp, so the staging
 //   of one chunk overlaps the TMA store of the previous one) and stored with TMA.
 // Every mbarrier wait is bounded; on timeout the kernel records an error flag, stops
 // issuing, waits (bounded) for its TMA loads in flight, frees its TMEM and returns.
@@ -112,10 +110,8 @@ constexpr int kEpiWarps = 8;                         // two per TMEM lane quarte
 constexpr int kThreads = 64 + 32 * kEpiWarps;        // producer warp, MMA warp, epilogue warps
 constexpr int CW = 32;                               // columns per epilogue chunk / staged store box
 
-// named barriers: 1 = all epilogue warps, 2 + h = the four epilogue warps of column half h
+// named barrier 1: all epilogue warps
 __device__ __forceinline__ void epi_bar() { asm volatile("bar.sync 1, %0;" ::"n"(32 * kEpiWarps) : "memory"); }
-__device__ __forceinline__ void half_bar(int h) { asm volatile("bar.sync %0, 128;" ::"r"(2 + h) : "memory"); }
-
 
 // 16-byte chunk j of row r in a 128-byte-swizzled staging tile (128-byte rows, 1024-byte aligned).
 __device__ __forceinline__ uint32_t swz(int r, int j) { return (uint32_t)(r * 128 + ((j ^ (r & 7)) << 4)); }
@@ -123,25 +119,12 @@ __device__ __forceinline__ uint32_t swz(int r, int j) { return (uint32_t)(r * 12
 // index is XORed with address bits 7-8, i.e. with (r >> 1) & 3.
 __device__ __forceinline__ uint32_t swz64(int r, int j) { return (uint32_t)(r * 64 + ((j ^ ((r >> 1) & 3)) << 4)); }
 
-// Forward-Laplacian scratch per epilogue warp: four per-column arrays for up to four electron
-// groups (value-row z and the coefficient rows d1 = 1 - tanh^2, y0 = tanh(z0),
-// cl = -2 y0 d1 sum_t z_t^2), pitch kFlP floats (16-byte aligned), then a zero row.
-constexpr int kFlP = CW + 4;
-constexpr int kFlWarp = 4 * 4 * kFlP + CW;
-
 struct TcArgs {
     int M, N, K, BN;
     GemmEpi epi;
-    int fl;             // forward-Laplacian epilogue (rows grouped by Tp channels)
-    int n3;             // 3 n_el: channels 1..n3 are gradients, n3 + 1 the Laplacian
     int stages;
     uint32_t tmem_cols;
     int n_tiles_n, n_tiles;
-    // Walker-block mode (nrb > 0): A and C are 3-D tensors {K or N, rows per walker block, walkers};
-    // M tile mi covers row block (mi % nrb) of 32 rows in walkers 4 (mi / nrb) .. + 3, and epilogue
-    // warp q stores the rows of walker 4 (mi / nrb) + q. Plain epilogue only (no bias, tanh or
-    // forward-Laplacian rows).
-    int nrb;
 };
 
 // OUT: 0 = fp32 C, 1 = bf16 C, 2 = split-BF16 C. BK: K-columns per pipeline stage (64 or 32).
@@ -159,9 +142,7 @@ k_gemm_tc(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__ CUte
     auto sA = [&](int s, int part) { return smem + (size_t)s * stage_bytes + (size_t)part * a_bytes; };
     auto sB = [&](int s, int part) { return smem + (size_t)s * stage_bytes + (size_t)NP * a_bytes + (size_t)part * b_bytes; };
     uint8_t* stage_out = smem + (size_t)S * stage_bytes;                   // [epilogue warp][2 buffers][SWB]
-    float* xchg = reinterpret_cast<float*>(stage_out + 2 * kEpiWarps * SWB); // [half][2 bufs][2 arrays][4][CW]
-    float* flbuf = xchg + 2 * 2 * 2 * 4 * CW;                              // [epilogue warp][kFlWarp]
-    uint64_t* full = reinterpret_cast<uint64_t*>(flbuf + kEpiWarps * kFlWarp);
+    uint64_t* full = reinterpret_cast<uint64_t*>(stage_out + 2 * kEpiWarps * SWB);
     uint64_t* empty = full + S;
     uint64_t* tfull = empty + S;     // [2]
     uint64_t* tempty = tfull + 2;    // [2]
@@ -203,14 +184,8 @@ k_gemm_tc(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__ CUte
                     const uint32_t use = cnt / S;
                     if (use > 0 && !mbar_wait(&empty[s], (use - 1) & 1)) { err = true; break; }
                     mbar_expect_tx(&full[s], stage_bytes);
-                    if (a.nrb) {
-                        const int mi = tile / a.n_tiles_n, rb = (mi % a.nrb) * 32, w0 = (mi / a.nrb) * 4;
-                        tma_load_3d(sA(s, 0), &tmA0, &full[s], kt * BK, rb, w0);
-                        if (NP == 2) tma_load_3d(sA(s, 1), &tmA1, &full[s], kt * BK, rb, w0);
-                    } else {
-                        tma_load_2d(sA(s, 0), &tmA0, &full[s], kt * BK, m0);
-                        if (NP == 2) tma_load_2d(sA(s, 1), &tmA1, &full[s], kt * BK, m0);
-                    }
+                    tma_load_2d(sA(s, 0), &tmA0, &full[s], kt * BK, m0);
+                    if (NP == 2) tma_load_2d(sA(s, 1), &tmA1, &full[s], kt * BK, m0);
                     tma_load_2d(sB(s, 0), &tmB0, &full[s], kt * BK, n0);
                     if (NP == 2) tma_load_2d(sB(s, 1), &tmB1, &full[s], kt * BK, n0);
                     issued[s] = use + 1;
@@ -263,7 +238,6 @@ k_gemm_tc(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__ CUte
         const int Tp = e.Tp;
         uint32_t nchunk = 0;                         // chunks staged by this warp (selects the buffer)
         uint32_t it = 0;
-        int xbuf = 0;
         for (int tile = blockIdx.x; tile < a.n_tiles; tile += gridDim.x, ++it) {
             const int m0 = (tile / a.n_tiles_n) * BM, n0 = (tile % a.n_tiles_n) * BN;
             const uint32_t acc = it & 1;
@@ -272,7 +246,7 @@ k_gemm_tc(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__ CUte
             const int t = m % Tp;
             const float* rb = (e.rowbias && m < a.M) ? e.rowbias + ((int64_t)(m / e.rows_per_walker) * Tp + t) * e.ldrb
                                                      : nullptr;
-            const bool is_val = t == 0, is_grad = t >= 1 && t <= a.n3, is_lap = a.fl && t == a.n3 + 1;
+            const bool is_val = t == 0;
             // bias / row-bias of one CW-column chunk (vectorized; rows of one walker share their
             // row-bias rows, so neighbouring warps hit in L1)
             float rbv[CW];
@@ -330,121 +304,7 @@ k_gemm_tc(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__ CUte
                 ++nchunk;
                 if (lane == 0) bulk_wait_read1();
                 __syncwarp();
-                if (a.fl) {
-                    // Forward-Laplacian tanh over the Tp channel rows of each electron:
-                    // y_0 = tanh(z_0), y_t = d1 z_t (gradients), y_lap = d1 z_lap - 2 y0 d1 sum_t z_t^2,
-                    // d1 = 1 - y0^2. Gradient rows stage their squares in the swizzled staging tile (free
-                    // here: its last TMA store has finished reading it) and the value row its value
-                    // in Z0. Lanes add float4 column chunks over 8-row blocks, the blocks of one electron
-                    // are combined in-lane, by shuffles or (Tp > 32) across warps, and the lane holding a
-                    // group's column sums writes that group's coefficient rows for its four columns.
-                    // Each row then takes y = alpha v + beta with coefficient rows chosen by its type.
-                    float* sq = reinterpret_cast<float*>(my_out);          // [32 rows][CW] swizzled by 16 B chunks
-                    float* fb = flbuf + (size_t)ew * kFlWarp;
-                    float* Z0 = fb;                                       // [group][kFlP]
-                    float* D1 = fb + 4 * kFlP;
-                    float* Y0 = fb + 8 * kFlP;
-                    float* CL = fb + 12 * kFlP;
-                    float* ZR = fb + 16 * kFlP;                           // zero row
-                    const int grp = Tp < 32 ? lane / Tp : 0;
-                    #pragma unroll
-                    for (int j4 = 0; j4 < CW / 4; ++j4) {
-                        const float4 x4 = make_float4(v[4 * j4], v[4 * j4 + 1], v[4 * j4 + 2], v[4 * j4 + 3]);
-                        const float4 s4 = is_grad ? make_float4(x4.x * x4.x, x4.y * x4.y, x4.z * x4.z, x4.w * x4.w)
-                                                  : make_float4(0.f, 0.f, 0.f, 0.f);
-                        *reinterpret_cast<float4*>(sq + lane * CW + ((j4 ^ (lane & 7)) << 2)) = s4;
-                        if (is_val) *reinterpret_cast<float4*>(Z0 + grp * kFlP + 4 * j4) = x4;
-                    }
-                    if (lane < CW / 4) reinterpret_cast<float4*>(ZR)[lane] = make_float4(0.f, 0.f, 0.f, 0.f);
-                    __syncwarp();
-                    // lane (rb, jc): column chunk jc (columns 4 jc .. 4 jc + 3), rows [rb RPL, (rb + 1) RPL)
-                    constexpr int NCH = CW / 4, RPL = NCH, NS = RPL / 8;
-                    const int jc = lane % NCH, rbk = lane / NCH;
-                    float4 ps[NS];
-                    #pragma unroll
-                    for (int s8 = 0; s8 < NS; ++s8) {
-                        float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
-                        #pragma unroll
-                        for (int i = 0; i < 8; ++i) {
-                            const int r = rbk * RPL + 8 * s8 + i;            // r & 7 == i
-                            const float4 y = *reinterpret_cast<const float4*>(sq + r * CW + ((jc ^ i) << 2));
-                            x.x += y.x; x.y += y.y; x.z += y.z; x.w += y.w;
-                        }
-                        ps[s8] = x;
-                    }
-                    auto coeffs = [&](int g, float4 ss, float4 z0) {
-                        const float y[4] = {tanhf(z0.x), tanhf(z0.y), tanhf(z0.z), tanhf(z0.w)};
-                        const float sv[4] = {ss.x, ss.y, ss.z, ss.w};
-                        float d1[4], cl[4];
-                        #pragma unroll
-                        for (int k = 0; k < 4; ++k) { d1[k] = 1.f - y[k] * y[k]; cl[k] = -2.f * y[k] * d1[k] * sv[k]; }
-                        *reinterpret_cast<float4*>(Y0 + g * kFlP + 4 * jc) = make_float4(y[0], y[1], y[2], y[3]);
-                        *reinterpret_cast<float4*>(D1 + g * kFlP + 4 * jc) = make_float4(d1[0], d1[1], d1[2], d1[3]);
-                        *reinterpret_cast<float4*>(CL + g * kFlP + 4 * jc) = make_float4(cl[0], cl[1], cl[2], cl[3]);
-                    };
-                    const int gsz = Tp < 32 ? Tp : 32;                      // rows of a group in this warp
-                    const int bpg = gsz / 8;                                // 8-row blocks per group
-                    if (bpg >= NS) {
-                        // all blocks of this lane lie in one group; add the lanes of the same group
-                        float4 g4 = ps[0];
-                        #pragma unroll
-                        for (int s8 = 1; s8 < NS; ++s8) { g4.x += ps[s8].x; g4.y += ps[s8].y; g4.z += ps[s8].z; g4.w += ps[s8].w; }
-                        for (int o = NCH; o < NCH * (bpg / NS); o <<= 1) {
-                            g4.x += __shfl_xor_sync(0xffffffffu, g4.x, o);
-                            g4.y += __shfl_xor_sync(0xffffffffu, g4.y, o);
-                            g4.z += __shfl_xor_sync(0xffffffffu, g4.z, o);
-                            g4.w += __shfl_xor_sync(0xffffffffu, g4.w, o);
-                        }
-                        const int g = (rbk * NS) / bpg;
-                        const bool holder = (rbk * NS) % bpg == 0;
-                        if (Tp <= 32) {
-                            if (holder) coeffs(g, g4, *reinterpret_cast<const float4*>(Z0 + g * kFlP + 4 * jc));
-                        } else {
-                            // a group spans several warps: exchange the partial sums and the value row
-                            float* xs = xchg + (size_t)(h * 2 + xbuf) * 2 * 4 * CW;
-                            const bool has_val = (q * 32) % Tp == 0;        // this warp holds the value row
-                            if (holder) {
-                                *reinterpret_cast<float4*>(xs + q * CW + 4 * jc) = g4;
-                                if (has_val)
-                                    *reinterpret_cast<float4*>(xs + 4 * CW + q * CW + 4 * jc) =
-                                        *reinterpret_cast<const float4*>(Z0 + 4 * jc);
-                            }
-                            half_bar(h);
-                            const int qs = Tp / 32, g0 = (q / qs) * qs;
-                            if (holder) {
-                                float4 tot = make_float4(0.f, 0.f, 0.f, 0.f);
-                                for (int k = 0; k < qs; ++k) {
-                                    const float4 pk = *reinterpret_cast<const float4*>(xs + (g0 + k) * CW + 4 * jc);
-                                    tot.x += pk.x; tot.y += pk.y; tot.z += pk.z; tot.w += pk.w;
-                                }
-                                coeffs(0, tot, *reinterpret_cast<const float4*>(xs + 4 * CW + g0 * CW + 4 * jc));
-                            }
-                            xbuf ^= 1;   // the other exchange buffer is written only after the next barrier
-                        }
-                    } else {
-                        // one 8-row block per group (Tp = 8 with 16 rows per lane)
-                        #pragma unroll
-                        for (int s8 = 0; s8 < NS; ++s8) {
-                            const int g = rbk * NS + s8;
-                            coeffs(g, ps[s8], *reinterpret_cast<const float4*>(Z0 + g * kFlP + 4 * jc));
-                        }
-                    }
-                    __syncwarp();
-                    // row type -> coefficient rows: value (0, y0), gradient (d1, 0), Laplacian
-                    // (d1, cl), padding channels (0, 0)
-                    const float* al = (is_grad || is_lap) ? D1 + grp * kFlP : ZR;
-                    const float* be = is_val ? Y0 + grp * kFlP : (is_lap ? CL + grp * kFlP : ZR);
-                    #pragma unroll
-                    for (int j4 = 0; j4 < CW / 4; ++j4) {
-                        const float4 a4 = *reinterpret_cast<const float4*>(al + 4 * j4);
-                        const float4 b4 = *reinterpret_cast<const float4*>(be + 4 * j4);
-                        v[4 * j4] = fmaf(a4.x, v[4 * j4], b4.x);
-                        v[4 * j4 + 1] = fmaf(a4.y, v[4 * j4 + 1], b4.y);
-                        v[4 * j4 + 2] = fmaf(a4.z, v[4 * j4 + 2], b4.z);
-                        v[4 * j4 + 3] = fmaf(a4.w, v[4 * j4 + 3], b4.w);
-                    }
-                    __syncwarp();
-                } else if (e.act == 1) {
+                if (e.act == 1) {
                     #pragma unroll
                     for (int j = 0; j < CW; ++j) v[j] = tanhf(v[j]);
                 }
@@ -479,13 +339,8 @@ k_gemm_tc(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__ CUte
                 fence_async_smem();
                 __syncwarp();
                 if (lane == 0) {
-                    if (a.nrb) {
-                        const int mi = tile / a.n_tiles_n;
-                        tma_store_3d(&tmC0, my_out, n0 + c0, (mi % a.nrb) * 32, (mi / a.nrb) * 4 + q);
-                    } else {
-                        tma_store_2d(&tmC0, my_out, n0 + c0, m0 + q * 32);
-                        if (OUT == 2) tma_store_2d(&tmC1, my_out + 2048, n0 + c0, m0 + q * 32);
-                    }
+                    tma_store_2d(&tmC0, my_out, n0 + c0, m0 + q * 32);
+                    if (OUT == 2) tma_store_2d(&tmC1, my_out + 2048, n0 + c0, m0 + q * 32);
                     bulk_commit();
                 }
             }
@@ -506,18 +361,12 @@ k_gemm_tc(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__ CUte
 // ------------------------------------------------------------------ host side
 // A: NP parts of a logical [M, lda] activation (NP = 2: [hi | lo] rows of width 2 lda).
 // W0/W1: [N, round_up(K, 64)] K-major weight parts. C: logical [M, ldc].
-// wb != nullptr: walker-block mode (FP32 output, plain epilogue); M is then ignored.
 // K-columns per stage of the split-BF16 GEMMs (instrumentation: dw_debug_set_gemm_bk).
 int g_split_bk = 64;
 
 template <int NP, int OUT, int BK>
 int launch_tc(const __nv_bfloat16* A, int lda, const __nv_bfloat16* W0, const __nv_bfloat16* W1, void* C, int ldc,
-              int M, int N, int K, const GemmEpi& epi, int fl, int n3, cudaStream_t s, const WalkerBlocks* wb = nullptr) {
-    if (wb) {
-        if (OUT != 0 || fl || epi.bias || epi.rowbias || epi.act || wb->rows % 32) return DW_ERR_ARG;
-        if (wb->nw <= 0) return DW_OK;
-        M = ((wb->nw + 3) / 4) * (wb->rows / 32) * BM;
-    }
+              int M, int N, int K, const GemmEpi& epi, cudaStream_t s) {
     if (M <= 0 || N <= 0 || K <= 0) return DW_OK;
     constexpr int BN_MAX = NP == 2 ? 128 : 256;      // keeps >= 2 pipeline stages in shared memory
     int ntn = (N + BN_MAX - 1) / BN_MAX;
@@ -525,22 +374,13 @@ int launch_tc(const __nv_bfloat16* A, int lda, const __nv_bfloat16* W0, const __
     while (BN > BN_MAX) { ntn += 1; BN = round_up((N + ntn - 1) / ntn, CW); }
     const int Kp = round_up(K, 64);
     CUtensorMap ma0, ma1, mb0, mb1, mc0, mc1;
-    if (wb) {
-        DW_CHECK(make_map3(&ma0, A, wb->nw, wb->rows, K, (int64_t)NP * lda, wb->a_wstride, BK, 32, 4, false));
-        if (NP == 2) DW_CHECK(make_map3(&ma1, A + lda, wb->nw, wb->rows, K, (int64_t)NP * lda, wb->a_wstride, BK, 32, 4, false));
-        else ma1 = ma0;
-    } else {
-        DW_CHECK(make_map(&ma0, A, M, K, (int64_t)NP * lda, BK, BM, false));
-        if (NP == 2) DW_CHECK(make_map(&ma1, A + lda, M, K, (int64_t)NP * lda, BK, BM, false));
-        else ma1 = ma0;
-    }
+    DW_CHECK(make_map(&ma0, A, M, K, (int64_t)NP * lda, BK, BM, false));
+    if (NP == 2) DW_CHECK(make_map(&ma1, A + lda, M, K, (int64_t)NP * lda, BK, BM, false));
+    else ma1 = ma0;
     DW_CHECK(make_map(&mb0, W0, N, K, Kp, BK, BN, false));
     if (NP == 2) DW_CHECK(make_map(&mb1, W1, N, K, Kp, BK, BN, false));
     else mb1 = mb0;
-    if (wb) {
-        DW_CHECK(make_map3(&mc0, C, wb->nw, wb->rows, N, ldc, wb->c_wstride, 32, 32, 1, true));
-        mc1 = mc0;
-    } else if (OUT == 0) {
+    if (OUT == 0) {
         DW_CHECK(make_map(&mc0, C, M, N, ldc, 32, 32, true));
         mc1 = mc0;
     } else if (OUT == 1) {
@@ -551,10 +391,9 @@ int launch_tc(const __nv_bfloat16* A, int lda, const __nv_bfloat16* W0, const __
         DW_CHECK(make_map(&mc1, reinterpret_cast<const __nv_bfloat16*>(C) + ldc, M, N, (int64_t)2 * ldc, 32, 32, false));
     }
     TcArgs a;
-    a.M = M; a.N = N; a.K = K; a.BN = BN; a.epi = epi; a.fl = fl; a.n3 = n3;
-    a.nrb = wb ? wb->rows / 32 : 0;
+    a.M = M; a.N = N; a.K = K; a.BN = BN; a.epi = epi;
     const int stage_bytes = NP * (BM * BK * 2 + BN * BK * 2);
-    const int fixed = 1024 + 2 * kEpiWarps * 4096 + 2 * 2 * 2 * 4 * CW * 4 + kEpiWarps * kFlWarp * 4 + 256;
+    const int fixed = 1024 + 2 * kEpiWarps * 4096 + 256;
     a.stages = std::min(8, (220 * 1024 - fixed) / stage_bytes);
     if (a.stages < 2) return DW_ERR_ARCH;
     a.tmem_cols = 32;
@@ -587,27 +426,17 @@ bool tc_available() {
     return cached == 1;
 }
 
-int gemm_tc_wb(int np, const void* A, int lda, const __nv_bfloat16* W0, const __nv_bfloat16* W1, float* C, int ldc,
-               const WalkerBlocks& wb, int N, int K, cudaStream_t s) {
-    const __nv_bfloat16* a = reinterpret_cast<const __nv_bfloat16*>(A);
-    GemmEpi e;
-    if (np == 1) return launch_tc<1, 0, 64>(a, lda, W0, W1, C, ldc, 0, N, K, e, 0, 0, s, &wb);
-    if (np == 2 && g_split_bk == 32) return launch_tc<2, 0, 32>(a, lda, W0, W1, C, ldc, 0, N, K, e, 0, 0, s, &wb);
-    if (np == 2) return launch_tc<2, 0, 64>(a, lda, W0, W1, C, ldc, 0, N, K, e, 0, 0, s, &wb);
-    return DW_ERR_ARG;
-}
-
 int gemm_tc(int np, int out, const void* A, int lda, const __nv_bfloat16* W0, const __nv_bfloat16* W1, void* C, int ldc,
-            int M, int N, int K, const GemmEpi& epi, int fl, int n3, cudaStream_t s) {
+            int M, int N, int K, const GemmEpi& epi, cudaStream_t s) {
     const __nv_bfloat16* a = reinterpret_cast<const __nv_bfloat16*>(A);
-    if (np == 1 && out == 0) return launch_tc<1, 0, 64>(a, lda, W0, W1, C, ldc, M, N, K, epi, fl, n3, s);
-    if (np == 1 && out == 1) return launch_tc<1, 1, 64>(a, lda, W0, W1, C, ldc, M, N, K, epi, fl, n3, s);
+    if (np == 1 && out == 0) return launch_tc<1, 0, 64>(a, lda, W0, W1, C, ldc, M, N, K, epi, s);
+    if (np == 1 && out == 1) return launch_tc<1, 1, 64>(a, lda, W0, W1, C, ldc, M, N, K, epi, s);
     if (g_split_bk == 32) {
-        if (np == 2 && out == 0) return launch_tc<2, 0, 32>(a, lda, W0, W1, C, ldc, M, N, K, epi, fl, n3, s);
-        if (np == 2 && out == 2) return launch_tc<2, 2, 32>(a, lda, W0, W1, C, ldc, M, N, K, epi, fl, n3, s);
+        if (np == 2 && out == 0) return launch_tc<2, 0, 32>(a, lda, W0, W1, C, ldc, M, N, K, epi, s);
+        if (np == 2 && out == 2) return launch_tc<2, 2, 32>(a, lda, W0, W1, C, ldc, M, N, K, epi, s);
     }
-    if (np == 2 && out == 0) return launch_tc<2, 0, 64>(a, lda, W0, W1, C, ldc, M, N, K, epi, fl, n3, s);
-    if (np == 2 && out == 2) return launch_tc<2, 2, 64>(a, lda, W0, W1, C, ldc, M, N, K, epi, fl, n3, s);
+    if (np == 2 && out == 0) return launch_tc<2, 0, 64>(a, lda, W0, W1, C, ldc, M, N, K, epi, s);
+    if (np == 2 && out == 2) return launch_tc<2, 2, 64>(a, lda, W0, W1, C, ldc, M, N, K, epi, s);
     return DW_ERR_ARG;
 }
 
@@ -622,7 +451,7 @@ int dw_debug_gemm_bf16(const void* A, int lda, const void* Wt, const void* Wt_lo
     if (!dw::tc_available()) return DW_ERR_UNSUPPORTED;
     dw::GemmEpi e;
     return dw::gemm_tc(Wt_lo ? 2 : 1, 0, A, lda, (const __nv_bfloat16*)Wt, (const __nv_bfloat16*)Wt_lo, C, ldc, M, N, K,
-                       e, 0, 0, (cudaStream_t)stream);
+                       e, (cudaStream_t)stream);
 }
 
 // Instrumentation: K-columns per pipeline stage of the split-BF16 GEMMs (64: two stages of 64 KB at

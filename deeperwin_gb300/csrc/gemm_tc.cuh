@@ -18,20 +18,18 @@ int make_map3(CUtensorMap* map, const void* base, int64_t nw, int rows, int cols
 // C[M, N] = epilogue(A[M, K] @ W[N, K]^T).
 // np = 1: A and W are BF16; np = 2: split-BF16 (A is [hi | lo] rows of logical width lda, W = W0 + W1).
 // out = 0: fp32 C (row stride ldc); 1: bf16 C; 2: split-BF16 C ([hi | lo] rows of logical width ldc).
-// fl = 1: forward-Laplacian tanh epilogue over groups of epi.Tp channel rows (n3 = 3 n_el);
-// fl = 0: bias / row bias and optional tanh (epi.act).
-// W rows have stride round_up(K, 64).
+// Bias / row bias and optional tanh (epi.act). W rows have stride round_up(K, 64).
 int gemm_tc(int np, int out, const void* A, int lda, const __nv_bfloat16* W0, const __nv_bfloat16* W1, void* C, int ldc,
-            int M, int N, int K, const GemmEpi& epi, int fl, int n3, cudaStream_t s);
+            int M, int N, int K, const GemmEpi& epi, cudaStream_t s);
 
-// Walker-block operands: per walker `rows` consecutive rows (a multiple of 32) of A (row stride
-// np * lda) and C (row stride ldc), walkers a_wstride / c_wstride elements apart.
-struct WalkerBlocks {
-    int nw, rows;
-    int64_t a_wstride, c_wstride;
+// Rows of a tangent pass: T channel rows of electrons [i0, i0 + ns) of each of nw walkers of n electrons.
+struct JetRows {
+    int nw, n, T, ns, i0;
 };
-// C (fp32) = A @ W^T over the rows of every walker block, plain epilogue.
-int gemm_tc_wb(int np, const void* A, int lda, const __nv_bfloat16* W0, const __nv_bfloat16* W1, float* C, int ldc,
-               const WalkerBlocks& wb, int N, int K, cudaStream_t s);
+// C[(e, t), f] over those rows (the same rows of A and C): fl = 1 with bias (value rows), row bias (one row
+// per walker and channel) and the forward-Laplacian tanh over each electron's T rows; fl = 0 the plain
+// product. np, out and the strides as for gemm_tc; no alignment is asked of C. T <= 128.
+int gemm_jet(int np, int out, int fl, const void* A, int lda, const __nv_bfloat16* W0, const __nv_bfloat16* W1, void* C,
+             int ldc, const JetRows& rows, int NF, int K, const GemmEpi& epi, cudaStream_t s);
 
 }  // namespace dw

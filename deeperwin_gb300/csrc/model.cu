@@ -124,7 +124,7 @@ Dims make_dims(const DwArch* a, bool tangents) {
     d.KN = d.K * d.n;
     if (tangents) {
         d.T = 3 * d.n + 2;
-        d.Tp = next_pow2(d.T);
+        d.Tp = d.T;
         d.lap = d.T - 1;
     } else {
         d.T = 1; d.Tp = 1; d.lap = -1;

@@ -1,11 +1,10 @@
 // Per-walker network kernels of the dpe4 wavefunction with forward-mode Laplacian.
 //
 // Channel convention for every per-electron tensor X[(b, i, t), col] (rows ordered walker,
-// electron, channel; Tp rows per electron):
+// electron, channel; Tp = T rows per electron):
 //   t = 0            value
 //   t = 1 + 3m + c   d/d r_{m,c}   (m = electron, c = x,y,z)
 //   t = 3n + 1       Laplacian over all 3n coordinates
-//   t > 3n + 1       zero padding up to Tp (a power of two)
 // In value-only mode Tp = 1.
 //
 // The 2-el streams depend on r only through d_ij = |r_j - r_i|, so they are carried in
@@ -854,7 +853,6 @@ __global__ void k_tanh_fl(const float* __restrict__ Zb, int ldz, int ncols, int 
         ActIO<Act>::store(Y, r0 + t, ldy, f, d1 * zt);
     }
     ActIO<Act>::store(Y, r0 + d.lap, ldy, f, d1 * z[(int64_t)d.lap * ldz] - 2.f * y0 * d1 * s);
-    for (int t = d.lap + 1; t < d.Tp; ++t) ActIO<Act>::store(Y, r0 + t, ldy, f, 0.f);
 }
 
 // ------------------------------------------------------------------ SchNet convolutions
@@ -930,7 +928,7 @@ __global__ void k_conv(const float* __restrict__ r, const float* __restrict__ WP
 }
 
 // Register-tiled tangent convolution. Block = (walker, tile of TI = 4 electrons i) with
-// NW = Tp / TT warps; lane = feature f, warp w owns channels [w TT, w TT + TT). The main loop
+// NW = (T rounded up to a power of two) / TT warps; lane = feature f, warp w owns channels [w TT, w TT + TT). The main loop
 // loads w_ij (4 rows) and h_j (TT channels) once per j and issues 4 TT FMAs. The results are
 // staged in shared memory, where the product-rule terms are added with per-(i, j) items spread
 // over the warps: single terms w'_im u_im h_m for the channels of the other electrons m, the
@@ -944,7 +942,7 @@ k_conv_tile(const float* __restrict__ r, const float* __restrict__ WPl, const fl
             int ldx, int ei_fused) {
     extern __shared__ __align__(16) float smc[];
     const int n = d.n, Tp = d.Tp, T = d.T;
-    const int NW = Tp / TT;
+    const int NW = blockDim.x >> 5;
     float* out = smc;                                   // [TI][Tp][32] conv_ee
     float* red = out + TI * Tp * 32;                    // [NW][TI][4][32] own-gradient / Laplacian partials
     float* eiv = red + NW * TI * 4 * 32;                // [TI][5][32] conv_ei channels
@@ -980,7 +978,8 @@ k_conv_tile(const float* __restrict__ r, const float* __restrict__ WPl, const fl
         #pragma unroll
         for (int ii = 0; ii < TI; ++ii)
             #pragma unroll
-            for (int k = 0; k < TT; ++k) out[(ii * Tp + t0 + k) * 32 + f] = acc[ii][k];
+            for (int k = 0; k < TT; ++k)
+                if (t0 + k < T) out[(ii * Tp + t0 + k) * 32 + f] = acc[ii][k];
     }
     // product-rule partials of the own-gradient channels and the Laplacian, j split over warps
     for (int ii = 0; ii < ni; ++ii) {
@@ -1036,7 +1035,9 @@ k_conv_tile(const float* __restrict__ r, const float* __restrict__ WPl, const fl
             const float dx = rb[m * 3] - rb[i * 3], dy = rb[m * 3 + 1] - rb[i * 3 + 1], dz = rb[m * 3 + 2] - rb[i * 3 + 2];
             const float inv = 1.f / sqrtf(dx * dx + dy * dy + dz * dz);
             const float g = __ldg(wpb + ((size_t)i * n + m) * 96 + 32) * __ldg(hmb + (size_t)m * Tp * 32) * inv;
-            o[(1 + 3 * m) * 32] += g * dx; o[(2 + 3 * m) * 32] += g * dy; o[(3 + 3 * m) * 32] += g * dz;
+            o[(1 + 3 * m) * 32] = fmaf(g, dx, o[(1 + 3 * m) * 32]);
+            o[(2 + 3 * m) * 32] = fmaf(g, dy, o[(2 + 3 * m) * 32]);
+            o[(3 + 3 * m) * 32] = fmaf(g, dz, o[(3 + 3 * m) * 32]);
         }
     }
     __syncthreads();
@@ -1052,7 +1053,7 @@ k_conv_tile(const float* __restrict__ r, const float* __restrict__ WPl, const fl
         if (u < 4) {
             const float* src = out + (ii * Tp + t) * 32 + 8 * u;
             #pragma unroll
-            for (int k = 0; k < 8; ++k) v[k] = t < T ? src[k] : 0.f;
+            for (int k = 0; k < 8; ++k) v[k] = src[k];
             col = hw + 8 * u;
         } else {
             int ch = -1;
@@ -1376,8 +1377,8 @@ void launch_conv(const float* r, const float* WPl, const float* HM, const float*
         // product-rule loops outweigh the extra reuse of each h_map load)
         constexpr int TI = 4;
         const unsigned grid = (unsigned)B * ((d.n + TI - 1) / TI);
-        const int TT = d.Tp >= 64 ? 8 : d.Tp / 8;
-        const int NW = d.Tp / TT;
+        const int rows = next_pow2(d.Tp), TT = rows >= 64 ? 8 : rows / 8;
+        const int NW = rows / TT;
         const size_t smem = ((size_t)TI * d.Tp * 32 + (size_t)NW * TI * 4 * 32 + (size_t)TI * 5 * 32) * sizeof(float);
         auto go = [&](auto kern) {
             cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
