@@ -241,11 +241,11 @@ template <class Act> struct MMTC {
     }
     static int mm_fl(const Act* A, int lda, const WRef& W, float* C, int ldc, int M, int N, int K, const GemmEpi& e,
                      const Dims& d, float*, cudaStream_t s) {
-        return gemm_jet(np, 0, 1, A, lda, W.hi, W.lo, C, ldc, jet_rows(M, d), N, K, e, s);
+        return gemm_jet(np, 0, A, lda, W.hi, W.lo, C, ldc, jet_rows(M, d), N, K, e, s);
     }
     static int mm_fl(const Act* A, int lda, const WRef& W, Act* C, int ldc, int M, int N, int K, const GemmEpi& e,
                      const Dims& d, float*, cudaStream_t s) {
-        return gemm_jet(np, out_act, 1, A, lda, W.hi, W.lo, C, ldc, jet_rows(M, d), N, K, e, s);
+        return gemm_jet(np, out_act, A, lda, W.hi, W.lo, C, ldc, jet_rows(M, d), N, K, e, s);
     }
 };
 template <> struct MM<__nv_bfloat16> : MMTC<__nv_bfloat16> {};
@@ -325,30 +325,29 @@ static int run_chunk(const Plan<Act>& p, int Bc, int precision, const float* P, 
         ldin = kXW;
     }
     const Act* H = xin;   // final embedding, logical row width kXW
-    // backflow (envelope_orbitals.py:46-75). Tensor-core tangent passes: one GEMM per spin over
-    // that spin's electron rows of every walker, so each row gets only its own spin's KN columns.
-    // Otherwise every row times [W_up | W_dn] and the envelope kernel takes the half that matches
-    // the electron's spin.
-    int ldbf = round_up(2 * d.KN, 4), spin_cols = d.KN;
+    // backflow (envelope_orbitals.py:46-75) and envelopes. Tensor-core tangent passes: one GEMM per spin
+    // over that spin's electron rows of every walker with the envelope in its epilogue. Otherwise
+    // every row times [W_up | W_dn], and the envelope kernel takes the half that matches the
+    // electron's spin.
     if (tang && pt >= 1) {
-        ldbf = d.KN;
-        spin_cols = 0;
         timer_begin("backflow_gemm", s);
         for (int spin = 0; spin < 2; ++spin) {
             const JetRows jr{Bc, d.n, d.T, spin == 0 ? d.nu : d.nd, spin == 0 ? 0 : d.nu};
             const int64_t wrow = (int64_t)spin * d.KN * d.D;           // W_up / W_dn rows of the K-major copy
-            DW_CHECK(gemm_jet(pt, 0, 0, H, kXW, pre.bf_bf[0] + wrow, pt >= 2 ? pre.bf_bf[1] + wrow : nullptr, p.BF, d.KN,
-                              jr, d.KN, d.D, GemmEpi(), s));
+            const EnvEpi env{r, R, Z, pre.sp_alpha + (int64_t)spin * d.N * d.KN, P + (spin == 0 ? L.weights_up : L.weights_dn),
+                             p.MO, d};
+            DW_CHECK(gemm_jet_env(pt, H, kXW, pre.bf_bf[0] + wrow, pt >= 2 ? pre.bf_bf[1] + wrow : nullptr, jr, d.D, env, s));
         }
         timer_end("backflow_gemm", s, 0.0, 0.0);
     } else {
+        const int ldbf = round_up(2 * d.KN, 4), spin_cols = d.KN;
         GemmEpi e0; e0.Tp = d.Tp; e0.rows_per_walker = d.n * d.Tp;
         WRef wb; wb.f32 = pre.bf_cat; wb.ldw = 2 * d.KN;
         if (pt >= 1) wb.hi = pre.bf_bf[0];
         if (pt >= 2) wb.lo = pre.bf_bf[1];
         DW_TIMED("backflow_gemm", DW_CHECK(MM<Act>::mm(H, kXW, wb, p.BF, ldbf, rows, 2 * d.KN, d.D, e0, s)));
+        DW_TIMED("envelope", launch_envelope(r, R, Z, P, L, pre.sp_alpha, d, Bc, p.BF, ldbf, spin_cols, p.MO, s));
     }
-    DW_TIMED("envelope", launch_envelope(r, R, Z, P, L, pre.sp_alpha, d, Bc, p.BF, ldbf, spin_cols, p.MO, s));
     if (det64_form(precision) && tang) {
         // FP64 LU, inverse and tangent traces of the FP32 Slater channels; the widened channels use
         // the backflow buffer (consumed by the envelope kernel, at least twice the Slater channels'

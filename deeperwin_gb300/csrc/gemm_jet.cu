@@ -1,5 +1,6 @@
 // Persistent tcgen05 GEMM of the tangent passes: the T = 3 n_el + 2 channel rows of each electron
-// (value, gradients, Laplacian) times the weights, with the forward-Laplacian tanh fused.
+// (value, gradients, Laplacian) times the weights, with the forward-Laplacian tanh fused (layers) or
+// the envelope orbitals (backflow: the Slater channels are written directly, not the backflow).
 //
 //   Y[(e, t), f] = epilogue( sum_k A[(e, t), k] W[f, k] )
 //
@@ -26,11 +27,17 @@
 // Bound by HBM: the layer of 16 electrons (K = 320, 409,600 rows) moves 943 MB in 204 us (4.6 TB/s, 69 %
 // of the measured copy rate; before, with rows as TMEM lanes, electrons padded to 64 rows and the jet
 // exchanged through shared memory, 390 us for the same rows), h_map (K = 256) 515 MB in 86 us (6.0 TB/s).
+// The envelope in the backflow's epilogue replaces a kernel that read the backflow back: backflow and
+// envelopes of a C2H4 local energy (4,096 walkers) 6.4 -> 4.0 ms, of 512 walkers at 40 electrons 23.1 ->
+// 13.4 ms; at 10 electrons and 10 ions, where a thread's envelope costs as much as its channels, 2.2 -> 2.35.
 // Every mbarrier wait is bounded; on timeout the kernel records an error flag, stops issuing, waits
 // (bounded) for its TMA loads in flight, frees its TMEM and returns.
 #include "gemm_tc.cuh"
 #include <algorithm>
 #include <type_traits>
+
+// lambdas that hold accumulator registers by reference: called out of line they would go through local memory
+#define DW_INLINE __attribute__((always_inline))
 
 namespace dw {
 
@@ -48,6 +55,7 @@ constexpr int kMaxStages = 8;
 
 struct JetArgs {
     int NF, K, nk;                                   // features, reduction width, stages per tile
+    int fpb;                                         // features per block (at most 128)
     int T, Tq, ept, ncol;                            // channel rows, their column pitch, electrons per tile, MMA N
     int n, ns, i0;                                   // electrons per walker; those taken: [i0, i0 + ns)
     int E;                                           // electrons in all (walkers * ns)
@@ -58,9 +66,11 @@ struct JetArgs {
     int single_load;                                 // a tile's rows are consecutive and unpadded
     int64_t rows;
     const float* bias; const float* rowbias;
-    void* C; int ldc;
+    void* C;
+    EnvEpi env;
     int* error;
 };
+enum Epilogue { kTanh, kEnvelope };
 
 // Position in the list of units.
 struct Unit {
@@ -69,10 +79,27 @@ struct Unit {
     __device__ void next(int ntiles) { if (++tile == ntiles) { tile = 0; ++group; } }
 };
 
-// Column chunks of one electron's accumulators: NV (8 or 16) TMEM columns from channel t0 on.
-template <int NV> __device__ __forceinline__ void tmem_ld(uint32_t taddr, float* v);
-template <> __device__ __forceinline__ void tmem_ld<16>(uint32_t taddr, float* v) { tmem_ld16(taddr, v); }
-template <> __device__ __forceinline__ void tmem_ld<8>(uint32_t taddr, float* v) { tmem_ld8(taddr, v); }
+// An electron's T accumulator columns, 16 at a time: mid(v, c) for every chunk but the last, last(v, c)
+// for that one. The next chunk's load is in flight while a chunk is worked on.
+template <class Mid, class Last>
+__device__ __forceinline__ void for_chunks(uint32_t col0, int T, Mid mid, Last last) {
+    float A[16], B[16];
+    const int lastc = (T - 1) / 16;
+    tmem_ld16(col0, A);
+    for (int c = 0;;) {
+        tmem_wait_ld16(A);
+        if (c == lastc) { last(A, c); break; }
+        tmem_ld16(col0 + 16 * (c + 1), B);
+        mid(A, c);
+        ++c;
+        tmem_wait_ld16(B);
+        if (c == lastc) { last(B, c); break; }
+        tmem_ld16(col0 + 16 * (c + 1), A);
+        mid(B, c);
+        ++c;
+    }
+    __syncwarp();
+}
 
 // Store of feature f of a row at o (row pitch LDC columns; split rows are [hi | lo]).
 template <int OUT, int LDC> struct RowOut;
@@ -125,22 +152,81 @@ struct Jet {
             sum = c < 2 ? s32 : __fadd_rn(sum, s32);
         }
         if (!fok) return;
+        const float cl = -2.f * y0 * d1 * sum;
         #pragma unroll
         for (int j = 0; j < NV; ++j) {
-            float y = d1 * v[j];
+            // (a branch on j == rem - 1 would index v dynamically, through local memory)
+            float y = LAST ? fmaf(d1, v[j], j == rem - 1 ? cl : 0.f) : d1 * v[j];
             if (FIRST && j == 0) y = fmaf(0.f, v[j], y0);
-            if (LAST && j == rem - 1) y = fmaf(d1, v[j], -2.f * y0 * d1 * sum);
             if (!LAST || j < rem) Row::put(o + j * Row::pitch, y);
         }
     }
 };
 
-// OUT: 0 = fp32, 1 = bf16, 2 = split-BF16. FL: forward-Laplacian tanh, else the plain product.
-// LDC: row pitch of C (0: a.ldc, plain product only). CG: CTAs per MMA. With CG = 2 a cluster of two
+// Electron i of walker b against the ions, ion `lane` per lane: difference vector and distance
+// (negative: no such ion, or padding of a packed geometry) and its reciprocal.
+struct Geo {
+    float s0, s1, s2, dd, inv;
+};
+// x / b from the correctly rounded reciprocal of b (P. W. Markstein, "Computation of elementary functions
+// on the IBM RISC System/6000 processor", IBM J. Res. Dev. 34, 1990: the quotient is correctly rounded
+// too, barring underflow): one reciprocal per (electron, ion) serves all orbital columns.
+__device__ __forceinline__ float quotient(float x, float b, float inv) {
+    const float q = x * inv;
+    return fmaf(fmaf(-q, b, x), inv, q);
+}
+__device__ __forceinline__ Geo geometry(const EnvEpi& p, int b, int i, int lane) {
+    const Dims& d = p.d;
+    Geo g{0.f, 0.f, 0.f, -1.f, -1.f};
+    if (lane < d.N) {
+        const float* ri = p.r + ((int64_t)b * d.n + i) * 3;
+        const int I = seg_of(d, b) * d.N + lane;
+        g.s0 = ri[0] - p.R[I * 3]; g.s1 = ri[1] - p.R[I * 3 + 1]; g.s2 = ri[2] - p.R[I * 3 + 2];
+        g.dd = p.Z[I] > 0 ? sqrtf(g.s0 * g.s0 + g.s1 * g.s1 + g.s2 * g.s2) : -1.f;
+        g.inv = 1.f / g.dd;
+    }
+    return g;
+}
+// The envelope of one orbital column (envelope_orbitals.py:96-127): value, gradient and Laplacian in
+// r_i. Called by a whole warp; two ions at a time, added in order.
+struct EnvValue {
+    float e, g[3], lap;
+};
+__device__ __forceinline__ EnvValue envelope_of(const EnvEpi& p, const Geo& geo, int col) {
+    const Dims& d = p.d;
+    float env = 0.f, g[3] = {0.f, 0.f, 0.f}, lapv = 0.f;
+    for (int I0 = 0; I0 < d.N; I0 += 2) {
+        float s0[2], s1[2], s2[2], dd[2], e[2], gs[2], q[2];
+        #pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            const int I = min(I0 + u, d.N - 1);
+            s0[u] = __shfl_sync(0xffffffffu, geo.s0, I);
+            s1[u] = __shfl_sync(0xffffffffu, geo.s1, I);
+            s2[u] = __shfl_sync(0xffffffffu, geo.s2, I);
+            dd[u] = __shfl_sync(0xffffffffu, geo.dd, I);
+            const float inv = __shfl_sync(0xffffffffu, geo.inv, I);
+            const float a = __ldg(p.sp_alpha + I * d.KN + col);
+            e[u] = __ldg(p.wts + I * d.KN + col) * expf(-a * dd[u]);
+            gs[u] = quotient(-a * e[u], dd[u], inv);
+            q[u] = __fsub_rn(__fmul_rn(a, a), quotient(2.f * a, dd[u], inv));
+        }
+        #pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            if (I0 + u >= d.N || dd[u] < 0.f) continue;
+            env += e[u];
+            g[0] = fmaf(gs[u], s0[u], g[0]); g[1] = fmaf(gs[u], s1[u], g[1]); g[2] = fmaf(gs[u], s2[u], g[2]);
+            lapv = fmaf(e[u], q[u], lapv);
+        }
+    }
+    return EnvValue{env, {g[0], g[1], g[2]}, lapv};
+}
+
+// OUT: 0 = fp32, 1 = bf16, 2 = split-BF16. EPI: forward-Laplacian tanh (C with row pitch LDC), or the
+// envelope (Slater channels). CG: CTAs per MMA. With CG = 2 a cluster of two
 // CTAs forms 256 features x 256 rows: each keeps the weights of 128 features and loads half of the
 // rows, so a stage is half as large for the same work; CTA 0 issues the MMAs, and the barriers it
 // waits on (full, wfull, tempty) count both CTAs.
-template <int NP, int OUT, bool FL, int LDC, int CG>
+template <int NP, int OUT, int EPI, int LDC, int CG>
 __global__ void __launch_bounds__(kThreads, 1)
 k_gemm_jet(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__ CUtensorMap tmA1,
            const __grid_constant__ CUtensorMap tmW0, const __grid_constant__ CUtensorMap tmW1, JetArgs a) {
@@ -208,11 +294,11 @@ k_gemm_jet(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__ CUt
                 for (int kt = 0; kt < nk; ++kt) {
                     uint8_t* dst = smem + (size_t)(kt * NP) * w_part;
                     if (CG == 2) {
-                        tma_load_2d_pair(dst, &tmW0, cta0_addr(wfull), kt * BK, blk * BM, lead);
-                        if (NP == 2) tma_load_2d_pair(dst + w_part, &tmW1, cta0_addr(wfull), kt * BK, blk * BM, lead);
+                        tma_load_2d_pair(dst, &tmW0, cta0_addr(wfull), kt * BK, blk * a.fpb, lead);
+                        if (NP == 2) tma_load_2d_pair(dst + w_part, &tmW1, cta0_addr(wfull), kt * BK, blk * a.fpb, lead);
                     } else {
-                        tma_load_2d(dst, &tmW0, wfull, kt * BK, blk * BM, lead);
-                        if (NP == 2) tma_load_2d(dst + w_part, &tmW1, wfull, kt * BK, blk * BM, lead);
+                        tma_load_2d(dst, &tmW0, wfull, kt * BK, blk * a.fpb, lead);
+                        if (NP == 2) tma_load_2d(dst + w_part, &tmW1, wfull, kt * BK, blk * a.fpb, lead);
                     }
                 }
                 wblk = blk;
@@ -311,42 +397,76 @@ k_gemm_jet(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__ CUt
         for (int64_t u = u0; u < u1; ++u, ++it, w.next(a.ntiles)) {
             if ((int)(it % kBufs) != buf) continue;
             const int blk = w.group * CG + rank, k0 = w.tile * CG * ept;
-            const int f = blk * BM + q * 32 + lane;
-            const bool fok = f < a.NF;
+            const int f = blk * a.fpb + q * 32 + lane;
+            const bool fok = q * 32 + lane < a.fpb && f < a.NF;
+            // geometry of the set's first electron, fetched while the accumulator is finished
+            Geo geo{0.f, 0.f, 0.f, -1.f, -1.f};
+            auto fetch = [&](int e) {
+                const int k = k0 + e, b = k / a.ns;
+                if (e < CG * ept && k < a.E) geo = geometry(a.env, b, a.i0 + k - b * a.ns, lane);
+            };
+            if (EPI == kEnvelope) fetch(h / kBufs);
             const bool ready = mbar_wait(&tfull[buf], (it / kBufs) & 1);
             if (!ready && lane == 0) s_set_err[h] = 1;
             asm volatile("bar.sync %0, 128;" ::"r"(1 + h) : "memory");      // the set agrees before leaving
             if (*(volatile int*)&s_set_err[h]) { if (lane == 0) atomicExch(&s_err, 1); break; }
             tc_fence_after();
-            if (blk * BM + q * 32 < a.NF) {
-                const float bias = FL && a.bias && fok ? __ldg(a.bias + f) : 0.f;
+            if (q * 32 < a.fpb && blk * a.fpb + q * 32 < a.NF) {
+                const float bias = EPI == kTanh && a.bias && fok ? __ldg(a.bias + f) : 0.f;
                 for (int e = h / kBufs; e < CG * ept && k0 + e < a.E; e += kSets / kBufs) {
-                    const int k = k0 + e, b = k / a.ns;
-                    const int64_t row0 = (int64_t)(b * a.n + a.i0 + k - b * a.ns) * T;
+                    const int k = k0 + e, b = k / a.ns, i = a.i0 + k - b * a.ns;
                     const uint32_t col0 = tmem + ((uint32_t)(q * 32) << 16) + buf * kBufCols +
                                           (CG == 2 && e >= ept ? a.ncol + (e - ept) * a.Tq : e * a.Tq);
-                    if constexpr (!FL) {
-                        float* o = static_cast<float*>(a.C) + row0 * a.ldc + f;
-                        for (int t0 = 0; t0 < T; t0 += 8) {
-                            float v[8];
-                            tmem_ld8(col0 + t0, v);
-                            tmem_wait_ld();
-                            if (fok) {
-                                #pragma unroll
-                                for (int j = 0; j < 8; ++j) {
-                                    if (t0 + j < T) *o = v[j];
-                                    o += a.ldc;
+                    if constexpr (EPI == kEnvelope) {
+                        const Dims& d = a.env.d;
+                        const EnvValue ev = envelope_of(a.env, geo, min(f, a.NF - 1));
+                        fetch(e + kSets / kBufs);                    // the next electron's, behind this one's stores
+                        const int n2 = d.n * d.n, ko = f / d.n, own = 1 + 3 * i;
+                        float* mo = a.env.MO + ((int64_t)b * d.K + ko) * T * n2 + i * d.n + f - ko * d.n;
+                        float bf0 = 0.f, bo[3] = {0.f, 0.f, 0.f};    // backflow value and own-coordinate rows
+                        // rem: channels from 16 c on (the last chunk has the Laplacian at rem - 1)
+                        auto general = [&](const float (&v)[16], int c, int rem) DW_INLINE {
+                            #pragma unroll
+                            for (int j = 0; j < 16; ++j) {
+                                if (j >= rem) break;
+                                float x = ev.e * v[j];
+                                const unsigned o3 = (unsigned)(16 * c + j - own);
+                                if (o3 < 3u) {
+                                    x = fmaf(o3 == 0 ? ev.g[0] : (o3 == 1 ? ev.g[1] : ev.g[2]), bf0, x);
+                                    if (o3 == 0) bo[0] = v[j];
+                                    else if (o3 == 1) bo[1] = v[j];
+                                    else bo[2] = v[j];
+                                } else if (j == rem - 1 && 16 * c + j == T - 1) {
+                                    x = fmaf(ev.lap, bf0, x);
+                                    #pragma unroll
+                                    for (int k3 = 0; k3 < 3; ++k3) x = fmaf(2.f * ev.g[k3], bo[k3], x);
                                 }
+                                mo[j * n2] = x;
                             }
-                            __syncwarp();
-                        }
+                        };
+                        for_chunks(col0, T,
+                            [&](const float (&v)[16], int c) DW_INLINE {
+                                if (c == 0) bf0 = v[0];
+                                if (!fok) return;
+                                if (own >= 16 * (c + 1) || own + 3 <= 16 * c) {
+                                    #pragma unroll
+                                    for (int j = 0; j < 16; ++j) mo[j * n2] = ev.e * v[j];
+                                } else {
+                                    general(v, c, 16);
+                                }
+                                mo += 16 * n2;
+                            },
+                            [&](const float (&v)[16], int c) DW_INLINE {
+                                if (c == 0) bf0 = v[0];
+                                if (fok) general(v, c, T - 16 * c);
+                            });
                     } else {
                         // the row bias of the next chunk is fetched while this one is worked on
                         const bool has_rb = a.rowbias && fok;
                         const float* rb = has_rb ? a.rowbias + (int64_t)b * T * kLdRb + f : nullptr;
-                        typename Row::T* o = static_cast<typename Row::T*>(a.C) + row0 * Row::pitch + f;
+                        typename Row::T* o = static_cast<typename Row::T*>(a.C) + (int64_t)(b * a.n + i) * T * Row::pitch + f;
                         float rv[16];
-                        auto load_rb = [&](int t0) {
+                        auto load_rb = [&](int t0) DW_INLINE {
                             if (t0 + 16 <= T) {
                                 #pragma unroll
                                 for (int j = 0; j < 16; ++j) rv[j] = has_rb ? __ldg(rb + j * kLdRb) : 0.f;
@@ -358,33 +478,29 @@ k_gemm_jet(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__ CUt
                         };
                         load_rb(0);
                         Jet<OUT, LDC> jet;
-                        auto step = [&](auto nv, auto first, auto last, int c) {
+                        using std::integral_constant;
+                        using std::true_type;
+                        using std::false_type;
+                        auto step = [&](float (&v)[16], auto nv, auto first, auto last, int c) DW_INLINE {
                             constexpr int NV = decltype(nv)::value;
-                            float v[16];
-                            tmem_ld<NV>(col0 + 16 * c, v);
-                            tmem_wait_ld();
                             #pragma unroll
                             for (int j = 0; j < NV; ++j) v[j] += rv[j];
                             if (!decltype(last)::value) load_rb(16 * (c + 1));
                             jet.template chunk<NV, decltype(first)::value, decltype(last)::value>(v, c, T - 16 * c, bias, fok, o);
                             o += 16 * Row::pitch;
-                            __syncwarp();
                         };
-                        using std::integral_constant;
-                        using std::true_type;
-                        using std::false_type;
                         const integral_constant<int, 16> n16;
                         const integral_constant<int, 8> n8;
-                        const int lastc = (T - 1) / 16, tail = T - 16 * lastc;      // tail: 1 .. 16 channels
-                        if (lastc == 0) {
-                            if (tail > 8) step(n16, true_type(), true_type(), 0);
-                            else step(n8, true_type(), true_type(), 0);
-                        } else {
-                            step(n16, true_type(), false_type(), 0);
-                            for (int c = 1; c < lastc; ++c) step(n16, false_type(), false_type(), c);
-                            if (tail > 8) step(n16, false_type(), true_type(), lastc);
-                            else step(n8, false_type(), true_type(), lastc);
-                        }
+                        for_chunks(col0, T,
+                            [&](float (&v)[16], int c) DW_INLINE {
+                                if (c == 0) step(v, n16, true_type(), false_type(), c);
+                                else step(v, n16, false_type(), false_type(), c);
+                            },
+                            [&](float (&v)[16], int c) DW_INLINE {
+                                if (c == 0) step(v, n16, true_type(), true_type(), c);
+                                else if (T - 16 * c > 8) step(v, n16, false_type(), true_type(), c);
+                                else step(v, n8, false_type(), true_type(), c);
+                            });
                     }
                 }
             }
@@ -406,9 +522,9 @@ k_gemm_jet(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__ CUt
     }
 }
 
-template <int NP, int OUT, bool FL, int LDC, int CG>
-int launch_jet_cg(const __nv_bfloat16* A, int lda, const __nv_bfloat16* W0, const __nv_bfloat16* W1, void* C, int ldc,
-               const JetRows& r, int NF, int K, const GemmEpi& epi, cudaStream_t s) {
+template <int NP, int OUT, int EPI, int LDC, int CG>
+int launch_jet_cg(const __nv_bfloat16* A, int lda, const __nv_bfloat16* W0, const __nv_bfloat16* W1, void* C,
+                  const JetRows& r, int NF, int K, const GemmEpi& epi, const EnvEpi* env, cudaStream_t s) {
     if (r.nw <= 0 || r.ns <= 0) return DW_OK;
     if (r.T < 1 || r.T > 128 || NF <= 0 || K <= 0 || (epi.rowbias && epi.ldrb != kLdRb)) return DW_ERR_ARG;
     JetArgs a;
@@ -418,7 +534,8 @@ int launch_jet_cg(const __nv_bfloat16* A, int lda, const __nv_bfloat16* W0, cons
     a.rows = (int64_t)r.nw * r.n * r.T;
     a.single_load = a.T == a.Tq && a.ns == a.n;
     a.bias = epi.bias; a.rowbias = epi.rowbias;
-    a.C = C; a.ldc = ldc;
+    a.C = C;
+    if (env) a.env = *env;
     a.error = tc_error_flag();
     if (!a.error) return DW_ERR_CUDA;
     // A part of a stage: whole 1024-byte swizzle atoms of 8 rows; the MMA reads ncol rows. A part of a
@@ -431,8 +548,12 @@ int launch_jet_cg(const __nv_bfloat16* A, int lda, const __nv_bfloat16* W0, cons
     // features at K = 256)
     int stage = 0;
     for (int cap = kTileRows / CG; cap >= 128; cap -= 128) {
-        a.ept = cap / a.Tq;
-        a.ncol = round_up(a.ept * a.Tq, 16);
+        // the last electron's chunks of 16 columns end within the buffer
+        const int last = round_up(a.T, 16);
+        for (a.ept = cap / a.Tq;; --a.ept) {
+            a.ncol = round_up(a.ept * a.Tq, 16);
+            if ((CG - 1) * a.ncol + (a.ept - 1) * a.Tq + last <= kBufCols) break;
+        }
         a.x_part = a.ncol * BK * 2;
         stage = NP * a.x_part;
         a.stages = std::min(kMaxStages, (227 * 1024 - fixed - w_bytes) / stage);
@@ -440,7 +561,10 @@ int launch_jet_cg(const __nv_bfloat16* A, int lda, const __nv_bfloat16* W0, cons
     }
     if (a.stages < 2) return DW_ERR_ARCH;
     a.ntiles = (a.E + CG * a.ept - 1) / (CG * a.ept);
-    a.units = (int64_t)a.ntiles * ((NF + CG * BM - 1) / (CG * BM));
+    // the features spread evenly over the blocks, so that the CTAs of a pair have equal epilogues
+    const int groups = (NF + CG * BM - 1) / (CG * BM);
+    a.fpb = round_up((NF + groups * CG - 1) / (groups * CG), 8);
+    a.units = (int64_t)a.ntiles * groups;
     const int Kp = round_up(K, 64), box = a.single_load ? a.ept * a.T : a.T;
     CUtensorMap ma0, ma1, mw0, mw1;
     DW_CHECK(make_map(&ma0, A, a.rows, K, (int64_t)NP * lda, BK, box, false));
@@ -451,7 +575,7 @@ int launch_jet_cg(const __nv_bfloat16* A, int lda, const __nv_bfloat16* W0, cons
         DW_CHECK(make_map(&mw1, W1, NF, K, Kp, BK, w_rows, false));
     }
     const size_t smem = (size_t)fixed + w_bytes + (size_t)a.stages * stage;
-    auto kern = k_gemm_jet<NP, OUT, FL, LDC, CG>;
+    auto kern = k_gemm_jet<NP, OUT, EPI, LDC, CG>;
     DW_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(CG * std::min<int64_t>(a.units, num_sms() / CG)));
@@ -468,28 +592,34 @@ int launch_jet_cg(const __nv_bfloat16* A, int lda, const __nv_bfloat16* W0, cons
     return DW_OK;
 }
 
-template <int NP, int OUT, bool FL, int LDC>
-int launch_jet(const __nv_bfloat16* A, int lda, const __nv_bfloat16* W0, const __nv_bfloat16* W1, void* C, int ldc,
-               const JetRows& r, int NF, int K, const GemmEpi& epi, cudaStream_t s) {
+template <int NP, int OUT, int EPI, int LDC>
+int launch_jet(const void* A, int lda, const __nv_bfloat16* W0, const __nv_bfloat16* W1, void* C, const JetRows& r, int NF,
+               int K, const GemmEpi& epi, const EnvEpi* env, cudaStream_t s) {
+    const __nv_bfloat16* a = reinterpret_cast<const __nv_bfloat16*>(A);
     // pairs of CTAs where there is more than one block of 128 features
-    if (NF > BM) return launch_jet_cg<NP, OUT, FL, LDC, 2>(A, lda, W0, W1, C, ldc, r, NF, K, epi, s);
-    return launch_jet_cg<NP, OUT, FL, LDC, 1>(A, lda, W0, W1, C, ldc, r, NF, K, epi, s);
+    if (NF > BM) return launch_jet_cg<NP, OUT, EPI, LDC, 2>(a, lda, W0, W1, C, r, NF, K, epi, env, s);
+    return launch_jet_cg<NP, OUT, EPI, LDC, 1>(a, lda, W0, W1, C, r, NF, K, epi, env, s);
 }
 
 }  // namespace
 
-int gemm_jet(int np, int out, int fl, const void* A, int lda, const __nv_bfloat16* W0, const __nv_bfloat16* W1, void* C,
+int gemm_jet(int np, int out, const void* A, int lda, const __nv_bfloat16* W0, const __nv_bfloat16* W1, void* C,
              int ldc, const JetRows& r, int NF, int K, const GemmEpi& epi, cudaStream_t s) {
-    const __nv_bfloat16* a = reinterpret_cast<const __nv_bfloat16*>(A);
     // row pitches of the layer input (320), the Jastrow layers (64) and h_map (32)
-    if (np == 2 && out == 2 && fl && ldc == 320) return launch_jet<2, 2, true, 320>(a, lda, W0, W1, C, ldc, r, NF, K, epi, s);
-    if (np == 2 && out == 2 && fl && ldc == 64) return launch_jet<2, 2, true, 64>(a, lda, W0, W1, C, ldc, r, NF, K, epi, s);
-    if (np == 2 && out == 0 && fl && ldc == 32) return launch_jet<2, 0, true, 32>(a, lda, W0, W1, C, ldc, r, NF, K, epi, s);
-    if (np == 2 && out == 0 && !fl) return launch_jet<2, 0, false, 0>(a, lda, W0, W1, C, ldc, r, NF, K, epi, s);
-    if (np == 1 && out == 1 && fl && ldc == 320) return launch_jet<1, 1, true, 320>(a, lda, W0, W1, C, ldc, r, NF, K, epi, s);
-    if (np == 1 && out == 1 && fl && ldc == 64) return launch_jet<1, 1, true, 64>(a, lda, W0, W1, C, ldc, r, NF, K, epi, s);
-    if (np == 1 && out == 0 && fl && ldc == 32) return launch_jet<1, 0, true, 32>(a, lda, W0, W1, C, ldc, r, NF, K, epi, s);
-    if (np == 1 && out == 0 && !fl) return launch_jet<1, 0, false, 0>(a, lda, W0, W1, C, ldc, r, NF, K, epi, s);
+    if (np == 2 && out == 2 && ldc == 320) return launch_jet<2, 2, kTanh, 320>(A, lda, W0, W1, C, r, NF, K, epi, nullptr, s);
+    if (np == 2 && out == 2 && ldc == 64) return launch_jet<2, 2, kTanh, 64>(A, lda, W0, W1, C, r, NF, K, epi, nullptr, s);
+    if (np == 2 && out == 0 && ldc == 32) return launch_jet<2, 0, kTanh, 32>(A, lda, W0, W1, C, r, NF, K, epi, nullptr, s);
+    if (np == 1 && out == 1 && ldc == 320) return launch_jet<1, 1, kTanh, 320>(A, lda, W0, W1, C, r, NF, K, epi, nullptr, s);
+    if (np == 1 && out == 1 && ldc == 64) return launch_jet<1, 1, kTanh, 64>(A, lda, W0, W1, C, r, NF, K, epi, nullptr, s);
+    if (np == 1 && out == 0 && ldc == 32) return launch_jet<1, 0, kTanh, 32>(A, lda, W0, W1, C, r, NF, K, epi, nullptr, s);
+    return DW_ERR_ARG;
+}
+
+int gemm_jet_env(int np, const void* A, int lda, const __nv_bfloat16* W0, const __nv_bfloat16* W1, const JetRows& r, int K,
+                 const EnvEpi& env, cudaStream_t s) {
+    const int NF = env.d.KN;
+    if (np == 2) return launch_jet<2, 0, kEnvelope, 1>(A, lda, W0, W1, nullptr, r, NF, K, GemmEpi(), &env, s);
+    if (np == 1) return launch_jet<1, 0, kEnvelope, 1>(A, lda, W0, W1, nullptr, r, NF, K, GemmEpi(), &env, s);
     return DW_ERR_ARG;
 }
 
@@ -498,13 +628,13 @@ int gemm_jet(int np, int out, int fl, const void* A, int lda, const __nv_bfloat1
 extern "C" {
 
 // Test hook: gemm_jet on split-BF16 rows (np = 2); out 0 (fp32) or 2 (split-BF16).
-int dw_debug_gemm_jet(int out, int fl, const void* A, int lda, const void* W0, const void* W1, void* C, int ldc, int nw,
+int dw_debug_gemm_jet(int out, const void* A, int lda, const void* W0, const void* W1, void* C, int ldc, int nw,
                       int n, int T, int ns, int i0, int NF, int K, const float* bias, const float* rowbias, void* stream) {
     using namespace dw;
     if (!tc_available()) return DW_ERR_UNSUPPORTED;
     GemmEpi e;
     e.bias = bias; e.rowbias = rowbias; e.ldrb = 256; e.Tp = T;
-    return gemm_jet(2, out, fl, A, lda, (const __nv_bfloat16*)W0, (const __nv_bfloat16*)W1, C, ldc,
+    return gemm_jet(2, out, A, lda, (const __nv_bfloat16*)W0, (const __nv_bfloat16*)W1, C, ldc,
                     JetRows{nw, n, T, ns, i0}, NF, K, e, (cudaStream_t)stream);
 }
 

@@ -26,10 +26,21 @@ int gemm_tc(int np, int out, const void* A, int lda, const __nv_bfloat16* W0, co
 struct JetRows {
     int nw, n, T, ns, i0;
 };
-// C[(e, t), f] over those rows (the same rows of A and C): fl = 1 with bias (value rows), row bias (one row
-// per walker and channel) and the forward-Laplacian tanh over each electron's T rows; fl = 0 the plain
-// product. np, out and the strides as for gemm_tc; no alignment is asked of C. T <= 128.
-int gemm_jet(int np, int out, int fl, const void* A, int lda, const __nv_bfloat16* W0, const __nv_bfloat16* W1, void* C,
+// C[(e, t), f] over those rows (the same rows of A and C) with bias (value rows), row bias (one row per
+// walker and channel) and the forward-Laplacian tanh over each electron's T rows. np, out and the
+// strides as for gemm_tc; no alignment is asked of C. T <= 128.
+int gemm_jet(int np, int out, const void* A, int lda, const __nv_bfloat16* W0, const __nv_bfloat16* W1, void* C,
              int ldc, const JetRows& rows, int NF, int K, const GemmEpi& epi, cudaStream_t s);
+
+// Backflow of one spin's rows times the envelope, straight into the Slater channels: features are the
+// orbital columns (k, o), MO[b][k][t][i][o] = env[i, (k, o)] * bf[(b, i, t), (k, o)] with the product rule.
+struct EnvEpi {
+    const float* r; const float* R; const int32_t* Z;       // walkers, nuclei (per geometry segment)
+    const float* sp_alpha; const float* wts;                // this spin's softplus(alpha), weights [N][KN]
+    float* MO;
+    Dims d;
+};
+int gemm_jet_env(int np, const void* A, int lda, const __nv_bfloat16* W0, const __nv_bfloat16* W1, const JetRows& rows,
+                 int K, const EnvEpi& env, cudaStream_t s);
 
 }  // namespace dw

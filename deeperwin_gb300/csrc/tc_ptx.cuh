@@ -164,6 +164,13 @@ __device__ __forceinline__ void tmem_ld8(uint32_t taddr, float* v) {
     #pragma unroll
     for (int j = 0; j < 8; ++j) v[j] = __uint_as_float(r[j]);
 }
+// Waits for this thread's TMEM loads; v passes through, so that nothing reads it earlier.
+__device__ __forceinline__ void tmem_wait_ld16(float (&v)[16]) {
+    asm volatile("tcgen05.wait::ld.sync.aligned;"
+                 : "+f"(v[0]), "+f"(v[1]), "+f"(v[2]), "+f"(v[3]), "+f"(v[4]), "+f"(v[5]), "+f"(v[6]), "+f"(v[7]),
+                   "+f"(v[8]), "+f"(v[9]), "+f"(v[10]), "+f"(v[11]), "+f"(v[12]), "+f"(v[13]), "+f"(v[14]), "+f"(v[15])
+                 :: "memory");
+}
 __device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
 }  // namespace dw
