@@ -180,14 +180,156 @@ k_gemm_f32v(const float* __restrict__ A, int lda, const float* __restrict__ W, i
     }
 }
 
-static bool vec_ok(const float* A, int lda, const float* W, int ldw, int N, int K, bool trans_w) {
+// Small grids. Every output of these kernels is one chain of FMAs over k = 0 .. K - 1 from zero, so all tile
+// shapes give the same bits and the shape is chosen by the grid alone.
+//
+// BM x BN tiles with a 4 x 4 patch per thread, 16-deep K slices double-buffered through registers (same
+// operand conditions as k_gemm_f32v, any N a multiple of 4): for matrices that 128 x 128 tiles would
+// spread over too few SMs.
+template <int BM, int BN>
+__global__ void __launch_bounds__(BM * BN / 16)
+k_gemm_f32s(const float* __restrict__ A, int lda, const float* __restrict__ W, int ldw, float* __restrict__ C, int ldc,
+            int M, int N, int K, GemmEpi epi) {
+    constexpr int BK = 16, NT = BM * BN / 16, TC = BN / 4;
+    constexpr int LA = BM * BK / 4 / NT, LW = BN * BK / 4 / NT;         // float4 loads per thread and slice
+    __shared__ __align__(16) float As[2][BK][BM + 4];
+    __shared__ __align__(16) float Ws[2][BK][BN];
+    const int tid = threadIdx.x, tr = tid / TC, tc = tid % TC;
+    const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
+    float acc[4][4];
+    #pragma unroll
+    for (int i = 0; i < 4; ++i)
+        #pragma unroll
+        for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
+    float4 ra[LA], rw[LW];
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    auto gload = [&](int k0) {
+        #pragma unroll
+        for (int u = 0; u < LA; ++u) {
+            const int e = tid + u * NT, gm = m0 + e / (BK / 4), gk = k0 + e % (BK / 4) * 4;
+            ra[u] = (gm < M && gk < K) ? __ldg(reinterpret_cast<const float4*>(A + (int64_t)gm * lda + gk)) : zero;
+        }
+        #pragma unroll
+        for (int u = 0; u < LW; ++u) {
+            const int e = tid + u * NT, gk = k0 + e / (BN / 4), gn = n0 + e % (BN / 4) * 4;
+            rw[u] = (gk < K && gn < N) ? __ldg(reinterpret_cast<const float4*>(W + (int64_t)gk * ldw + gn)) : zero;
+        }
+    };
+    auto sstore = [&](int buf) {
+        #pragma unroll
+        for (int u = 0; u < LA; ++u) {
+            const int e = tid + u * NT, r = e / (BK / 4), k = e % (BK / 4) * 4;
+            As[buf][k][r] = ra[u].x; As[buf][k + 1][r] = ra[u].y; As[buf][k + 2][r] = ra[u].z; As[buf][k + 3][r] = ra[u].w;
+        }
+        #pragma unroll
+        for (int u = 0; u < LW; ++u) {
+            const int e = tid + u * NT;
+            *reinterpret_cast<float4*>(&Ws[buf][e / (BN / 4)][e % (BN / 4) * 4]) = rw[u];
+        }
+    };
+    const int nk = (K + BK - 1) / BK;
+    gload(0);
+    sstore(0);
+    __syncthreads();
+    for (int kt = 0; kt < nk; ++kt) {
+        const int buf = kt & 1;
+        if (kt + 1 < nk) gload((kt + 1) * BK);
+        #pragma unroll
+        for (int kk = 0; kk < BK; ++kk) {
+            const float4 a4 = *reinterpret_cast<const float4*>(&As[buf][kk][4 * tr]);
+            const float4 w4 = *reinterpret_cast<const float4*>(&Ws[buf][kk][4 * tc]);
+            const float a[4] = {a4.x, a4.y, a4.z, a4.w}, w[4] = {w4.x, w4.y, w4.z, w4.w};
+            #pragma unroll
+            for (int i = 0; i < 4; ++i)
+                #pragma unroll
+                for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(a[i], w[j], acc[i][j]);
+        }
+        if (kt + 1 < nk) sstore(buf ^ 1);
+        __syncthreads();
+    }
+    #pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int m = m0 + 4 * tr + i;
+        if (m >= M) continue;
+        const int t = m % epi.Tp;
+        const float* rb = epi.rowbias ? epi.rowbias + ((int64_t)(m / epi.rows_per_walker) * epi.Tp + t) * epi.ldrb : nullptr;
+        #pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const int n = n0 + 4 * tc + j;
+            if (n >= N) continue;
+            float v = acc[i][j];
+            if (epi.bias && t == 0) v += epi.bias[n];
+            if (rb) v += rb[n];
+            if (epi.act == 1) v = tanhf(v);
+            C[(int64_t)m * ldc + n] = v;
+        }
+    }
+}
+
+// A few rows: block of 8 rows x 32 columns, one output per thread (warp per row), the K x 32 weight slice
+// and the rows staged in shared memory by all threads at once, so that the launch waits for one round of
+// loads and one FMA chain.
+constexpr int kTinyK = 512, kTinyM = 64;
+__global__ void __launch_bounds__(256)
+k_gemm_f32_tiny(const float* __restrict__ A, int lda, const float* __restrict__ W, int ldw, float* __restrict__ C, int ldc,
+                int M, int N, int K, GemmEpi epi) {
+    extern __shared__ __align__(16) float tiny_smem[];
+    float* Ws = tiny_smem;                                              // [K][32]
+    float* As = tiny_smem + K * 32;                                     // [8][K]
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int m0 = blockIdx.y * 8, n0 = blockIdx.x * 32;
+    #pragma unroll 8
+    for (int e = tid; e < K * 32; e += 256) {
+        const int n = n0 + (e & 31);
+        Ws[e] = n < N ? __ldg(W + (int64_t)(e >> 5) * ldw + n) : 0.f;
+    }
+    for (int r = 0; r < min(8, M - m0); ++r)
+        for (int k = tid; k < K; k += 256) As[r * K + k] = __ldg(A + (int64_t)(m0 + r) * lda + k);
+    __syncthreads();
+    const int m = m0 + warp, n = n0 + lane;
+    if (m >= M) return;
+    float acc = 0.f;
+    #pragma unroll 16
+    for (int k = 0; k < K; ++k) acc = fmaf(As[warp * K + k], Ws[k * 32 + lane], acc);
+    if (n >= N) return;
+    const int t = m % epi.Tp;
+    if (epi.bias && t == 0) acc += epi.bias[n];
+    if (epi.rowbias) acc += epi.rowbias[((int64_t)(m / epi.rows_per_walker) * epi.Tp + t) * epi.ldrb + n];
+    if (epi.act == 1) acc = tanhf(acc);
+    C[(int64_t)m * ldc + n] = acc;
+}
+
+static bool operands_ok(const float* A, int lda, const float* W, int ldw, int N, int K, bool trans_w) {
     auto al = [](const void* p) { return ((uintptr_t)p & 15) == 0; };
-    return N >= 128 && K % 4 == 0 && lda % 4 == 0 && ldw % 4 == 0 && al(A) && al(W) && (trans_w || N % 4 == 0);
+    return K % 4 == 0 && lda % 4 == 0 && ldw % 4 == 0 && al(A) && al(W) && (trans_w || N % 4 == 0);
+}
+static bool vec_ok(const float* A, int lda, const float* W, int ldw, int N, int K, bool trans_w) {
+    return N >= 128 && operands_ok(A, lda, W, ldw, N, K, trans_w);
 }
 
 void gemm_f32(const float* A, int lda, const float* W, int ldw, float* C, int ldc, int M, int N, int K,
               const GemmEpi& epi, int batch, int64_t sA, int64_t sC, cudaStream_t s) {
     if (M <= 0 || N <= 0) return;
+    // Tile by the grid: a few rows (a single walker's launches are load latency and one FMA chain); 64 x 64
+    // (64 x 32 for N <= 32) where 128-row tiles give less than two blocks per SM (2,048 LiH walkers: the
+    // layers' 8,192 x 256 are 128 blocks, the spin means' 2,048 x 256 only 32); larger tiles reuse more
+    // per shared load. Measured: log psi^2 of one LiH walker 579 -> 229 us; 2,048 walkers, per launch: spin
+    // means 62 -> 27 us, layers 45 -> 43 us, h_map 24 -> 16 us, Jastrow 62 -> 35 us.
+    if (batch == 1 && M <= kTinyM && K <= kTinyK) {
+        const size_t sm = (size_t)K * (32 + 8) * sizeof(float);
+        if (sm > 48 * 1024) cudaFuncSetAttribute(k_gemm_f32_tiny, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+        k_gemm_f32_tiny<<<dim3((N + 31) / 32, (M + 7) / 8), 256, sm, s>>>(A, lda, W, ldw, C, ldc, M, N, K, epi);
+        count_launch();
+        return;
+    }
+    const bool narrow = N <= 32;
+    const int64_t big = (int64_t)((M + 127) / 128) * ((N + 127) / 128);
+    if (batch == 1 && big < 2 * num_sms_simt() && operands_ok(A, lda, W, ldw, N, K, false)) {
+        if (narrow) k_gemm_f32s<64, 32><<<dim3(1, (M + 63) / 64), 128, 0, s>>>(A, lda, W, ldw, C, ldc, M, N, K, epi);
+        else k_gemm_f32s<64, 64><<<dim3((N + 63) / 64, (M + 63) / 64), 256, 0, s>>>(A, lda, W, ldw, C, ldc, M, N, K, epi);
+        count_launch();
+        return;
+    }
     if (vec_ok(A, lda, W, ldw, N, K, false) && (batch == 1 || (sA % 4 == 0))) {
         dim3 g((N + 127) / 128, (M + 127) / 128, batch);
         k_gemm_f32v<false, false><<<g, 256, 0, s>>>(A, lda, W, ldw, C, ldc, M, N, K, epi, sA, sC);
