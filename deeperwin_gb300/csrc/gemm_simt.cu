@@ -18,6 +18,15 @@ static int num_sms_simt() {
     return n;
 }
 
+// Two FP32 FMAs in one instruction (each rounded as fmaf).
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+    float2 d;
+    asm("{\n .reg .b64 x, y, z;\n mov.b64 x, {%2, %3};\n mov.b64 y, {%4, %5};\n mov.b64 z, {%6, %7};\n"
+        " fma.rn.f32x2 z, x, y, z;\n mov.b64 {%0, %1}, z;\n}\n"
+        : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+    return d;
+}
+
 template <int BM, int BN, int BK, int TM, int TN, bool TRANS_W = false, bool ACC = false>
 __global__ void __launch_bounds__((BM / TM) * (BN / TN))
 k_gemm_f32(const float* __restrict__ A, int lda, const float* __restrict__ W, int ldw, float* __restrict__ C, int ldc,
@@ -96,7 +105,7 @@ k_gemm_f32(const float* __restrict__ A, int lda, const float* __restrict__ W, in
 // warp's 16-byte shared reads are consecutive: 4 LDS.128 feed 64 FMAs), 16-byte global loads
 // staged through registers into double-buffered shared memory. Same epilogue as k_gemm_f32.
 template <bool TRANS_W, bool ACC>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, 2)
 k_gemm_f32v(const float* __restrict__ A, int lda, const float* __restrict__ W, int ldw, float* __restrict__ C, int ldc,
             int M, int N, int K, GemmEpi epi, int64_t sA, int64_t sC) {
     constexpr int BM = 128, BN = 128, BK = 8;
@@ -106,11 +115,11 @@ k_gemm_f32v(const float* __restrict__ A, int lda, const float* __restrict__ W, i
     __shared__ __align__(16) float Ws[2][BK][BN];
     const int tid = threadIdx.x, tr = tid / 16, tc = tid % 16;
     const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
-    float acc[8][8];
+    float2 acc[8][4];                                      // column pairs
     #pragma unroll
     for (int i = 0; i < 8; ++i)
         #pragma unroll
-        for (int j = 0; j < 8; ++j) acc[i][j] = 0.f;
+        for (int j = 0; j < 4; ++j) acc[i][j] = make_float2(0.f, 0.f);
     // per thread: one float4 of A (row tid / 2, k half tid % 2) and one of W
     const int ar = tid / 2, ah = (tid % 2) * 4;
     const int wk = tid / 32, wn = (tid % 32) * 4;          // non-transposed W: [K][N]
@@ -151,11 +160,11 @@ k_gemm_f32v(const float* __restrict__ A, int lda, const float* __restrict__ W, i
             const float4 b0 = *reinterpret_cast<const float4*>(&Ws[buf][kk][4 * tc]);
             const float4 b1 = *reinterpret_cast<const float4*>(&Ws[buf][kk][64 + 4 * tc]);
             const float a[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
-            const float b[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
+            const float2 b[4] = {make_float2(b0.x, b0.y), make_float2(b0.z, b0.w), make_float2(b1.x, b1.y), make_float2(b1.z, b1.w)};
             #pragma unroll
             for (int i = 0; i < 8; ++i)
                 #pragma unroll
-                for (int j = 0; j < 8; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
+                for (int j = 0; j < 4; ++j) acc[i][j] = fma2(make_float2(a[i], a[i]), b[j], acc[i][j]);
         }
         if (kt + 1 < nk) sstore(buf ^ 1);
         __syncthreads();
@@ -170,7 +179,7 @@ k_gemm_f32v(const float* __restrict__ A, int lda, const float* __restrict__ W, i
         for (int j = 0; j < 8; ++j) {
             const int n = n0 + (j < 4 ? 4 * tc + j : 64 + 4 * tc + j - 4);
             if (n >= N) continue;
-            float v = acc[i][j];
+            float v = j % 2 ? acc[i][j / 2].y : acc[i][j / 2].x;
             if (epi.bias && t == 0) v += epi.bias[n];
             if (rb) v += rb[n];
             if (epi.act == 1) v = tanhf(v);
@@ -183,24 +192,22 @@ k_gemm_f32v(const float* __restrict__ A, int lda, const float* __restrict__ W, i
 // Small grids. Every output of these kernels is one chain of FMAs over k = 0 .. K - 1 from zero, so all tile
 // shapes give the same bits and the shape is chosen by the grid alone.
 //
-// BM x BN tiles with a 4 x 4 patch per thread, 16-deep K slices double-buffered through registers (same
+// BM x BN tiles with a TM x 4 patch per thread (TM = 8: two 4-row groups), 16-deep K slices double-buffered through registers (same
 // operand conditions as k_gemm_f32v, any N a multiple of 4): for matrices that 128 x 128 tiles would
 // spread over too few SMs.
-template <int BM, int BN>
-__global__ void __launch_bounds__(BM * BN / 16)
+template <int BM, int BN, int TM>
+__global__ void __launch_bounds__(BM * BN / 4 / TM)
 k_gemm_f32s(const float* __restrict__ A, int lda, const float* __restrict__ W, int ldw, float* __restrict__ C, int ldc,
             int M, int N, int K, GemmEpi epi) {
-    constexpr int BK = 16, NT = BM * BN / 16, TC = BN / 4;
+    constexpr int BK = 16, NT = BM * BN / 4 / TM, TC = BN / 4;
     constexpr int LA = BM * BK / 4 / NT, LW = BN * BK / 4 / NT;         // float4 loads per thread and slice
     __shared__ __align__(16) float As[2][BK][BM + 4];
     __shared__ __align__(16) float Ws[2][BK][BN];
     const int tid = threadIdx.x, tr = tid / TC, tc = tid % TC;
     const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
-    float acc[4][4];
+    float2 acc[TM][2];                                                  // column pairs
     #pragma unroll
-    for (int i = 0; i < 4; ++i)
-        #pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
+    for (int i = 0; i < TM; ++i) acc[i][0] = acc[i][1] = make_float2(0.f, 0.f);
     float4 ra[LA], rw[LW];
     const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
     auto gload = [&](int k0) {
@@ -236,20 +243,25 @@ k_gemm_f32s(const float* __restrict__ A, int lda, const float* __restrict__ W, i
         if (kt + 1 < nk) gload((kt + 1) * BK);
         #pragma unroll
         for (int kk = 0; kk < BK; ++kk) {
-            const float4 a4 = *reinterpret_cast<const float4*>(&As[buf][kk][4 * tr]);
-            const float4 w4 = *reinterpret_cast<const float4*>(&Ws[buf][kk][4 * tc]);
-            const float a[4] = {a4.x, a4.y, a4.z, a4.w}, w[4] = {w4.x, w4.y, w4.z, w4.w};
+            float a[TM];
             #pragma unroll
-            for (int i = 0; i < 4; ++i)
-                #pragma unroll
-                for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(a[i], w[j], acc[i][j]);
+            for (int h = 0; h < TM / 4; ++h) {
+                const float4 a4 = *reinterpret_cast<const float4*>(&As[buf][kk][4 * tr + h * (BM / 2)]);
+                a[4 * h] = a4.x; a[4 * h + 1] = a4.y; a[4 * h + 2] = a4.z; a[4 * h + 3] = a4.w;
+            }
+            const float4 w4 = *reinterpret_cast<const float4*>(&Ws[buf][kk][4 * tc]);
+            #pragma unroll
+            for (int i = 0; i < TM; ++i) {
+                acc[i][0] = fma2(make_float2(a[i], a[i]), make_float2(w4.x, w4.y), acc[i][0]);
+                acc[i][1] = fma2(make_float2(a[i], a[i]), make_float2(w4.z, w4.w), acc[i][1]);
+            }
         }
         if (kt + 1 < nk) sstore(buf ^ 1);
         __syncthreads();
     }
     #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const int m = m0 + 4 * tr + i;
+    for (int i = 0; i < TM; ++i) {
+        const int m = m0 + 4 * tr + i % 4 + i / 4 * (BM / 2);
         if (m >= M) continue;
         const int t = m % epi.Tp;
         const float* rb = epi.rowbias ? epi.rowbias + ((int64_t)(m / epi.rows_per_walker) * epi.Tp + t) * epi.ldrb : nullptr;
@@ -257,7 +269,7 @@ k_gemm_f32s(const float* __restrict__ A, int lda, const float* __restrict__ W, i
         for (int j = 0; j < 4; ++j) {
             const int n = n0 + 4 * tc + j;
             if (n >= N) continue;
-            float v = acc[i][j];
+            float v = j % 2 ? acc[i][j / 2].y : acc[i][j / 2].x;
             if (epi.bias && t == 0) v += epi.bias[n];
             if (rb) v += rb[n];
             if (epi.act == 1) v = tanhf(v);
@@ -325,8 +337,10 @@ void gemm_f32(const float* A, int lda, const float* W, int ldw, float* C, int ld
     const bool narrow = N <= 32;
     const int64_t big = (int64_t)((M + 127) / 128) * ((N + 127) / 128);
     if (batch == 1 && big < 2 * num_sms_simt() && operands_ok(A, lda, W, ldw, N, K, false)) {
-        if (narrow) k_gemm_f32s<64, 32><<<dim3(1, (M + 63) / 64), 128, 0, s>>>(A, lda, W, ldw, C, ldc, M, N, K, epi);
-        else k_gemm_f32s<64, 64><<<dim3((N + 63) / 64, (M + 63) / 64), 256, 0, s>>>(A, lda, W, ldw, C, ldc, M, N, K, epi);
+        const bool tall = !narrow && (int64_t)((M + 127) / 128) * ((N + 63) / 64) >= num_sms_simt();
+        if (narrow) k_gemm_f32s<64, 32, 4><<<dim3(1, (M + 63) / 64), 128, 0, s>>>(A, lda, W, ldw, C, ldc, M, N, K, epi);
+        else if (tall) k_gemm_f32s<128, 64, 8><<<dim3((N + 63) / 64, (M + 127) / 128), 256, 0, s>>>(A, lda, W, ldw, C, ldc, M, N, K, epi);
+        else k_gemm_f32s<64, 64, 4><<<dim3((N + 63) / 64, (M + 63) / 64), 256, 0, s>>>(A, lda, W, ldw, C, ldc, M, N, K, epi);
         count_launch();
         return;
     }
@@ -423,53 +437,88 @@ k_wgrad_f32_64(const float* __restrict__ A, int lda, const float* __restrict__ G
     }
 }
 
-// Weight gradient dW[K, N] += sum_r A[r, k] G[r, n]: 128 x 128 output tiles, rows split into
-// segments over grid.z and accumulated atomically; each block stages 16-row slabs of A and G in
-// shared memory and accumulates an 8 x 8 patch per thread.
-__global__ void __launch_bounds__(256)
+// Weight gradients dW[K, N] += A[rows, K]^T G[rows, N]: output tiles by rows split into segments over
+// grid.z and accumulated atomically.
+// 128 x 128 tile of dW per block, 8 x 8 per thread (two 4-wide groups in each direction so that the
+// 16-byte shared-memory reads of a warp are consecutive), 16 rows per step, the next step's rows
+// fetched into registers (VEC: as float4) while this one's products run.
+template <bool VEC>
+__global__ void __launch_bounds__(256, 2)
 k_wgrad_f32(const float* __restrict__ A, int lda, const float* __restrict__ G, int ldg, int rows, int K, int N,
             float* __restrict__ dW, int lddw, float* __restrict__ dB, const int8_t* __restrict__ sel, int want,
             int rows_per_seg) {
-    // 128 x 128 tile of dW per block, 8 x 8 per thread (two 4-wide groups in each direction so that
-    // the 16-byte shared-memory reads of a warp are consecutive), 16 rows staged per step.
     constexpr int TB = 128, RB = 16;
-    __shared__ __align__(16) float As[RB][TB];
-    __shared__ __align__(16) float Gs[RB][TB];
+    __shared__ __align__(16) float As[2][RB][TB];
+    __shared__ __align__(16) float Gs[2][RB][TB];
     const int k0 = blockIdx.y * TB, n0 = blockIdx.x * TB;
     const int r_begin = blockIdx.z * rows_per_seg, r_end = min(rows, r_begin + rows_per_seg);
     const int tid = threadIdx.x, tk = tid / 16, tn = tid % 16;
-    float acc[8][8];
+    float2 acc[8][4];
     #pragma unroll
     for (int u = 0; u < 8; ++u)
         #pragma unroll
-        for (int v = 0; v < 8; ++v) acc[u][v] = 0.f;
+        for (int v = 0; v < 4; ++v) acc[u][v] = make_float2(0.f, 0.f);
     float bacc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
     const bool do_bias = dB && blockIdx.y == 0 && tk == 0;
-    for (int r0 = r_begin; r0 < r_end; r0 += RB) {
-        for (int e = tid; e < RB * TB; e += 256) {
-            const int rr = e / TB, cc = e % TB, r = r0 + rr;
-            const bool ok = r < r_end && (!sel || sel[r] == want);
-            As[rr][cc] = (ok && k0 + cc < K) ? __ldg(A + (int64_t)r * lda + k0 + cc) : 0.f;
-            Gs[rr][cc] = (ok && n0 + cc < N) ? __ldg(G + (int64_t)r * ldg + n0 + cc) : 0.f;
+    // this thread's share of a step: rows tid / 32 and tid / 32 + 8, columns 4 (tid % 32) .. + 3
+    const int lc = tid % 32 * 4, lr = tid / 32;
+    float4 ra[2], rg[2];
+    auto row4 = [&](const float* X, int ld, int c0, int C, int r, bool ok) {
+        float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (!ok) return x;
+        const float* p = X + (int64_t)r * ld + c0 + lc;
+        if (VEC) {
+            if (c0 + lc < C) x = __ldg(reinterpret_cast<const float4*>(p));
+        } else {
+            if (c0 + lc < C) x.x = __ldg(p);
+            if (c0 + lc + 1 < C) x.y = __ldg(p + 1);
+            if (c0 + lc + 2 < C) x.z = __ldg(p + 2);
+            if (c0 + lc + 3 < C) x.w = __ldg(p + 3);
         }
-        __syncthreads();
+        return x;
+    };
+    auto gload = [&](int r0) {
+        #pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int r = r0 + lr + 8 * h;
+            const bool ok = r < r_end && (!sel || sel[r] == want);
+            ra[h] = row4(A, lda, k0, K, r, ok);
+            rg[h] = row4(G, ldg, n0, N, r, ok);
+        }
+    };
+    auto sstore = [&](int buf) {
+        #pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            *reinterpret_cast<float4*>(&As[buf][lr + 8 * h][lc]) = ra[h];
+            *reinterpret_cast<float4*>(&Gs[buf][lr + 8 * h][lc]) = rg[h];
+        }
+    };
+    if (r_begin < r_end) {
+        gload(r_begin);
+        sstore(0);
+    }
+    __syncthreads();
+    int buf = 0;
+    for (int r0 = r_begin; r0 < r_end; r0 += RB, buf ^= 1) {
+        if (r0 + RB < r_end) gload(r0 + RB);
         #pragma unroll 2
         for (int rr = 0; rr < RB; ++rr) {
-            const float4 a0 = *reinterpret_cast<const float4*>(&As[rr][4 * tk]);
-            const float4 a1 = *reinterpret_cast<const float4*>(&As[rr][64 + 4 * tk]);
-            const float4 g0 = *reinterpret_cast<const float4*>(&Gs[rr][4 * tn]);
-            const float4 g1 = *reinterpret_cast<const float4*>(&Gs[rr][64 + 4 * tn]);
+            const float4 a0 = *reinterpret_cast<const float4*>(&As[buf][rr][4 * tk]);
+            const float4 a1 = *reinterpret_cast<const float4*>(&As[buf][rr][64 + 4 * tk]);
+            const float4 g0 = *reinterpret_cast<const float4*>(&Gs[buf][rr][4 * tn]);
+            const float4 g1 = *reinterpret_cast<const float4*>(&Gs[buf][rr][64 + 4 * tn]);
             const float a[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
-            const float g[8] = {g0.x, g0.y, g0.z, g0.w, g1.x, g1.y, g1.z, g1.w};
+            const float2 g[4] = {make_float2(g0.x, g0.y), make_float2(g0.z, g0.w), make_float2(g1.x, g1.y), make_float2(g1.z, g1.w)};
             #pragma unroll
             for (int u = 0; u < 8; ++u)
                 #pragma unroll
-                for (int v = 0; v < 8; ++v) acc[u][v] = fmaf(a[u], g[v], acc[u][v]);
+                for (int v = 0; v < 4; ++v) acc[u][v] = fma2(make_float2(a[u], a[u]), g[v], acc[u][v]);
             if (do_bias) {
                 #pragma unroll
-                for (int v = 0; v < 8; ++v) bacc[v] += g[v];
+                for (int v = 0; v < 4; ++v) { bacc[2 * v] += g[v].x; bacc[2 * v + 1] += g[v].y; }
             }
         }
+        if (r0 + RB < r_end) sstore(buf ^ 1);
         __syncthreads();
     }
     #pragma unroll
@@ -479,7 +528,7 @@ k_wgrad_f32(const float* __restrict__ A, int lda, const float* __restrict__ G, i
         #pragma unroll
         for (int v = 0; v < 8; ++v) {
             const int n = n0 + (v < 4 ? 4 * tn + v : 64 + 4 * tn + v - 4);
-            if (n < N) atomicAdd(dW + (int64_t)k * lddw + n, acc[u][v]);
+            if (n < N) atomicAdd(dW + (int64_t)k * lddw + n, v % 2 ? acc[u][v / 2].y : acc[u][v / 2].x);
         }
     }
     if (do_bias) {
@@ -616,7 +665,9 @@ void wgrad_f32(const float* A, int lda, const float* G, int ldg, int rows, int K
     rps = (rps + 15) / 16 * 16;
     segs = (rows + rps - 1) / rps;
     dim3 g((N + 127) / 128, (K + 127) / 128, segs);
-    k_wgrad_f32<<<g, 256, 0, s>>>(A, lda, G, ldg, rows, K, N, dW, lddw, dB, sel, want, rps);
+    const bool vec = lda % 4 == 0 && ldg % 4 == 0 && K % 4 == 0 && N % 4 == 0 && (((uintptr_t)A | (uintptr_t)G) & 15) == 0;
+    if (vec) k_wgrad_f32<true><<<g, 256, 0, s>>>(A, lda, G, ldg, rows, K, N, dW, lddw, dB, sel, want, rps);
+    else k_wgrad_f32<false><<<g, 256, 0, s>>>(A, lda, G, ldg, rows, K, N, dW, lddw, dB, sel, want, rps);
     count_launch();
 }
 
