@@ -943,18 +943,23 @@ __global__ void k_conv(const float* __restrict__ r, const float* __restrict__ WP
 // over the warps: single terms w'_im u_im h_m for the channels of the other electrons m, the
 // j-sums of the electron's own gradient channels and of the Laplacian. Columns are then written
 // eight at a time (16-byte stores). conv_ei is non-zero on 5 channels per electron only. Same
-// mathematics as k_conv.
+// mathematics as k_conv. Bound by the latency of its loads between barriers: the pair geometry is formed
+// once per block (a square root and a division per term before), only the warps with channels are
+// launched, and two j are in flight. Per local energy: H10, 8,192 walkers 3.36 -> 2.62 ms, C2H4, 4,096
+// walkers 4.08 -> 3.57 ms, 27 electrons, 1,500 walkers 7.1 -> 6.1 ms. (Keeping the tile in registers to the
+// store instead of staging it took 2.5 times as long.)
 template <class Act, int TT, int TI>
 __global__ void __launch_bounds__(512)
 k_conv_tile(const float* __restrict__ r, const float* __restrict__ WPl, const float* __restrict__ HM,
             const float* __restrict__ HEl, const float* __restrict__ himl, Dims d, int l, int B, Act* __restrict__ X,
-            int ldx, int ei_fused) {
+            int ldx, int ei_fused, int G) {
     extern __shared__ __align__(16) float smc[];
     const int n = d.n, Tp = d.Tp, T = d.T;
     const int NW = blockDim.x >> 5;
     float* out = smc;                                   // [TI][Tp][32] conv_ee
-    float* red = out + TI * Tp * 32;                    // [NW][TI][4][32] own-gradient / Laplacian partials
-    float* eiv = red + NW * TI * 4 * 32;                // [TI][5][32] conv_ei channels
+    float* red = out + TI * Tp * 32;                    // [G][TI][4][32] own-gradient / Laplacian partials
+    float* eiv = red + G * TI * 4 * 32;                 // [TI][5][32] conv_ei channels
+    float4* geo = reinterpret_cast<float4*>(eiv + TI * 5 * 32);   // [TI][n]: r_j - r_i, 1 / |r_j - r_i|
     const int f = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int ntile = (n + TI - 1) / TI;
     const int b = blockIdx.x / ntile, i0 = (blockIdx.x % ntile) * TI;
@@ -964,6 +969,11 @@ k_conv_tile(const float* __restrict__ r, const float* __restrict__ WPl, const fl
     const float* rb = r + (size_t)b * n * 3;
     const float* wpb = WPl + (size_t)b * n * n * 96 + f;           // records [i * n + j][3][32]
     const float* hmb = HM + (size_t)b * n * Tp * 32 + f;           // [j][Tp][32]
+    for (int e = threadIdx.x; e < ni * n; e += blockDim.x) {
+        const int i = i0 + e / n, j = e % n;
+        const float dx = rb[j * 3] - rb[i * 3], dy = rb[j * 3 + 1] - rb[i * 3 + 1], dz = rb[j * 3 + 2] - rb[i * 3 + 2];
+        geo[e] = make_float4(dx, dy, dz, 1.f / sqrtf(dx * dx + dy * dy + dz * dz));
+    }
     {
         float acc[TI][TT];
         #pragma unroll
@@ -971,6 +981,7 @@ k_conv_tile(const float* __restrict__ r, const float* __restrict__ WPl, const fl
             #pragma unroll
             for (int k = 0; k < TT; ++k) acc[ii][k] = 0.f;
         const int i_last = i0 + ni - 1;
+        #pragma unroll 2
         for (int j = 0; j < n; ++j) {
             const float* hj = hmb + (size_t)j * Tp * 32;
             float h[TT];
@@ -990,26 +1001,26 @@ k_conv_tile(const float* __restrict__ r, const float* __restrict__ WPl, const fl
             for (int k = 0; k < TT; ++k)
                 if (t0 + k < T) out[(ii * Tp + t0 + k) * 32 + f] = acc[ii][k];
     }
-    // product-rule partials of the own-gradient channels and the Laplacian, j split over warps
-    for (int ii = 0; ii < ni; ++ii) {
-        const int i = i0 + ii;
-        const float rx = rb[i * 3], ry = rb[i * 3 + 1], rz = rb[i * 3 + 2];
+    __syncthreads();                                    // geo
+    // product-rule partials of the own-gradient channels and the Laplacian: j = q, q + G, ... per partial
+    for (int it = w; it < G * ni; it += NW) {
+        const int q = it / ni, ii = it % ni, i = i0 + ii;
         float o0 = 0.f, o1 = 0.f, o2 = 0.f, ol = 0.f;
-        for (int j = w; j < n; j += NW) {
+        for (int j = q; j < n; j += G) {
             if (j == i) continue;
             const float* wr = wpb + ((size_t)i * n + j) * 96;
             const float* hj = hmb + (size_t)j * Tp * 32;
             const float w1 = __ldg(wr + 32), w2 = __ldg(wr + 64), h0 = __ldg(hj);
-            const float dx = rb[j * 3] - rx, dy = rb[j * 3 + 1] - ry, dz = rb[j * 3 + 2] - rz;
-            const float inv = 1.f / sqrtf(dx * dx + dy * dy + dz * dz);
-            const float ux = dx * inv, uy = dy * inv, uz = dz * inv;
+            const float4 u = geo[ii * n + j];
+            const float inv = u.w;
+            const float ux = u.x * inv, uy = u.y * inv, uz = u.z * inv;
             o0 += w1 * ux * h0; o1 += w1 * uy * h0; o2 += w1 * uz * h0;
             const float cross = ux * (__ldg(hj + (1 + 3 * j) * 32) - __ldg(hj + (1 + 3 * i) * 32)) +
                                 uy * (__ldg(hj + (2 + 3 * j) * 32) - __ldg(hj + (2 + 3 * i) * 32)) +
                                 uz * (__ldg(hj + (3 + 3 * j) * 32) - __ldg(hj + (3 + 3 * i) * 32));
             ol += 2.f * (w2 + 2.f * w1 * inv) * h0 + 2.f * w1 * cross;
         }
-        float* rr = red + ((w * TI + ii) * 4) * 32 + f;
+        float* rr = red + ((q * TI + ii) * 4) * 32 + f;
         rr[0] = o0; rr[32] = o1; rr[64] = o2; rr[96] = ol;
     }
     // conv_ei on its 5 non-zero channels: items (ii, ch) over the warps
@@ -1034,16 +1045,16 @@ k_conv_tile(const float* __restrict__ r, const float* __restrict__ WPl, const fl
         float* o = out + (ii * Tp) * 32 + f;
         if (m == i) {
             float s0 = 0.f, s1 = 0.f, s2 = 0.f, sl = 0.f;
-            for (int q = 0; q < NW; ++q) {
+            for (int q = 0; q < G; ++q) {
                 const float* rr = red + ((q * TI + ii) * 4) * 32 + f;
                 s0 += rr[0]; s1 += rr[32]; s2 += rr[64]; sl += rr[96];
             }
             o[(1 + 3 * i) * 32] -= s0; o[(2 + 3 * i) * 32] -= s1; o[(3 + 3 * i) * 32] -= s2;
             o[d.lap * 32] += sl;
         } else {
-            const float dx = rb[m * 3] - rb[i * 3], dy = rb[m * 3 + 1] - rb[i * 3 + 1], dz = rb[m * 3 + 2] - rb[i * 3 + 2];
-            const float inv = 1.f / sqrtf(dx * dx + dy * dy + dz * dz);
-            const float g = __ldg(wpb + ((size_t)i * n + m) * 96 + 32) * __ldg(hmb + (size_t)m * Tp * 32) * inv;
+            const float4 u = geo[ii * n + m];
+            const float dx = u.x, dy = u.y, dz = u.z;
+            const float g = __ldg(wpb + ((size_t)i * n + m) * 96 + 32) * __ldg(hmb + (size_t)m * Tp * 32) * u.w;
             o[(1 + 3 * m) * 32] = fmaf(g, dx, o[(1 + 3 * m) * 32]);
             o[(2 + 3 * m) * 32] = fmaf(g, dy, o[(2 + 3 * m) * 32]);
             o[(3 + 3 * m) * 32] = fmaf(g, dz, o[(3 + 3 * m) * 32]);
@@ -1054,8 +1065,13 @@ k_conv_tile(const float* __restrict__ r, const float* __restrict__ WPl, const fl
     const int ei_units = (eiw + 7) / 8;
     const int units = 4 + ei_units;
     const bool rowvec = (hw % 8) == 0 && (ldx % 8) == 0;      // 16-byte aligned column groups
-    for (int it = threadIdx.x; it < ni * Tp * units; it += blockDim.x) {
-        const int u = it % units, rt = it / units, t = rt % Tp, ii = rt / Tp, i = i0 + ii;
+    // (row position carried along instead of divided out of a flat index)
+    const int rstep = blockDim.x / units, u = threadIdx.x % units;
+    int t = threadIdx.x / units, ii = 0;
+    if (t >= rstep) ii = ni;                             // threads beyond the last whole row of units
+    for (; t >= Tp; t -= Tp) ++ii;
+    for (; ii < ni;) {
+        const int i = i0 + ii;
         const int64_t row = ((int64_t)b * n + i) * Tp + t;
         float v[8];
         int col;
@@ -1082,6 +1098,7 @@ k_conv_tile(const float* __restrict__ r, const float* __restrict__ WPl, const fl
             for (int k = 0; k < 8; ++k)
                 if (k < lim) ActIO<Act>::store(X, row, ldx, col + k, v[k]);
         }
+        for (t += rstep; t >= Tp; t -= Tp) ++ii;
     }
 }
 
@@ -1394,11 +1411,11 @@ void launch_conv(const float* r, const float* WPl, const float* HM, const float*
         constexpr int TI = 4;
         const unsigned grid = (unsigned)B * ((d.n + TI - 1) / TI);
         const int rows = next_pow2(d.Tp), TT = rows >= 64 ? 8 : rows / 8;
-        const int NW = rows / TT;
-        const size_t smem = ((size_t)TI * d.Tp * 32 + (size_t)NW * TI * 4 * 32 + (size_t)TI * 5 * 32) * sizeof(float);
+        const int G = rows / TT, NW = (d.Tp + TT - 1) / TT;
+        const size_t smem = ((size_t)TI * d.Tp * 32 + (size_t)G * TI * 4 * 32 + (size_t)TI * 5 * 32 + (size_t)TI * d.n * 4) * sizeof(float);
         auto go = [&](auto kern) {
             cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-            kern<<<grid, NW * 32, smem, s>>>(r, WPl, HM, HEl, himl, d, l, B, X, ldx, ei_fused);
+            kern<<<grid, NW * 32, smem, s>>>(r, WPl, HM, HEl, himl, d, l, B, X, ldx, ei_fused, G);
         };
         auto pick = [&](auto ti) {
             constexpr int T_I = decltype(ti)::value;
