@@ -3,6 +3,7 @@
 #include "net.cuh"
 #include "mcmc.cuh"
 #include "gemm_tc.cuh"
+#include "fp64_gemm.cuh"
 #include <string.h>
 #include <algorithm>
 #include <type_traits>
@@ -146,6 +147,7 @@ struct Plan {
     double* logdet; double* sign; float* Ainv; double* g; double* lapdet;
     Act* J1; Act* J2; double* jas;
     size_t bytes;
+    void* scratch = nullptr; size_t scratch_bytes = 0;     // what the caller's region holds beyond the plan
 };
 
 static const int kXW = 320;   // row width of the layer-1..3 inputs: 256 (h) + 32 (conv_ee) + 32 (conv_ei)
@@ -354,7 +356,7 @@ static int run_chunk(const Plan<Act>& p, int Bc, int precision, const float* P, 
         // size) and the inverses the layer buffer XA (the embedding H is in XB)
         DW_TIMED("det_tangents", DW_CHECK(fp64_dets_from_f32(p.MO, d, Bc, reinterpret_cast<double*>(p.BF),
                                                              reinterpret_cast<double*>(p.XA), p.logdet, p.sign, p.g,
-                                                             p.lapdet, s)));
+                                                             p.lapdet, p.scratch, p.scratch_bytes, s)));
     } else {
         if (precision == DW_PRECISION_FP32) DW_TIMED("slogdet", launch_slogdet<float>(p.MO, d, Bc, p.logdet, p.sign, p.Ainv, s));
         else DW_TIMED("slogdet", launch_slogdet<double>(p.MO, d, Bc, p.logdet, p.sign, p.Ainv, s));
@@ -451,6 +453,8 @@ static int forward_all(const DwArch* a, int precision, const float* P, const voi
     int bc = choose_chunk<Act>(d, B, budget);
     Plan<Act> p = carve_plan<Act>(d, bc, ws);
     if (p.bytes > ws_bytes) return DW_ERR_WORKSPACE;
+    p.scratch = static_cast<char*>(ws) + p.bytes;
+    p.scratch_bytes = ws_bytes - p.bytes;
     d.nseg = nseg;
     p.d.nseg = nseg;      // the chunks index geometries through the plan's dims
     launch_ion_maps(P, L, d, Z, p.him, s);
@@ -514,7 +518,13 @@ static int local_energy_impl(const DwArch* a, int precision, const float* params
 // FP32 network, DW_PRECISION_MIXED_DET64: split-BF16 network): the mixed form's re-evaluation of
 // flagged walkers (guard.cu).
 size_t det64_plan_bytes(const DwArch* a, int precision, int B) {
-    return precision == DW_PRECISION_MIXED_DET64 ? plan_bytes<Split>(a, B, true) : plan_bytes<float>(a, B, true);
+    const Dims d = make_dims(a, true);
+    // and the scratch of the FP64 determinant tangents of a chunk
+    auto bytes = [&](auto tag) {
+        using Act = act_of<decltype(tag)>;
+        return plan_bytes<Act>(a, B, true) + dets64_scratch_bytes(d.n, d.T, (int64_t)choose_chunk<Act>(d, std::max(B, 1)) * d.K);
+    };
+    return precision == DW_PRECISION_MIXED_DET64 ? bytes((Split*)nullptr) : bytes((float*)nullptr);
 }
 int det64_local_energy(const DwArch* a, int precision, const float* P, const void* prepared, const float* r, int B,
                        const float* R, const int32_t* Z, const int32_t* seg, int nseg, float* E, float* lp, float* grad,

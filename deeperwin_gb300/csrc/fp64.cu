@@ -482,6 +482,19 @@ k64_det_tangents(const double* __restrict__ MO, const double* __restrict__ Ainv,
     if (tid == 0) lapdet[mat] = lap_acc;
 }
 
+// By digit products where they are faster and the scratch holds enough matrices, else by k64_det_tangents.
+static int launch_tangents64(const double* MO, const double* Ainv, const double* sign, const Run64& q, int nmat, double* g,
+                             double* lapdet, void* scratch, size_t scratch_bytes, cudaStream_t s) {
+    const int n = q.d.n;
+    int status = DW_OK;
+    if (dets64_tangents(MO, Ainv, sign, n, q.C, q.d.K, nmat, q.nvalid, g, lapdet, scratch, scratch_bytes, s, &status)) return status;
+    const size_t sm = (size_t)3 * n * n * sizeof(double);
+    if (sm > 48 * 1024) cudaFuncSetAttribute(k64_det_tangents, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    k64_det_tangents<<<nmat, 128, sm, s>>>(MO, Ainv, sign, q, g, lapdet);
+    count_launch();
+    return DW_OK;
+}
+
 // Jastrow output: jas[(b, t)] = sum_i sum_c J2[(b, i, t)][c] w2[c] (wavefunction.py:57-59, linear
 // output without bias, summed over electrons). Warp per (walker, channel).
 __global__ void k64_jastrow_out(const double* __restrict__ J2, int ldj, const float* __restrict__ w2, Run64 q,
@@ -506,6 +519,7 @@ struct Plan64 {
     int Bc, C;
     double* him;
     double *XA, *XB, *Zt, *HM, *M, *WB, *WP, *CE, *BF, *MO, *logdet, *sign, *Ainv, *g, *lapdet, *J1, *J2, *jas;
+    void* scratch; size_t scratch_bytes;             // dets64_tangents
     Digits act, mean;              // digit planes of the activation rows and of the spin-mean rows
     Weight64 w[kMaxW64];           // h_map[4], mean rows[4], main rows[4], backflow[2], Jastrow[2] (w.w set per call)
     size_t bytes;
@@ -542,7 +556,13 @@ static Plan64 carve64(const Dims& d, int C, int Bc, void* ws, bool digits = true
     p.J1 = c.take<double>(rows * d.J0);
     p.J2 = c.take<double>(rows * d.J1);
     p.jas = c.take<double>((int64_t)Bc * C);
+    p.scratch = nullptr;
+    p.scratch_bytes = 0;
     if (digits) {
+        if (C > 1) {
+            p.scratch_bytes = dets64_scratch_bytes(d.n, C, (int64_t)Bc * d.K);
+            p.scratch = c.take<unsigned char>(p.scratch_bytes);
+        }
         auto take = [&](int64_t r, int K) {
             const int Kp = pad_k64(K);
             __nv_bfloat16* dig = c.take<__nv_bfloat16>((size_t)kDig * r * Kp);
@@ -661,12 +681,9 @@ static int run_chunk64(const Plan64& p, const Dims& d0, int Bc, const float* P, 
     timer_end("fp64_lu", s, 0.0, 0.0);
     count_launch();
     if (tang) {
-        const size_t sm_t = (size_t)3 * n * n * sizeof(double);
-        if (sm_t > 48 * 1024) cudaFuncSetAttribute(k64_det_tangents, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_t);
         timer_begin("fp64_det_tangents", s);
-        k64_det_tangents<<<nmat, 128, sm_t, s>>>(p.MO, p.Ainv, p.sign, q, p.g, p.lapdet);
+        DW_CHECK(launch_tangents64(p.MO, p.Ainv, p.sign, q, nmat, p.g, p.lapdet, p.scratch, p.scratch_bytes, s));
         timer_end("fp64_det_tangents", s, 0.0, 0.0);
-        count_launch();
     }
     // Jastrow MLP([64, 64, 1]) on the final embedding (wavefunction.py:42-60)
     Epi64 j0; j0.bias = P + L.jas_b[0];
@@ -697,7 +714,7 @@ __global__ void k64_widen(const float* __restrict__ x, int64_t n, double* __rest
 }
 
 int fp64_dets_from_f32(const float* MO, const Dims& d, int Bc, double* MO64, double* Ainv64, double* logdet,
-                       double* sign, double* g, double* lapdet, cudaStream_t s) {
+                       double* sign, double* g, double* lapdet, void* scratch, size_t scratch_bytes, cudaStream_t s) {
     Run64 q;
     q.d = d; q.C = d.T; q.B = Bc; q.nvalid = nullptr;
     const int n = d.n, nmat = Bc * d.K;
@@ -709,12 +726,7 @@ int fp64_dets_from_f32(const float* MO, const Dims& d, int Bc, double* MO64, dou
     if (sm_lu > 48 * 1024) cudaFuncSetAttribute(k64_slogdet_inv, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_lu);
     k64_slogdet_inv<<<nmat, 128, sm_lu, s>>>(MO64, q, logdet, sign, tang ? Ainv64 : nullptr);
     count_launch();
-    if (tang) {
-        const size_t sm_t = (size_t)3 * n * n * sizeof(double);
-        if (sm_t > 48 * 1024) cudaFuncSetAttribute(k64_det_tangents, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_t);
-        k64_det_tangents<<<nmat, 128, sm_t, s>>>(MO64, Ainv64, sign, q, g, lapdet);
-        count_launch();
-    }
+    if (tang) DW_CHECK(launch_tangents64(MO64, Ainv64, sign, q, nmat, g, lapdet, scratch, scratch_bytes, s));
     DW_CHECK_CUDA(cudaGetLastError());
     return DW_OK;
 }

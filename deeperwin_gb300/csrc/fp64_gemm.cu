@@ -40,7 +40,7 @@ constexpr int kStageBytes = kDig * (kABytes + kBBytes);          // 101,376
 constexpr int kSmem64 = 1024 + kStages * kStageBytes + 256;
 constexpr int kFlagged = 0x7fffffff;                 // exponent of a row that the digits do not represent
 
-__device__ __forceinline__ int valid_of(const Rows64& r) { return r.nvalid ? min(r.B, max(0, *r.nvalid)) : r.B; }
+__device__ __forceinline__ int valid_of(const Rows64& r) { return r.nvalid ? min(r.B, max(0, *r.nvalid * r.mul - r.first)) : r.B; }
 
 // Biased exponent field of x.
 __device__ __forceinline__ int exp_field(double x) { return (__double2hiint(x) >> 20) & 0x7ff; }
@@ -71,7 +71,8 @@ __device__ __forceinline__ uint32_t pack_digits(int a, int b) {
 }
 
 // One row held by a warp (columns 64 u + 2 lane, + 1): common exponent and digit planes.
-__device__ __forceinline__ void slice_row(const double2 (&x)[kMaxK64 / 64], int emax, bool nonzero, int64_t m,
+template <int NU>
+__device__ __forceinline__ void slice_row(const double2 (&x)[NU], int emax, bool nonzero, int64_t m,
                                           const Digits& d) {
     const int lane = threadIdx.x & 31, Kp = d.Kp;
     emax = __reduce_max_sync(0xffffffffu, emax);
@@ -81,7 +82,7 @@ __device__ __forceinline__ void slice_row(const double2 (&x)[kMaxK64 / 64], int 
     __nv_bfloat16* o = d.dig + m * Kp;
     const int64_t plane = d.rows * Kp;
     #pragma unroll
-    for (int u = 0; u < kMaxK64 / 64; ++u) {
+    for (int u = 0; u < NU; ++u) {
         const int c = u * 64 + 2 * lane;
         if (c >= Kp) continue;
         long long f0 = 0, f1 = 0;
@@ -96,8 +97,10 @@ __device__ __forceinline__ void slice_row(const double2 (&x)[kMaxK64 / 64], int 
 
 // Warp per row: the largest exponent, then the digits of two neighbouring columns per lane and step.
 // HBM-bound: 8 K bytes read, 18 Kp written per row.
+// es: distance of a row's elements; NU: groups of 64 columns.
+template <int NU>
 __global__ void __launch_bounds__(256)
-k64_slice_rows(const double* __restrict__ A, int lda, int K, Rows64 rows, Digits d) {
+k64_slice_rows(const double* __restrict__ A, int lda, int es, int K, Rows64 rows, Digits d) {
     const int nv = valid_of(rows), lane = threadIdx.x & 31;
     const int64_t w = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int gi = rows.ngroups > 1 && w >= (int64_t)rows.B * rows.g[0].rpw ? 1 : 0;
@@ -107,15 +110,15 @@ k64_slice_rows(const double* __restrict__ A, int lda, int K, Rows64 rows, Digits
     if (b >= nv) return;
     const int64_t m = g.base + k;
     const double* src = A + (b * g.out_rpw + g.out_off + k % g.rpw) * lda;
-    double2 x[kMaxK64 / 64];
+    double2 x[NU];
     int emax = 0;
     bool sub = false;
     #pragma unroll
-    for (int u = 0; u < kMaxK64 / 64; ++u) {
+    for (int u = 0; u < NU; ++u) {
         const int c = u * 64 + 2 * lane;
         x[u] = make_double2(0.0, 0.0);
-        if (c < K) x[u].x = src[c];
-        if (c + 1 < K) x[u].y = src[c + 1];
+        if (c < K) x[u].x = src[(int64_t)c * es];
+        if (c + 1 < K) x[u].y = src[(int64_t)(c + 1) * es];
         emax = max(emax, max(exp_field(x[u].x), exp_field(x[u].y)));
         sub |= x[u].x != 0.0 || x[u].y != 0.0;
     }
@@ -217,6 +220,9 @@ struct Args64 {
     Rows64 rows;
     Epi64 e;
     int N, K, channels, ntn;
+    // batched form (determinants): `per` rows and N columns per matrix, W FP64 [matrix][K][N]
+    const double* W64;
+    int per;
     int* error;                    // set when a bounded wait ran out
 };
 
@@ -260,11 +266,16 @@ __device__ __forceinline__ double combine_digits(const float* acc, int stride, i
 // MMAs of a stage into nine TMEM accumulators (432 columns), eight warps combine and store them. Bound
 // by the MMAs' shared-memory reads of A (N = 48: 32 clocks of reads for 24 of products); nine
 // accumulators leave no room for a second set, so the epilogue (about a fifth) is not overlapped.
+// BATCH: each matrix has its own weights (rows [matrix N, + N) of their digit planes) and whole tiles.
+template <bool BATCH>
 __global__ void __launch_bounds__(kThreads64, 1)
 k64_gemm_tc(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, Args64 a) {
     const int nv = valid_of(a.rows);
     int64_t tiles_of[2] = {0, 0};
-    for (int g = 0; g < a.rows.ngroups; ++g) tiles_of[g] = ((int64_t)nv * a.rows.g[g].rpw + BM - 1) / BM * a.ntn;
+    const int tpm = BATCH ? (a.per + BM - 1) / BM : 1;          // tiles per matrix
+    if (BATCH) tiles_of[0] = (int64_t)nv * tpm;
+    else
+        for (int g = 0; g < a.rows.ngroups; ++g) tiles_of[g] = ((int64_t)nv * a.rows.g[g].rpw + BM - 1) / BM * a.ntn;
     const int64_t n_tiles = tiles_of[0] + tiles_of[1];
     if ((int64_t)blockIdx.x >= n_tiles) return;       // before any barrier or TMEM allocation
     extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -295,7 +306,14 @@ k64_gemm_tc(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
     // tile -> row group, first row within the group, first column
+    // (BATCH: the matrix, first row within it)
     auto locate = [&](int64_t tile, int& g, int64_t& k0, int& n0) {
+        if (BATCH) {
+            g = (int)(tile / tpm);
+            k0 = tile % tpm * BM;
+            n0 = 0;
+            return;
+        }
         g = tile >= tiles_of[0] ? 1 : 0;
         const int64_t u = g ? tile - tiles_of[0] : tile;
         k0 = u / a.ntn * BM;
@@ -310,7 +328,8 @@ k64_gemm_tc(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
                 int g, n0;
                 int64_t k0;
                 locate(tile, g, k0, n0);
-                const int row = (int)(a.rows.g[g].base + k0);
+                const int row = BATCH ? (int)(g * a.per + k0) : (int)(a.rows.g[g].base + k0);
+                const int wrow = BATCH ? g * a.N : n0;
                 for (int kt = 0; kt < nk; ++kt, ++cnt) {
                     const int s = cnt % kStages;
                     const uint32_t use = cnt / kStages;
@@ -318,7 +337,7 @@ k64_gemm_tc(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
                     mbar_expect_tx(&full[s], kStageBytes);
                     uint8_t* st = smem + s * kStageBytes;
                     tma_load_3d(st, &tmA, &full[s], kt * BK, row, 0);
-                    tma_load_3d(st + kDig * kABytes, &tmB, &full[s], kt * BK, n0, 0);
+                    tma_load_3d(st + kDig * kABytes, &tmB, &full[s], kt * BK, wrow, 0);
                     issued[s] = use + 1;
                 }
             }
@@ -342,7 +361,8 @@ k64_gemm_tc(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
                     tc_fence_after();
                     const uint64_t da = smem_desc_sw64(smem + s * kStageBytes);
                     const uint64_t db = smem_desc_sw64(smem + s * kStageBytes + kDig * kABytes);
-                    for (int kk = 0; kk < BK / 16; ++kk) {
+                    const int nkk = BATCH ? min(BK / 16, (a.K - kt * BK + 15) / 16) : BK / 16;   // 16-column steps with data
+                    for (int kk = 0; kk < nkk; ++kk) {
                         #pragma unroll
                         for (int i = 0; i < kDig; ++i) {
                             #pragma unroll
@@ -364,13 +384,15 @@ k64_gemm_tc(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
             int g, n0;
             int64_t k0;
             locate(tile, g, k0, n0);
-            const RowGroup& rg = a.rows.g[g];
-            const int64_t k = k0 + q * 32 + lane;             // row within the group
-            const bool live = k < (int64_t)nv * rg.rpw;
-            const int64_t b = live ? k / rg.rpw : 0;
-            const int64_t row = b * rg.out_rpw + rg.out_off + (live ? k % rg.rpw : 0);
+            const RowGroup& rg = a.rows.g[BATCH ? 0 : g];
+            const int64_t k = k0 + q * 32 + lane;             // row within the group (matrix)
+            const bool live = k < (BATCH ? (int64_t)a.per : (int64_t)nv * rg.rpw);
+            const int64_t b = BATCH ? g : (live ? k / rg.rpw : 0);
+            const int64_t rem = live ? k - (BATCH ? 0 : b * rg.rpw) : 0;
+            const int64_t row = b * rg.out_rpw + rg.out_off + rem;              // of A
+            const int64_t crow = BATCH ? b * a.per + rem : row;                 // of C
             const int t = (int)(row % a.channels);
-            const int ea = live ? a.ea[rg.base + k] : 0;
+            const int ea = live ? a.ea[BATCH ? crow : rg.base + k] : 0;
             const double* rb = a.e.rowbias ? a.e.rowbias + (b * a.channels + t) * a.e.ldrb : nullptr;
             const bool ready = mbar_wait(tfull, it & 1);
             if (!ready && lane == 0) s_epi_err = 1;
@@ -390,12 +412,13 @@ k64_gemm_tc(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
                         #pragma unroll
                         for (int u = 0; u < 2; ++u) {
                             const int n = min(n0 + c0 + j + u, a.N - 1);
-                            const int ew = a.ew[n];
+                            const int ew = a.ew[BATCH ? g * a.N + n : n];
                             const int scale = ea + ew - 68;
                             if (ea == kFlagged || ew == kFlagged || scale < -900 || scale > 900) {
                                 double x = 0.0;
                                 for (int kk = 0; kk < a.K; ++kk)
-                                    x = fma(a.A[row * a.lda + kk], (double)a.W[(int64_t)kk * a.ldw + n], x);
+                                    x = fma(a.A[row * a.lda + kk], BATCH ? a.W64[((int64_t)g * a.K + kk) * a.N + n]
+                                                                             : (double)a.W[(int64_t)kk * a.ldw + n], x);
                                 v[u] = x;
                             } else {
                                 v[u] = combine_digits(acc + j + u, 8, scale);
@@ -404,7 +427,7 @@ k64_gemm_tc(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
                             if (rb) v[u] += rb[n];
                         }
                         const int n = n0 + c0 + j;
-                        double* o = a.C + row * a.ldc + n;
+                        double* o = a.C + crow * a.ldc + n;
                         if (n + 1 < a.N && !(a.ldc & 1)) *reinterpret_cast<double2*>(o) = make_double2(v[0], v[1]);
                         else {
                             if (n < a.N) o[0] = v[0];
@@ -425,13 +448,61 @@ k64_gemm_tc(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
     if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem) : "memory");
 }
 
+// Traces of E = dA_t A^-1 (cyclic: those of A^-1 dA_t), block per (matrix, channel): tr E to g (tr1 for the
+// Laplacian channel), tr E^2 to tr2.
+__global__ void __launch_bounds__(128)
+k64_traces(const double* __restrict__ E, const double* __restrict__ sign, int n, int C, Rows64 rows, double* __restrict__ g,
+           double* __restrict__ tr1, double* __restrict__ tr2) {
+    const int mat = blockIdx.x / C, t = blockIdx.x % C;            // C = T - 1 channels: gradients, Laplacian
+    if (mat >= valid_of(rows)) return;
+    extern __shared__ double es[];                                  // [n][n + 1]
+    __shared__ double red[2][4];
+    const int tid = threadIdx.x, nn = n * n;
+    const double* src = E + ((int64_t)mat * C + t) * nn;
+    for (int e = tid; e < nn; e += 128) es[e / n * (n + 1) + e % n] = src[e];
+    __syncthreads();
+    double s1 = 0.0, s2 = 0.0;
+    for (int e = tid; e < nn; e += 128) {
+        const int i = e / n, j = e % n;
+        const double x = es[i * (n + 1) + j];
+        if (i == j) s1 += x;
+        s2 = fma(x, es[j * (n + 1) + i], s2);
+    }
+    s1 = warp_sum(s1);
+    s2 = warp_sum(s2);
+    if (tid % 32 == 0) { red[0][tid / 32] = s1; red[1][tid / 32] = s2; }
+    __syncthreads();
+    if (tid == 0) {
+        const bool ok = sign[mat] != 0.0;
+        s1 = ok ? red[0][0] + red[0][1] + red[0][2] + red[0][3] : 0.0;
+        if (t < C - 1) g[(int64_t)mat * (C - 1) + t] = s1;
+        else tr1[mat] = s1;
+        tr2[(int64_t)mat * C + t] = ok ? red[1][0] + red[1][1] + red[1][2] + red[1][3] : 0.0;
+    }
+}
+// lapdet = tr E_lap - sum over the gradient channels of tr E_t^2, warp per matrix.
+__global__ void k64_lapdet(const double* __restrict__ tr1, const double* __restrict__ tr2, int C, Rows64 rows,
+                           double* __restrict__ lapdet) {
+    const int mat = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    if (mat >= valid_of(rows)) return;
+    double s = 0.0;
+    for (int t = lane; t < C - 1; t += 32) s += tr2[(int64_t)mat * C + t];
+    s = warp_sum(s);
+    if (lane == 0) lapdet[mat] = tr1[mat] - s;
+}
+
 }  // namespace
+
+static void slice_any(const double* A, int lda, int es, int K, const Rows64& rows, const Digits& d, int64_t n, cudaStream_t s) {
+    if (d.Kp <= 64) k64_slice_rows<1><<<(unsigned)((n + 7) / 8), 256, 0, s>>>(A, lda, es, K, rows, d);
+    else k64_slice_rows<kMaxK64 / 64><<<(unsigned)((n + 7) / 8), 256, 0, s>>>(A, lda, es, K, rows, d);
+    count_launch();
+}
 
 void slice_rows64(const double* A, int lda, int K, const Rows64& rows, const Digits& d, cudaStream_t s) {
     int64_t n = 0;
     for (int g = 0; g < rows.ngroups; ++g) n += (int64_t)rows.B * rows.g[g].rpw;
-    k64_slice_rows<<<(unsigned)((n + 7) / 8), 256, 0, s>>>(A, lda, K, rows, d);
-    count_launch();
+    slice_any(A, lda, 1, K, rows, d, n, s);
 }
 
 void spin_means64(const double* X, int ldx, int hw, int n, int nu, int C, const Rows64& rows, double* M, const Digits& d,
@@ -464,18 +535,101 @@ int gemm64_tc(const double* A, int lda, const Digits& da, const Weight64& w, dou
     a.ea = da.ex; a.ew = w.d.ex;
     a.rows = rows; a.e = e;
     a.N = w.N; a.K = w.K; a.channels = channels;
+    a.W64 = nullptr; a.per = 0;
     a.ntn = (w.N + BN - 1) / BN;
     a.error = tc_error_flag();
     if (!a.error) return DW_ERR_CUDA;
     int64_t tiles = 0;
     for (int g = 0; g < rows.ngroups; ++g) tiles += ((int64_t)rows.B * rows.g[g].rpw + BM - 1) / BM * a.ntn;
-    DW_CHECK_CUDA(cudaFuncSetAttribute(k64_gemm_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem64));
+    DW_CHECK_CUDA(cudaFuncSetAttribute(k64_gemm_tc<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem64));
     timer_begin("fp64_gemm", s);
-    k64_gemm_tc<<<(unsigned)std::min<int64_t>(tiles, num_sms()), kThreads64, kSmem64, s>>>(ma, mb, a);
+    k64_gemm_tc<false><<<(unsigned)std::min<int64_t>(tiles, num_sms()), kThreads64, kSmem64, s>>>(ma, mb, a);
     timer_end("fp64_gemm", s, 0.0, 0.0);
     count_launch();
     DW_CHECK_CUDA(cudaGetLastError());
     return DW_OK;
+}
+
+// Scratch of dets64_tangents for `m` matrices at a time.
+struct DetScratch {
+    Digits a, w;
+    double *E, *tr1, *tr2;
+    size_t bytes;
+};
+static DetScratch carve_dets(int n, int T, int64_t m, void* base) {
+    Carver c(base, (size_t)-1);
+    DetScratch d;
+    const int64_t per = (int64_t)(T - 1) * n;
+    const int Kp = pad_k64(n);
+    d.a = Digits{c.take<__nv_bfloat16>((size_t)kDig * m * per * Kp), c.take<int>(m * per), m * per, Kp};
+    d.w = Digits{c.take<__nv_bfloat16>((size_t)kDig * m * n * Kp), c.take<int>(m * n), m * n, Kp};
+    d.E = c.take<double>(m * per * n);
+    d.tr1 = c.take<double>(m);
+    d.tr2 = c.take<double>(m * (T - 1));
+    d.bytes = c.used;
+    return d;
+}
+// A matrix costs the FP64 loop (3 n + 1)(n^3 + n^2) FMAs and the digits (3 n + 1) n / 128 tiles whatever n:
+// 4,096 matrices of 16 took 2.1 ms by the loop and 3.9 ms by digits, 376 of 27 1.6 and 1.2 ms, 1,536 of 40
+// 29.9 and 12.8 ms (slicing, products and traces), so the line lies at 24. One tile holds up to 48 columns.
+static bool dets64_fits(int n) { return n >= 24 && n <= BN; }
+
+size_t dets64_scratch_bytes(int n, int T, int64_t nmat) {
+    if (!dets64_fits(n) || T < 2) return 0;
+    // up to 512 MB: some thousand tiles per launch
+    const size_t one = carve_dets(n, T, 1, nullptr).bytes;
+    const int64_t m = std::min<int64_t>(nmat, std::max<int64_t>(32, (int64_t)(((size_t)512 << 20) / one)));
+    return carve_dets(n, T, m, nullptr).bytes + 256;
+}
+
+bool dets64_tangents(const double* MO64, const double* Ainv64, const double* sign, int n, int T, int K, int nmat,
+                     const int* nvalid, double* g, double* lapdet, void* scratch, size_t scratch_bytes, cudaStream_t s,
+                     int* status) {
+    *status = DW_OK;
+    if (!dets64_fits(n) || T < 2 || !scratch) return false;
+    char* base = reinterpret_cast<char*>(((uintptr_t)scratch + 255) / 256 * 256);
+    const size_t lost = (size_t)(base - static_cast<char*>(scratch)), avail = scratch_bytes > lost ? scratch_bytes - lost : 0;
+    const size_t one = carve_dets(n, T, 1, nullptr).bytes;
+    int m = (int)std::min<size_t>(nmat, avail / std::max<size_t>(one, 1));
+    while (m > 0 && carve_dets(n, T, m, nullptr).bytes > avail) --m;
+    if (m < std::min(nmat, 32)) return false;
+    const int per = (T - 1) * n;
+    const DetScratch d = carve_dets(n, T, m, base);
+    auto run = [&](int m0, int nm) -> int {
+        Rows64 rows;                                 // the matrices' derivative channels: rows of n
+        rows.ngroups = 1; rows.B = nm; rows.nvalid = nvalid; rows.mul = K; rows.first = m0;
+        rows.g[0] = rows.g[1] = RowGroup{0, per, (int64_t)T * n, n};
+        Rows64 cols = rows;                          // the inverses' columns
+        cols.g[0] = cols.g[1] = RowGroup{0, n, (int64_t)n * n, 0};
+        const double* A = MO64 + (int64_t)m0 * T * n * n;
+        const double* W = Ainv64 + (int64_t)m0 * n * n;
+        slice_any(A, n, 1, n, rows, d.a, (int64_t)nm * per, s);
+        slice_any(W, 1, n, n, cols, d.w, (int64_t)nm * n, s);
+        CUtensorMap ma, mb;
+        DW_CHECK(make_map3(&ma, d.a.dig, kDig, (int)d.a.rows, d.a.Kp, d.a.Kp, d.a.rows * d.a.Kp, BK, BM, kDig, false));
+        DW_CHECK(make_map3(&mb, d.w.dig, kDig, (int)d.w.rows, d.w.Kp, d.w.Kp, d.w.rows * d.w.Kp, BK, BN, kDig, false));
+        Args64 a;
+        a.A = A; a.lda = n; a.W = nullptr; a.ldw = 0; a.C = d.E; a.ldc = n;
+        a.ea = d.a.ex; a.ew = d.w.ex;
+        a.rows = rows;
+        a.N = n; a.K = n; a.channels = 1; a.ntn = 1;
+        a.W64 = W; a.per = per;
+        a.error = tc_error_flag();
+        if (!a.error) return DW_ERR_CUDA;
+        DW_CHECK_CUDA(cudaFuncSetAttribute(k64_gemm_tc<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem64));
+        const int64_t tiles = (int64_t)nm * ((per + BM - 1) / BM);
+        k64_gemm_tc<true><<<(unsigned)std::min<int64_t>(tiles, num_sms()), kThreads64, kSmem64, s>>>(ma, mb, a);
+        count_launch();
+        k64_traces<<<(unsigned)((int64_t)nm * (T - 1)), 128, (size_t)n * (n + 1) * sizeof(double), s>>>(
+            d.E, sign + m0, n, T - 1, rows, g + (int64_t)m0 * (T - 2), d.tr1, d.tr2);
+        count_launch();
+        k64_lapdet<<<(nm + 7) / 8, 256, 0, s>>>(d.tr1, d.tr2, T - 1, rows, lapdet + m0);
+        count_launch();
+        DW_CHECK_CUDA(cudaGetLastError());
+        return DW_OK;
+    };
+    for (int m0 = 0; m0 < nmat && *status == DW_OK; m0 += m) *status = run(m0, std::min(m, nmat - m0));
+    return true;
 }
 
 }  // namespace dw

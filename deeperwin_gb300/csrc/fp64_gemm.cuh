@@ -33,7 +33,8 @@ struct Rows64 {
     int ngroups;
     RowGroup g[2];
     int B;                         // walkers
-    const int* nvalid;             // device-side walker count (null: B)
+    const int* nvalid;             // device-side walker count (null: B); valid are *nvalid mul - first
+    int mul = 1, first = 0;
 };
 inline Rows64 plain_rows(int B, int rpw, const int* nvalid) {
     Rows64 r;
@@ -58,6 +59,15 @@ struct Epi64 {
     const double* rowbias = nullptr;
     int ldrb = 0;
 };
+// FP64 determinant tangents of nmat matrices with T - 1 derivative channels (MO64 [mat][T][n][n], Ainv64
+// [mat][n][n], sign): g[mat][3 n] = tr(A^-1 dA_t), lapdet[mat] = tr(A^-1 Lap A) - sum_t tr((A^-1 dA_t)^2), as
+// digit products. K determinants per walker (nvalid counts walkers). Returns false, having done nothing,
+// where the FP64 loop is as fast (n < 24), for n > 48, or with scratch for less than 32 matrices at a time.
+size_t dets64_scratch_bytes(int n, int T, int64_t nmat);
+bool dets64_tangents(const double* MO64, const double* Ainv64, const double* sign, int n, int T, int K, int nmat,
+                     const int* nvalid, double* g, double* lapdet, void* scratch, size_t scratch_bytes, cudaStream_t s,
+                     int* status);
+
 int gemm64_tc(const double* A, int lda, const Digits& da, const Weight64& w, double* C, int ldc, const Rows64& rows,
               int channels, const Epi64& e, cudaStream_t s);
 

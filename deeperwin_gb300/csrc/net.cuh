@@ -140,8 +140,9 @@ size_t fp64_plan_bytes(const DwArch* a, int B, bool tang);
 int fp64_max_chunk(const DwArch* a, bool tang);     // walkers of one FP64 chunk
 // FP64 LU, inverse and determinant tangents of float32 Slater channels (MO layout of the forward
 // plans, d.T channels); MO64 holds Bc K T n^2 doubles, Ainv64 Bc K n^2.
+// scratch (may be null): dets64_scratch_bytes for the digit products of the tangents.
 int fp64_dets_from_f32(const float* MO, const Dims& d, int Bc, double* MO64, double* Ainv64, double* logdet,
-                       double* sign, double* g, double* lapdet, cudaStream_t s);
+                       double* sign, double* g, double* lapdet, void* scratch, size_t scratch_bytes, cudaStream_t s);
 int fp64_forward_all(const DwArch* a, const float* P, const void* prepared, const float* r, int B, const float* R,
                      const int32_t* Z, float* lp, float* phase, float* E, float* grad, bool tang, void* ws,
                      size_t ws_bytes, cudaStream_t s, const int32_t* seg, int nseg, const int* nvalid);

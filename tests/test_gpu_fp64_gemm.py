@@ -70,3 +70,33 @@ def test_rows_and_columns_outside_the_digits_range(cuda):
     # sequential FP64 sums of 40 terms, and the subnormal spacing
     bound = 40 * 2.0 ** -53 * np.abs(ref) + 40 * 40 * 2.0 ** -53 * scale + 40 * 5e-324
     assert np.all(np.abs(c[ok] - ref[ok]) <= bound[ok])
+
+
+@pytest.mark.parametrize("n_el", [23, 24, 27, 33, 40, 48, 49])
+def test_determinant_tangents_by_digits(cuda, n_el):
+    """The FP64 form's local energy across the electron counts where the determinant tangents change from the
+    FP64 loop to digit products and back: E_L and the gradient of walkers and nuclei translated together (an exact
+    symmetry; the coordinates are multiples of 2^-12, so nothing is rounded) agree to the FP32 rounding of the outputs
+    plus 1e-10 of the magnitudes summed. (Their values are pinned to the oracle in test_gpu_fp64.py, n = 34 and 40.)"""
+    from deeperwin_gb300 import api, arch as A, params as P
+    n_ions = 8
+    Z = np.array([8] * n_ions)
+    mol = A.Molecule(R=np.stack([np.arange(n_ions) * 2.0, np.arange(n_ions) % 2 * 1.5, np.zeros(n_ions)], 1), Z=Z, n_el=n_el,
+                     n_up=(n_el + 1) // 2)
+    a = A.arch_for(mol, 2)
+    p = P.init_params(a, 3, bias_std=0.1, envelope_jitter=0.2)
+    r = A.init_walkers(mol, 5, seed=9).astype(np.float32)
+    params = api.Params.from_dict(a, p, "fp64")
+    E, lp, g = api.local_energy(params, (a.n_up, a.n_dn), r, mol.R, mol.Z, return_grad=True)
+    assert bool(torch.isfinite(E).all())
+    r = np.round(r * 4096) / 4096
+    E0, lp0, g0 = api.local_energy(params, (a.n_up, a.n_dn), r, mol.R, mol.Z, return_grad=True)
+    E1, lp1, g1 = api.local_energy(params, (a.n_up, a.n_dn), r + 4.0, mol.R + 4.0, mol.Z, return_grad=True)
+    S = (g0.double() ** 2).sum(1) + E0.double().abs() + 1e3
+    assert bool(((E0.double() - E1.double()).abs() <= 2.4e-7 * E0.double().abs() + 1e-10 * S).all())
+    assert bool(((g0 - g1).abs() <= 2.4e-7 * g0.abs() + 1e-10 * g0.abs().max()).all())
+    assert L_flag() == 0
+
+
+def L_flag():
+    return _lib.lib().dw_debug_tc_error_flag()
