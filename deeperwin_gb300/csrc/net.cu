@@ -1447,13 +1447,13 @@ void launch_conv(const float* r, const float* WPl, const float* HM, const float*
     }
     count_launch();
 }
-// Envelopes by rows: grid (walker groups of kEnvWG, column chunks, spin); each thread owns one
+// Value envelopes by rows: grid (walker groups of kEnvWG, column chunks, spin); each thread owns one
 // orbital column (k, o) of one spin. softplus(alpha) and the weight of every ion for that column
-// stay in registers across all rows of the block; per (electron, ion) the difference vector,
-// distance and inverse distance are formed once in shared memory (a negative distance marks a
-// padding ion of a packed geometry). Same mathematics as k_envelope.
+// stay in registers across all rows of the block; distances are formed once per (electron, ion) in
+// shared memory (negative: a padding ion of a packed geometry), rows of an ion side by side, so that
+// one 16-byte load serves an ion's four exponentials in flight. Same mathematics as k_envelope.
 // NI bounds the ions held in registers; with NI = 8 four blocks fit an SM, which doubles the loads
-// in flight of this memory-bound kernel.
+// in flight of this memory-bound kernel. ENV_NUMBERS
 constexpr int kEnvWG = 4;
 constexpr int kEnvMaxIons = 16;
 template <int NI>
@@ -1461,24 +1461,21 @@ __global__ void __launch_bounds__(256, NI <= 8 ? 4 : 2)
 k_envelope_rows(const float* __restrict__ r, const float* __restrict__ Rall, const int32_t* __restrict__ Zall,
                 const float* __restrict__ P, ParamLayout L, const float* __restrict__ spA, Dims d, int B,
                 const float* __restrict__ BF, int ldbf, int spin_cols, float* __restrict__ MO) {
-    extern __shared__ float se[];                            // [row][ion][5]: dx, dy, dz, dist, 1/dist
+    extern __shared__ __align__(16) float se[];              // [ion][row]: distance
     const int spin = blockIdx.z;
     const int ns = spin == 0 ? d.nu : d.nd, i0 = spin == 0 ? 0 : d.nu;
     const int b0 = blockIdx.x * kEnvWG;
     const int nb = min(kEnvWG, B - b0);
-    const int rows = nb * ns, N = d.N;
-    for (int e = threadIdx.x; e < rows * N; e += blockDim.x) {
-        const int rr = e / N, I = e % N;
+    const int rows = nb * ns, N = d.N, pitch = (rows + 3) / 4 * 4;
+    for (int e = threadIdx.x; e < pitch * N; e += blockDim.x) {
+        const int rr = min(e / N, rows - 1), I = e % N;
         const int b = b0 + rr / ns, i = i0 + rr % ns;
         const int sg = seg_of(d, b);
         const float* R = Rall + (size_t)sg * N * 3;
         const float* ri = r + ((int64_t)b * d.n + i) * 3;
         const float s0 = ri[0] - R[I * 3], s1 = ri[1] - R[I * 3 + 1], s2 = ri[2] - R[I * 3 + 2];
         const float dd = sqrtf(s0 * s0 + s1 * s1 + s2 * s2);
-        float* o = se + (size_t)e * 5;
-        o[0] = s0; o[1] = s1; o[2] = s2;
-        o[3] = Zall[(size_t)sg * N + I] > 0 ? dd : -1.f;
-        o[4] = 1.f / dd;
+        se[I * pitch + e / N] = Zall[(size_t)sg * N + I] > 0 ? dd : -1.f;
     }
     __syncthreads();
     const int col = blockIdx.y * blockDim.x + threadIdx.x;
@@ -1492,74 +1489,37 @@ k_envelope_rows(const float* __restrict__ r, const float* __restrict__ Rall, con
         wv[I] = I < N ? __ldg(wts + (size_t)I * d.KN + col) : 0.f;
     }
     const int k = col / d.n, o = col - (col / d.n) * d.n;
-    const int64_t mstride = (int64_t)d.n * d.n;              // per channel
-    const bool tang = d.Tp > 1;
-    if (!tang) {
-        // value rows four at a time: the four backflow loads are in flight together
-        for (int r4 = 0; r4 < rows; r4 += 4) {
-            float bfv[4], env4[4];
-            #pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                const int rr = min(r4 + u, rows - 1);
-                const int b = b0 + rr / ns, i = i0 + rr % ns;
-                bfv[u] = __ldg(BF + ((int64_t)b * d.n + i) * ldbf + (spin ? spin_cols : 0) + col);
-            }
-            #pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                const float* gv = se + (size_t)min(r4 + u, rows - 1) * N * 5;
-                float env = 0.f;
-                #pragma unroll
-                for (int I = 0; I < NI; ++I) {
-                    if (I >= N) break;
-                    const float dd = gv[I * 5 + 3];
-                    if (dd < 0.f) continue;                  // padding ion
-                    env += wv[I] * expf(-av[I] * dd);
-                }
-                env4[u] = env;
-            }
-            #pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                if (r4 + u >= rows) break;
-                const int rr = r4 + u, b = b0 + rr / ns, i = i0 + rr % ns;
-                MO[((int64_t)b * d.K + k) * mstride + i * d.n + o] = env4[u] * bfv[u];
+    const int64_t mstride = (int64_t)d.n * d.n;              // per determinant
+    // rows four at a time: the four backflow loads are in flight together
+    int b = b0, i = 0;                                        // walker and electron (of this spin) of row r4
+    for (int r4 = 0; r4 < rows; r4 += 4) {
+        float bfv[4], env[4] = {0.f, 0.f, 0.f, 0.f};
+        float* mo[4];
+        #pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            if (r4 + u < rows) {
+                bfv[u] = __ldg(BF + ((int64_t)b * d.n + i0 + i) * ldbf + (spin ? spin_cols : 0) + col);
+                mo[u] = MO + ((int64_t)b * d.K + k) * mstride + (i0 + i) * d.n + o;
+                if (++i == ns) { i = 0; ++b; }
+            } else {
+                bfv[u] = 0.f;
+                mo[u] = nullptr;
             }
         }
-        return;
-    }
-    for (int rr = 0; rr < rows; ++rr) {
-        const int b = b0 + rr / ns, i = i0 + rr % ns;
-        const float* gv = se + (size_t)rr * N * 5;
-        float env = 0.f, g0 = 0.f, g1 = 0.f, g2 = 0.f, lapv = 0.f;
         #pragma unroll
         for (int I = 0; I < NI; ++I) {
             if (I >= N) break;
-            const float dd = gv[I * 5 + 3];
-            if (dd < 0.f) continue;                          // padding ion
-            const float a = av[I];
-            const float e = wv[I] * expf(-a * dd);
-            env += e;
-            if (tang) {
-                const float inv = gv[I * 5 + 4];
-                const float gs = -a * e * inv;
-                g0 += gs * gv[I * 5]; g1 += gs * gv[I * 5 + 1]; g2 += gs * gv[I * 5 + 2];
-                lapv += e * (a * a - 2.f * a * inv);
+            const float4 d4 = *reinterpret_cast<const float4*>(se + I * pitch + r4);
+            const float dd[4] = {d4.x, d4.y, d4.z, d4.w};
+            #pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const float x = fmaf(wv[I], expf(-av[I] * dd[u]), env[u]);
+                env[u] = dd[u] < 0.f ? env[u] : x;            // padding ion
             }
         }
-        const float* bf = BF + ((int64_t)b * d.n + i) * d.Tp * ldbf + (spin ? spin_cols : 0) + col;
-        float* mo = MO + (((int64_t)b * d.K + k) * d.T) * mstride + i * d.n + o;
-        const float bf0 = bf[0];
-        mo[0] = env * bf0;
-        if (!tang) continue;
-        for (int t = 1; t <= 3 * d.n; ++t) {
-            float v = env * bf[(int64_t)t * ldbf];
-            const unsigned c = (unsigned)(t - 1 - 3 * i);     // own coordinate channels
-            if (c < 3u) v += (c == 0 ? g0 : (c == 1 ? g1 : g2)) * bf0;
-            mo[t * mstride] = v;
-        }
-        float vl = env * bf[(int64_t)d.lap * ldbf] + lapv * bf0;
-        vl += 2.f * (g0 * bf[(int64_t)(1 + 3 * i) * ldbf] + g1 * bf[(int64_t)(2 + 3 * i) * ldbf] +
-                     g2 * bf[(int64_t)(3 + 3 * i) * ldbf]);
-        mo[d.lap * mstride] = vl;
+        #pragma unroll
+        for (int u = 0; u < 4; ++u)
+            if (mo[u]) *mo[u] = env[u] * bfv[u];
     }
 }
 
@@ -1571,7 +1531,7 @@ void launch_envelope(const float* r, const float* R, const int32_t* Z, const flo
     if (d.N <= kEnvMaxIons && d.Tp == 1) {
         const int threads = std::min(256, round_up(d.KN, 32));
         const int ns_max = std::max(d.nu, d.nd);
-        const size_t sm = (size_t)kEnvWG * ns_max * d.N * 5 * sizeof(float);
+        const size_t sm = (size_t)((kEnvWG * ns_max + 3) / 4 * 4) * d.N * sizeof(float);
         dim3 grid((unsigned)((B + kEnvWG - 1) / kEnvWG), (unsigned)((d.KN + threads - 1) / threads), d.nd > 0 ? 2 : 1);
         if (d.N <= 8) k_envelope_rows<8><<<grid, threads, sm, s>>>(r, R, Z, P, L, sp_alpha, d, B, BF, ldbf, spin_cols, MO);
         else k_envelope_rows<16><<<grid, threads, sm, s>>>(r, R, Z, P, L, sp_alpha, d, B, BF, ldbf, spin_cols, MO);
