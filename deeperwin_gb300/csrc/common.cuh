@@ -110,6 +110,15 @@ __device__ __forceinline__ float softplus_f(float x) {
     return fmaxf(x, 0.f) + log1pf(expf(-fabsf(x)));
 }
 
+// Two FP32 FMAs in one instruction (each rounded as fmaf).
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+    float2 d;
+    asm("{\n .reg .b64 x, y, z;\n mov.b64 x, {%2, %3};\n mov.b64 y, {%4, %5};\n mov.b64 z, {%6, %7};\n"
+        " fma.rn.f32x2 z, x, y, z;\n mov.b64 {%0, %1}, z;\n}\n"
+        : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+    return d;
+}
+
 // Philox-4x32-10 counter-based generator (Salmon, Moraes, Dror, Shaw, "Parallel random
 // numbers: as easy as 1, 2, 3", SC'11). Round multipliers and Weyl key increments are
 // the published Philox4x32 constants.

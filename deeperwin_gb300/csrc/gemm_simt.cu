@@ -18,15 +18,6 @@ static int num_sms_simt() {
     return n;
 }
 
-// Two FP32 FMAs in one instruction (each rounded as fmaf).
-__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
-    float2 d;
-    asm("{\n .reg .b64 x, y, z;\n mov.b64 x, {%2, %3};\n mov.b64 y, {%4, %5};\n mov.b64 z, {%6, %7};\n"
-        " fma.rn.f32x2 z, x, y, z;\n mov.b64 {%0, %1}, z;\n}\n"
-        : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
-    return d;
-}
-
 template <int BM, int BN, int BK, int TM, int TN, bool TRANS_W = false, bool ACC = false>
 __global__ void __launch_bounds__((BM / TM) * (BN / TN))
 k_gemm_f32(const float* __restrict__ A, int lda, const float* __restrict__ W, int ldw, float* __restrict__ C, int ldc,

@@ -258,13 +258,45 @@ __device__ __forceinline__ void mlp_tile(const MlpSmem& sm, int cur, int in_w, i
     }
 }
 
+// Two products of the same rows at once (weights sm.W and W2, biases sm.bias and bias2): one load of 4
+// rows serves both, and each weight pair is one paired FMA (rounded as fmaf).
+__device__ __forceinline__ void mlp_tile2(const MlpSmem& sm, const float* W2, const float* bias2, int cur, int in_w, int rg,
+                                          int fg, float (&z)[4][4], float (&y)[4][4]) {
+    float2 a[4][2], c[4][2];
+    const float4 b4 = *reinterpret_cast<const float4*>(&sm.bias[4 * fg]), d4 = *reinterpret_cast<const float4*>(bias2 + 4 * fg);
+    #pragma unroll
+    for (int rr = 0; rr < 4; ++rr) {
+        a[rr][0] = make_float2(b4.x, b4.y); a[rr][1] = make_float2(b4.z, b4.w);
+        c[rr][0] = make_float2(d4.x, d4.y); c[rr][1] = make_float2(d4.z, d4.w);
+    }
+    #pragma unroll 8
+    for (int k = 0; k < in_w; ++k) {
+        const float4 h4 = *reinterpret_cast<const float4*>(&sm.H[cur][k][4 * rg]);
+        const float4 w4 = *reinterpret_cast<const float4*>(&sm.W[k * 32 + 4 * fg]);
+        const float4 v4 = *reinterpret_cast<const float4*>(W2 + k * 32 + 4 * fg);
+        const float hv[4] = {h4.x, h4.y, h4.z, h4.w};
+        #pragma unroll
+        for (int rr = 0; rr < 4; ++rr) {
+            const float2 h = make_float2(hv[rr], hv[rr]);
+            a[rr][0] = fma2(h, make_float2(w4.x, w4.y), a[rr][0]); a[rr][1] = fma2(h, make_float2(w4.z, w4.w), a[rr][1]);
+            c[rr][0] = fma2(h, make_float2(v4.x, v4.y), c[rr][0]); c[rr][1] = fma2(h, make_float2(v4.z, v4.w), c[rr][1]);
+        }
+    }
+    #pragma unroll
+    for (int rr = 0; rr < 4; ++rr) {
+        z[rr][0] = a[rr][0].x; z[rr][1] = a[rr][0].y; z[rr][2] = a[rr][1].x; z[rr][3] = a[rr][1].y;
+        y[rr][0] = c[rr][0].x; y[rr][1] = c[rr][0].y; y[rr][2] = c[rr][1].x; y[rr][3] = c[rr][1].y;
+    }
+}
+
 // Blocks [0, blocks_same) take same-spin pairs (up-up then down-down, i <= j), the rest the
-// up-down pairs. WP[l][b][i n + j][32] gets both orders; HP (optional) the stream levels 1..3
+// up-down pairs. A level's convolution weights and its stream layer are formed in one pass. WP[l][b][i n + j][32] gets both orders; HP (optional) the stream levels 1..3
 // at the unordered-pair index used by the backward pass.
 __global__ void __launch_bounds__(128)
 k_pair_mlp(const float* __restrict__ r, const float* __restrict__ P, ParamLayout L, Dims d, int B, int blocks_same,
            float* __restrict__ WP, float* __restrict__ HP) {
     __shared__ __align__(16) MlpSmem sm;
+    __shared__ __align__(16) float W2[32 * 32], bias2[32];
     __shared__ int rw[kRB], ri[kRB], rj[kRB];
     const int tid = threadIdx.x;
     const int n = d.n, nu = d.nu, nd = d.nd;
@@ -307,9 +339,15 @@ k_pair_mlp(const float* __restrict__ r, const float* __restrict__ P, ParamLayout
         const int in_w = d.eew[l];
         __syncthreads();
         mlp_load_w(sm, P + (same ? L.w_same_w[l] : L.w_diff_w[l]), P + (same ? L.w_same_b[l] : L.w_diff_b[l]), in_w);
+        if (l < 3) {
+            const float* w = P + (same ? L.h_same_w[l] : L.h_diff_w[l]);
+            for (int e = tid; e < in_w * 32; e += blockDim.x) W2[e] = __ldg(w + e);
+            if (tid < 32) bias2[tid] = __ldg(P + (same ? L.h_same_b[l] : L.h_diff_b[l]) + tid);
+        }
         __syncthreads();
-        float z[4][4];
-        mlp_tile(sm, cur, in_w, rg, fg, z);
+        float z[4][4], zs[4][4];
+        if (l < 3) mlp_tile2(sm, W2, bias2, cur, in_w, rg, fg, z, zs);
+        else mlp_tile(sm, cur, in_w, rg, fg, z);
         #pragma unroll
         for (int rr = 0; rr < 4; ++rr) {
             const int q = 4 * rg + rr, b = rw[q];
@@ -321,10 +359,6 @@ k_pair_mlp(const float* __restrict__ r, const float* __restrict__ P, ParamLayout
             if (i != j) *reinterpret_cast<float4*>(WP + (wb + j * n + i) * 32 + 4 * fg) = v;
         }
         if (l == 3) break;
-        __syncthreads();
-        mlp_load_w(sm, P + (same ? L.h_same_w[l] : L.h_diff_w[l]), P + (same ? L.h_same_b[l] : L.h_diff_b[l]), in_w);
-        __syncthreads();
-        mlp_tile(sm, cur, in_w, rg, fg, z);
         #pragma unroll
         for (int rr = 0; rr < 4; ++rr) {
             const int q = 4 * rg + rr;
@@ -332,7 +366,7 @@ k_pair_mlp(const float* __restrict__ r, const float* __restrict__ P, ParamLayout
             #pragma unroll
             for (int ff = 0; ff < 4; ++ff) {
                 const int f = 4 * fg + ff;
-                const float y = tanhf(z[rr][ff]);
+                const float y = tanhf(zs[rr][ff]);
                 hn[ff] = l > 0 ? (sm.H[cur][f][q] + y) * rs : y;        // residual (mlp.py:13-17)
                 sm.H[cur ^ 1][f][q] = hn[ff];
             }
