@@ -979,11 +979,14 @@ __global__ void k_conv(const float* __restrict__ r, const float* __restrict__ WP
 // eight at a time (16-byte stores). conv_ei is non-zero on 5 channels per electron only. Same
 // mathematics as k_conv. Bound by the latency of its loads between barriers: the pair geometry is formed
 // once per block (a square root and a division per term before), only the warps with channels are
-// launched, and two j are in flight. Per local energy: H10, 8,192 walkers 3.36 -> 2.62 ms, C2H4, 4,096
-// walkers 4.08 -> 3.57 ms, 27 electrons, 1,500 walkers 7.1 -> 6.1 ms. (Keeping the tile in registers to the
-// store instead of staging it took 2.5 times as long.)
+// launched, and two j of the main loop and of the product-rule sums and four single terms are in flight.
+// Its working set in L1 (the h_map rows of the walkers in flight) sets the rest: 64 registers is the best
+// point, with more blocks per SM (56 or 48 registers, or the partials in the tile's memory) or more loads in
+// flight (three or four j) it is slower, up to twice. Per local energy: H10, 8,192 walkers 3.36 -> 2.62 ms,
+// C2H4, 4,096 walkers 4.08 -> 3.37 ms, 27 electrons, 1,500 walkers 7.1 -> 5.6 ms. (Keeping the tile in
+// registers to the store instead of staging it took 2.5 times as long.)
 template <class Act, int TT, int TI>
-__global__ void __launch_bounds__(512)
+__global__ void __launch_bounds__(512, 2)
 k_conv_tile(const float* __restrict__ r, const float* __restrict__ WPl, const float* __restrict__ HM,
             const float* __restrict__ HEl, const float* __restrict__ himl, Dims d, int l, int B, Act* __restrict__ X,
             int ldx, int ei_fused, int G) {
@@ -1040,19 +1043,21 @@ k_conv_tile(const float* __restrict__ r, const float* __restrict__ WPl, const fl
     for (int it = w; it < G * ni; it += NW) {
         const int q = it / ni, ii = it % ni, i = i0 + ii;
         float o0 = 0.f, o1 = 0.f, o2 = 0.f, ol = 0.f;
+        #pragma unroll 2
         for (int j = q; j < n; j += G) {
-            if (j == i) continue;
             const float* wr = wpb + ((size_t)i * n + j) * 96;
             const float* hj = hmb + (size_t)j * Tp * 32;
             const float w1 = __ldg(wr + 32), w2 = __ldg(wr + 64), h0 = __ldg(hj);
+            const float gx = __ldg(hj + (1 + 3 * j) * 32) - __ldg(hj + (1 + 3 * i) * 32), gy = __ldg(hj + (2 + 3 * j) * 32) - __ldg(hj + (2 + 3 * i) * 32),
+                        gz = __ldg(hj + (3 + 3 * j) * 32) - __ldg(hj + (3 + 3 * i) * 32);
             const float4 u = geo[ii * n + j];
             const float inv = u.w;
             const float ux = u.x * inv, uy = u.y * inv, uz = u.z * inv;
-            o0 += w1 * ux * h0; o1 += w1 * uy * h0; o2 += w1 * uz * h0;
-            const float cross = ux * (__ldg(hj + (1 + 3 * j) * 32) - __ldg(hj + (1 + 3 * i) * 32)) +
-                                uy * (__ldg(hj + (2 + 3 * j) * 32) - __ldg(hj + (2 + 3 * i) * 32)) +
-                                uz * (__ldg(hj + (3 + 3 * j) * 32) - __ldg(hj + (3 + 3 * i) * 32));
-            ol += 2.f * (w2 + 2.f * w1 * inv) * h0 + 2.f * w1 * cross;
+            const float cross = ux * gx + uy * gy + uz * gz;
+            const float p0 = o0 + w1 * ux * h0, p1 = o1 + w1 * uy * h0, p2 = o2 + w1 * uz * h0;
+            const float pl = ol + (2.f * (w2 + 2.f * w1 * inv) * h0 + 2.f * w1 * cross);
+            const bool on = j != i;                     // (0 * inf of the electron itself is not selected)
+            o0 = on ? p0 : o0; o1 = on ? p1 : o1; o2 = on ? p2 : o2; ol = on ? pl : ol;
         }
         float* rr = red + ((q * TI + ii) * 4) * 32 + f;
         rr[0] = o0; rr[32] = o1; rr[64] = o2; rr[96] = ol;
@@ -1073,25 +1078,37 @@ k_conv_tile(const float* __restrict__ r, const float* __restrict__ WPl, const fl
         eiv[(ii * 5 + ch) * 32 + f] = v;
     }
     __syncthreads();
-    // single product-rule terms: channel 1 + 3m + c of electron i gains w'_im u_im,c h_m,0 (m != i)
-    for (int it = w; it < ni * n; it += NW) {
-        const int ii = it / n, m = it % n, i = i0 + ii;
-        float* o = out + (ii * Tp) * 32 + f;
-        if (m == i) {
-            float s0 = 0.f, s1 = 0.f, s2 = 0.f, sl = 0.f;
-            for (int q = 0; q < G; ++q) {
-                const float* rr = red + ((q * TI + ii) * 4) * 32 + f;
-                s0 += rr[0]; s1 += rr[32]; s2 += rr[64]; sl += rr[96];
+    // single product-rule terms: channel 1 + 3m + c of electron i gains w'_im u_im,c h_m,0 (m != i), U
+    // terms per round so that their loads overlap
+    constexpr int U = 4;
+    for (int it0 = w; it0 < ni * n; it0 += U * NW) {
+        float g[U];
+        int ii[U], m[U];
+        #pragma unroll
+        for (int x = 0; x < U; ++x) {
+            const int it = min(it0 + x * NW, ni * n - 1);
+            ii[x] = it / n; m[x] = it - ii[x] * n;
+            g[x] = __ldg(wpb + ((size_t)(i0 + ii[x]) * n + m[x]) * 96 + 32) * __ldg(hmb + (size_t)m[x] * Tp * 32);
+        }
+        #pragma unroll
+        for (int x = 0; x < U; ++x) {
+            if (it0 + x * NW >= ni * n) break;
+            float* o = out + (ii[x] * Tp + 1 + 3 * m[x]) * 32 + f;
+            if (m[x] == i0 + ii[x]) {
+                float s0 = 0.f, s1 = 0.f, s2 = 0.f, sl = 0.f;
+                for (int q = 0; q < G; ++q) {
+                    const float* rr = red + ((q * TI + ii[x]) * 4) * 32 + f;
+                    s0 += rr[0]; s1 += rr[32]; s2 += rr[64]; sl += rr[96];
+                }
+                o[0] -= s0; o[32] -= s1; o[64] -= s2;
+                out[(ii[x] * Tp + d.lap) * 32 + f] += sl;
+            } else {
+                const float4 u = geo[ii[x] * n + m[x]];
+                const float gu = g[x] * u.w;
+                o[0] = fmaf(gu, u.x, o[0]);
+                o[32] = fmaf(gu, u.y, o[32]);
+                o[64] = fmaf(gu, u.z, o[64]);
             }
-            o[(1 + 3 * i) * 32] -= s0; o[(2 + 3 * i) * 32] -= s1; o[(3 + 3 * i) * 32] -= s2;
-            o[d.lap * 32] += sl;
-        } else {
-            const float4 u = geo[ii * n + m];
-            const float dx = u.x, dy = u.y, dz = u.z;
-            const float g = __ldg(wpb + ((size_t)i * n + m) * 96 + 32) * __ldg(hmb + (size_t)m * Tp * 32) * u.w;
-            o[(1 + 3 * m) * 32] = fmaf(g, dx, o[(1 + 3 * m) * 32]);
-            o[(2 + 3 * m) * 32] = fmaf(g, dy, o[(2 + 3 * m) * 32]);
-            o[(3 + 3 * m) * 32] = fmaf(g, dz, o[(3 + 3 * m) * 32]);
         }
     }
     __syncthreads();
