@@ -1082,8 +1082,9 @@ k_det_tangents_warp(const float* __restrict__ MO, const float* __restrict__ Ainv
 // transposed tile for its part of tr(C_t^2). A channel's traces are FP32 sums of products of
 // FP32 entries (as C_t itself is FP32), formed from the tile partials by one lane per channel;
 // the traces of all channels are accumulated in FP64 into
-// lap = tr(A^-1 Lap A) - sum_t tr(C_t^2). Matrices are zero-padded to NP = round_up(n, 4) for n <= 32
-// and to 40 for n = 33..40 (a channel's 100 tiles then leave 28 of the 128 threads idle).
+// lap = tr(A^-1 Lap A) - sum_t tr(C_t^2). Matrices are zero-padded to NP = round_up(n, 4).
+// Used for n <= 12; above that k_det_tangents_t8 is the faster (its comment), and the wider
+// instantiations serve as its oracle in the tests.
 template <int NP>
 __global__ void __launch_bounds__(128)
 k_det_tangents_tile(const float* __restrict__ MO, const float* __restrict__ Ainv, const double* __restrict__ sign,
@@ -1677,8 +1678,8 @@ int dw_debug_slogdet_small(const float* MO, int n, int T, int nmat, int scalar, 
 }
 
 // Instrumentation: determinant-tangent kernels (0: the default choice; 1: the single-buffer tile
-// kernel for n in {4, 8, 16} instead of the pipelined one, and the general kernel instead of the
-// tile kernel for n = 33..40). Returns the previous choice.
+// kernel for n <= 32 and the general kernel for n = 33..40, in place of the pipelined and the
+// 8 x 8 ones). Returns the previous choice.
 int dw_debug_set_det_tangents_kernel(int which) {
     if (which != 0 && which != 1) return -DW_ERR_ARG;
     const int old = dw::g_det_tangents_tile ? 1 : 0;

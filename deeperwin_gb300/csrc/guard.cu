@@ -37,7 +37,7 @@ constexpr float kGuardTol = 0.015f;
 // traces). The catastrophic errors of ill-conditioned walkers come from the determinant algebra:
 // on 4,096 C2H4-shaped walkers near the initial weights the plain FP32 form is off by up to 14 Ha,
 // the same network with FP64 determinants by at most 95 mHa (mean 0.03 mHa), at about 1.5x the
-// plain form's cost per walker. The FP64 form (fp64.cu) would cost about 15x more per walker.
+// plain form's cost per walker. The FP64 form (fp64.cu) costs about 5.5 times the plain form.
 // Second tier: walkers whose cancelled magnitude exceeds kGuardFp64Key Ha. At the end of the C2H4
 // optimisation bench (random-init weights after 14 Adam steps) 4-37 of 4,096 walkers exceed it; the
 // FP32 network with FP64 determinants is off by 0.1-4 Ha on those between 1e5 and 1e7 and by up to
@@ -165,7 +165,7 @@ int guard_capacity(const DwArch* a, int B) {
 
 // second tier: up to 1 / 128 of the batch (at least 8) in one FP64 chunk; its kernels skip the
 // unused capacity through the device-side count, so it costs FP64 work only for the walkers
-// flagged (about 0.6 ms per C2H4-shaped walker)
+// flagged (0.14 ms per C2H4-shaped walker)
 static int guard64_capacity(const DwArch* a, int B) {
     return std::max(1, std::min(std::min(B, std::max(8, (B + 127) / 128)), fp64_max_chunk(a, true)));
 }
