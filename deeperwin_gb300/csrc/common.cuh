@@ -94,6 +94,13 @@ struct Carver {
     bool ok() const { return dry || used <= cap; }
 };
 
+// Allows launches of a kernel with up to `bytes` of dynamic shared memory. The limit belongs to the kernel, not
+// to a launch, and all threads of the process share it: `bytes` is the most that any launch of the kernel
+// takes, never one launch's own size, which would make another thread's larger launch fail.
+template <class K> inline cudaError_t allow_smem(K kernel, int bytes) {
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+}
+
 // ------------------------------------------------------------------ device helpers
 __device__ __forceinline__ float warp_sum(float v) {
     #pragma unroll

@@ -920,23 +920,23 @@ void launch_slogdet_impl(const float* MO, const Dims& d, int B, double* logdet, 
         count_launch();
         return;
     }
+    constexpr int kWideSmem = 96 * 1024;                     // at least one matrix of 64 fits
     if (!want_inv && n <= 64) {
         const size_t per = (size_t)n * (n + 1) * sizeof(S);
-        int wpb = (int)(96 * 1024 / per);
+        int wpb = (int)(kWideSmem / per);
         wpb = wpb < 1 ? 1 : (wpb > 8 ? 8 : wpb);
         const size_t sm = per * wpb;
-        if (sm > 48 * 1024) cudaFuncSetAttribute(k_slogdet_wide<S>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+        if (sm > 48 * 1024) allow_smem(k_slogdet_wide<S>, kWideSmem);
         k_slogdet_wide<S><<<(nmat + wpb - 1) / wpb, wpb * 32, sm, s>>>(MO, n, d.T, nmat, logdet, sign);
         count_launch();
         return;
     }
     if (want_inv && n <= 64) {
         const size_t per = (size_t)n * (2 * n + 1) * sizeof(S);
-        int wpb = (int)(96 * 1024 / per);
+        int wpb = (int)(kWideSmem / per);
         wpb = wpb < 1 ? 1 : (wpb > 8 ? 8 : wpb);
         const size_t sm = per * wpb;
-        if (sm > 48 * 1024)
-            cudaFuncSetAttribute(k_slogdet_wide_inv<S>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+        if (sm > 48 * 1024) allow_smem(k_slogdet_wide_inv<S>, kWideSmem);
         k_slogdet_wide_inv<S><<<(nmat + wpb - 1) / wpb, wpb * 32, sm, s>>>(MO, n, d.T, nmat, logdet, sign, Ainv);
         count_launch();
         return;

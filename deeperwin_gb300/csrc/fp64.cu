@@ -489,7 +489,7 @@ static int launch_tangents64(const double* MO, const double* Ainv, const double*
     int status = DW_OK;
     if (dets64_tangents(MO, Ainv, sign, n, q.C, q.d.K, nmat, q.nvalid, g, lapdet, scratch, scratch_bytes, s, &status)) return status;
     const size_t sm = (size_t)3 * n * n * sizeof(double);
-    if (sm > 48 * 1024) cudaFuncSetAttribute(k64_det_tangents, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    if (sm > 48 * 1024) allow_smem(k64_det_tangents, 3 * kMaxEl * kMaxEl * (int)sizeof(double));
     k64_det_tangents<<<nmat, 128, sm, s>>>(MO, Ainv, sign, q, g, lapdet);
     count_launch();
     return DW_OK;
@@ -675,7 +675,7 @@ static int run_chunk64(const Plan64& p, const Dims& d0, int Bc, const float* P, 
     count_launch();
     const int nmat = Bc * d.K;
     const size_t sm_lu = ((size_t)n * (2 * n + 1) + n) * sizeof(double);
-    if (sm_lu > 48 * 1024) cudaFuncSetAttribute(k64_slogdet_inv, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_lu);
+    if (sm_lu > 48 * 1024) allow_smem(k64_slogdet_inv, (kMaxEl * (2 * kMaxEl + 1) + kMaxEl) * (int)sizeof(double));
     timer_begin("fp64_lu", s);
     k64_slogdet_inv<<<nmat, 128, sm_lu, s>>>(p.MO, q, p.logdet, p.sign, tang ? p.Ainv : nullptr);
     timer_end("fp64_lu", s, 0.0, 0.0);
@@ -723,7 +723,7 @@ int fp64_dets_from_f32(const float* MO, const Dims& d, int Bc, double* MO64, dou
     count_launch();
     const bool tang = d.T > 1;
     const size_t sm_lu = ((size_t)n * (2 * n + 1) + n) * sizeof(double);
-    if (sm_lu > 48 * 1024) cudaFuncSetAttribute(k64_slogdet_inv, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_lu);
+    if (sm_lu > 48 * 1024) allow_smem(k64_slogdet_inv, (kMaxEl * (2 * kMaxEl + 1) + kMaxEl) * (int)sizeof(double));
     k64_slogdet_inv<<<nmat, 128, sm_lu, s>>>(MO64, q, logdet, sign, tang ? Ainv64 : nullptr);
     count_launch();
     if (tang) DW_CHECK(launch_tangents64(MO64, Ainv64, sign, q, nmat, g, lapdet, scratch, scratch_bytes, s));

@@ -541,7 +541,7 @@ int gemm64_tc(const double* A, int lda, const Digits& da, const Weight64& w, dou
     if (!a.error) return DW_ERR_CUDA;
     int64_t tiles = 0;
     for (int g = 0; g < rows.ngroups; ++g) tiles += ((int64_t)rows.B * rows.g[g].rpw + BM - 1) / BM * a.ntn;
-    DW_CHECK_CUDA(cudaFuncSetAttribute(k64_gemm_tc<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem64));
+    DW_CHECK_CUDA(allow_smem(k64_gemm_tc<false>, kSmem64));
     timer_begin("fp64_gemm", s);
     k64_gemm_tc<false><<<(unsigned)std::min<int64_t>(tiles, num_sms()), kThreads64, kSmem64, s>>>(ma, mb, a);
     timer_end("fp64_gemm", s, 0.0, 0.0);
@@ -616,7 +616,7 @@ bool dets64_tangents(const double* MO64, const double* Ainv64, const double* sig
         a.W64 = W; a.per = per;
         a.error = tc_error_flag();
         if (!a.error) return DW_ERR_CUDA;
-        DW_CHECK_CUDA(cudaFuncSetAttribute(k64_gemm_tc<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem64));
+        DW_CHECK_CUDA(allow_smem(k64_gemm_tc<true>, kSmem64));
         const int64_t tiles = (int64_t)nm * ((per + BM - 1) / BM);
         k64_gemm_tc<true><<<(unsigned)std::min<int64_t>(tiles, num_sms()), kThreads64, kSmem64, s>>>(ma, mb, a);
         count_launch();

@@ -52,6 +52,7 @@ constexpr int kThreads = 64 + 128 * kSets;
 constexpr int kBufCols = kTileRows;                  // TMEM columns of a buffer
 constexpr int kLdRb = 256;                           // row pitch of the row bias (the layer width)
 constexpr int kMaxStages = 8;
+constexpr int kSmemMax = 226 * 1024;                 // dynamic shared memory of a CTA at most (1 KB aligned)
 
 struct JetArgs {
     int NF, K, nk;                                   // features, reduction width, stages per tile
@@ -556,7 +557,7 @@ int launch_jet_cg(const __nv_bfloat16* A, int lda, const __nv_bfloat16* W0, cons
         }
         a.x_part = a.ncol * BK * 2;
         stage = NP * a.x_part;
-        a.stages = std::min(kMaxStages, (227 * 1024 - fixed - w_bytes) / stage);
+        a.stages = std::min(kMaxStages, (kSmemMax - fixed - w_bytes) / stage);
         if (a.stages >= 2) break;
     }
     if (a.stages < 2) return DW_ERR_ARCH;
@@ -576,7 +577,7 @@ int launch_jet_cg(const __nv_bfloat16* A, int lda, const __nv_bfloat16* W0, cons
     }
     const size_t smem = (size_t)fixed + w_bytes + (size_t)a.stages * stage;
     auto kern = k_gemm_jet<NP, OUT, EPI, LDC, CG>;
-    DW_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    DW_CHECK_CUDA(allow_smem(kern, kSmemMax));
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(CG * std::min<int64_t>(a.units, num_sms() / CG)));
     cfg.blockDim = dim3(kThreads);

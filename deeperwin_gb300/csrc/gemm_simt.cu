@@ -320,7 +320,7 @@ void gemm_f32(const float* A, int lda, const float* W, int ldw, float* C, int ld
     // means 62 -> 27 us, layers 45 -> 43 us, h_map 24 -> 16 us, Jastrow 62 -> 35 us.
     if (batch == 1 && M <= kTinyM && K <= kTinyK) {
         const size_t sm = (size_t)K * (32 + 8) * sizeof(float);
-        if (sm > 48 * 1024) cudaFuncSetAttribute(k_gemm_f32_tiny, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+        if (sm > 48 * 1024) allow_smem(k_gemm_f32_tiny, kTinyK * (32 + 8) * (int)sizeof(float));
         k_gemm_f32_tiny<<<dim3((N + 31) / 32, (M + 7) / 8), 256, sm, s>>>(A, lda, W, ldw, C, ldc, M, N, K, epi);
         count_launch();
         return;

@@ -109,6 +109,7 @@ constexpr int BM = 128;
 constexpr int kEpiWarps = 8;                         // two per TMEM lane quarter
 constexpr int kThreads = 64 + 32 * kEpiWarps;        // producer warp, MMA warp, epilogue warps
 constexpr int CW = 32;                               // columns per epilogue chunk / staged store box
+constexpr int kSmemMax = 220 * 1024;                 // dynamic shared memory of a CTA at most
 
 // named barrier 1: all epilogue warps
 __device__ __forceinline__ void epi_bar() { asm volatile("bar.sync 1, %0;" ::"n"(32 * kEpiWarps) : "memory"); }
@@ -394,7 +395,7 @@ int launch_tc(const __nv_bfloat16* A, int lda, const __nv_bfloat16* W0, const __
     a.M = M; a.N = N; a.K = K; a.BN = BN; a.epi = epi;
     const int stage_bytes = NP * (BM * BK * 2 + BN * BK * 2);
     const int fixed = 1024 + 2 * kEpiWarps * 4096 + 256;
-    a.stages = std::min(8, (220 * 1024 - fixed) / stage_bytes);
+    a.stages = std::min(8, (kSmemMax - fixed) / stage_bytes);
     if (a.stages < 2) return DW_ERR_ARCH;
     a.tmem_cols = 32;
     while ((int)a.tmem_cols < 2 * BN) a.tmem_cols <<= 1;
@@ -403,7 +404,7 @@ int launch_tc(const __nv_bfloat16* A, int lda, const __nv_bfloat16* W0, const __
     a.n_tiles = mt * ntn;
     size_t smem = (size_t)fixed + (size_t)a.stages * stage_bytes;
     auto kern = k_gemm_tc<NP, OUT, BK>;
-    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    DW_CHECK_CUDA(allow_smem(kern, kSmemMax));
     int grid = std::min(a.n_tiles, num_sms());
     kern<<<grid, kThreads, smem, s>>>(ma0, ma1, mb0, mb1, mc0, mc1, a);
     count_launch();

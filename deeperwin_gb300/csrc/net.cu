@@ -1479,9 +1479,12 @@ void launch_conv(const float* r, const float* WPl, const float* HM, const float*
         const unsigned grid = (unsigned)B * ((d.n + TI - 1) / TI);
         const int rows = next_pow2(d.Tp), TT = rows >= 64 ? 8 : rows / 8;
         const int G = rows / TT, NW = (d.Tp + TT - 1) / TT;
-        const size_t smem = ((size_t)TI * d.Tp * 32 + (size_t)G * TI * 4 * 32 + (size_t)TI * 5 * 32 + (size_t)TI * d.n * 4) * sizeof(float);
+        auto bytes = [](int n, int T, int g) {
+            return (int)((TI * T * 32 + g * TI * 4 * 32 + TI * 5 * 32 + TI * n * 4) * sizeof(float));
+        };
+        const size_t smem = bytes(d.n, d.Tp, G);
         auto go = [&](auto kern) {
-            cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+            allow_smem(kern, bytes(kMaxEl, 128, 16));
             kern<<<grid, NW * 32, smem, s>>>(r, WPl, HM, HEl, himl, d, l, B, X, ldx, ei_fused, G);
         };
         auto pick = [&](auto ti) {
@@ -1505,9 +1508,9 @@ void launch_conv(const float* r, const float* WPl, const float* HM, const float*
         return;
     }
     const size_t smem = ((size_t)d.n * d.Tp * 32 + (size_t)d.n * d.n * 4) * sizeof(float);
-    if (smem <= 200 * 1024) {
-        if (smem > 48 * 1024)
-            cudaFuncSetAttribute(k_conv_walker<Act>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    constexpr int kWalkerSmem = 200 * 1024;
+    if (smem <= kWalkerSmem) {
+        if (smem > 48 * 1024) allow_smem(k_conv_walker<Act>, kWalkerSmem);
         k_conv_walker<Act><<<B, 256, smem, s>>>(r, WPl, HM, HEl, himl, d, l, B, X, ldx);
     } else {
         k_conv<Act><<<B * d.n, 256, 0, s>>>(r, WPl, HM, HEl, himl, d, l, B, X, ldx);
