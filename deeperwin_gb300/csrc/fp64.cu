@@ -367,7 +367,7 @@ k64_slogdet_inv(const double* __restrict__ MO, Run64 q, double* __restrict__ log
     extern __shared__ double aug[];                  // [n][2n + 1], then n factors
     double* fac = aug + (int64_t)n * w2;
     __shared__ int s_piv;
-    __shared__ double s_logabs, s_sign;
+    __shared__ double s_pv, s_logabs, s_sign;
     const int tid = threadIdx.x;
     const double* A = MO + (mat * C) * (int64_t)n * n;
     const bool want_inv = Ainv != nullptr;
@@ -391,11 +391,13 @@ k64_slogdet_inv(const double* __restrict__ MO, Run64 q, double* __restrict__ log
                 const int oi = __shfl_xor_sync(0xffffffffu, bi, off);
                 if (ov > best || (ov == best && oi < bi)) { best = ov; bi = oi; }
             }
-            if (tid == 0) s_piv = bi;
+            // the pivot itself is handed over too: a warp that read it from the matrix could come after the
+            // first warp has exchanged the rows
+            if (tid == 0) { s_piv = bi; s_pv = aug[bi * w2 + p]; }
         }
         __syncthreads();
         const int piv = s_piv;
-        const double pv = aug[piv * w2 + p];
+        const double pv = s_pv;
         if (pv == 0.0 || !isfinite(pv)) { singular = true; break; }
         if (piv != p) {
             for (int cc = p + tid; cc < cols; cc += blockDim.x) {

@@ -57,3 +57,43 @@ def test_threads_with_different_shapes(cuda, prec, energy):
     for t in threads:
         t.join()
     assert failed == [0] * len(states) and different == [0] * len(states), (failed, different)
+
+
+def test_fp64_inverse_under_contention(cuda):
+    """Inverses and log|det| of the FP64 determinant algebra while other streams' blocks share the SMs, so that the
+    warps of a block run far apart: the same bits on every call."""
+    L = _lib.lib()
+    mol = A.scale_molecule(5)
+    a = A.arch_for(mol, 4)
+    params = api.Params.from_dict(a, P.init_params(a, 0, bias_std=0.1), "fp32_det64")
+    r = torch.as_tensor(A.init_walkers(mol, 1, seed=3).astype("float32"), device="cuda")
+    R, Z = api._geometry(mol.R, mol.Z, torch.device("cuda"))
+    nb = L.dw_workspace_bytes(ctypes.byref(params.c_arch), params.prec, 1, 1)
+    states = [(torch.empty(nb, dtype=torch.uint8, device="cuda"), torch.empty(1, device="cuda"), torch.empty(1, device="cuda"),
+               torch.cuda.Stream()) for _ in range(4)]
+    torch.cuda.synchronize()
+
+    def call(s):
+        return L.dw_local_energy(ctypes.byref(params.c_arch), params.prec, api._ptr(params.flat), api._ptr(params.prepared),
+                                 api._ptr(r), 1, api._ptr(R), api._ptr(Z), api._ptr(s[1]), api._ptr(s[2]), None, api._ptr(s[0]),
+                                 nb, ctypes.c_void_p(s[3].cuda_stream))
+
+    assert call(states[0]) == 0
+    torch.cuda.synchronize()
+    alone = [states[0][1].item(), states[0][2].item()]
+    wrong = []
+
+    def work(s):
+        for _ in range(2000):
+            status = call(s)
+            s[3].synchronize()
+            got = [s[1].item(), s[2].item()]
+            if status or got != alone:
+                wrong.append((status, got))
+
+    threads = [threading.Thread(target=work, args=(s,)) for s in states]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not wrong, (len(wrong), wrong[:4], alone)
