@@ -129,7 +129,7 @@ static int prepare(const DwArch* a, int precision, const float* P, void* prep, s
         tr(P + L.jas_w[0], d.D, d.D, d.J0, d.J0, p.jas0[part]);
         tr(P + L.jas_w[1], d.J0, d.J0, d.J1, d.J1, p.jas1[part]);
     }
-    DW_CHECK_CUDA(cudaGetLastError());
+    DW_CHECK_CUDA(launch_error());
     return DW_OK;
 }
 
@@ -378,7 +378,7 @@ static int run_chunk(const Plan<Act>& p, int Bc, int precision, const float* P, 
     timer_end("jastrow", s, 0.0, 0.0);
     DW_TIMED("combine", launch_combine(p.logdet, p.sign, p.g, p.lapdet, p.jas, r, R, Z, d, Bc, lp, phase, E_loc, grad, s,
                                        0, nullptr, esc));
-    DW_CHECK_CUDA(cudaGetLastError());
+    DW_CHECK_CUDA(launch_error());
     return DW_OK;
 }
 
@@ -618,7 +618,7 @@ int dw_potential_energy(const float* r, int B, int n, const float* R, const int3
     reset_launch_count();
     if (!r || !R || !Z || !E || B <= 0 || n <= 0 || N <= 0) return DW_ERR_ARG;
     launch_coulomb(r, B, n, R, Z, N, E, (cudaStream_t)stream);
-    DW_CHECK_CUDA(cudaGetLastError());
+    DW_CHECK_CUDA(launch_error());
     return DW_OK;
 }
 
@@ -683,7 +683,7 @@ static int mcmc_impl(const DwArch* a, int precision, const float* params, const 
         }
         reset_launch_count();
         count_launch((int)launches);
-        DW_CHECK_CUDA(cudaGetLastError());
+        DW_CHECK_CUDA(launch_error());
         return (int)DW_OK;
     });
 }
@@ -765,7 +765,7 @@ int dw_energy_stats(const float* E, int n, double* out, void* stream) {
     reset_launch_count();
     if (!E || !out || n <= 0) return DW_ERR_ARG;
     launch_stats(E, n, 0, 0.0, 1.0, 1.0, nullptr, out, (cudaStream_t)stream);
-    DW_CHECK_CUDA(cudaGetLastError());
+    DW_CHECK_CUDA(launch_error());
     return DW_OK;
 }
 
@@ -793,7 +793,7 @@ int dw_clip_energies(const float* E, int n, double center, double width, double 
     reset_launch_count();
     if (!E || !out || !E_clip || n <= 0 || !(width > 0)) return DW_ERR_ARG;
     launch_stats(E, n, 1, center, width, clip_by, E_clip, out, (cudaStream_t)stream);
-    DW_CHECK_CUDA(cudaGetLastError());
+    DW_CHECK_CUDA(launch_error());
     return DW_OK;
 }
 

@@ -588,7 +588,7 @@ static int backward_chunk(const Bwd& w, int Bc, const float* P, const ParamLayou
     // ion maps / embedding
     k_ion_bwd<<<1, 256, 0, s>>>(P, L, d, Z, w.him, w.dHIM, grad);
     count_launch(40);
-    DW_CHECK_CUDA(cudaGetLastError());
+    DW_CHECK_CUDA(launch_error());
     return DW_OK;
 }
 

@@ -21,6 +21,10 @@ namespace dw {
 
 void set_last_cuda_error(cudaError_t e);
 void count_launch(int n = 1);
+// The first error of the launches since the last call (kept, or the runtime's last error); clears it.
+cudaError_t launch_error();
+// Keeps the pending launch error, for calls that would clear it (a successful cudaFuncSetAttribute does).
+void keep_launch_error();
 int64_t launch_count();
 void reset_launch_count();
 
@@ -98,6 +102,7 @@ struct Carver {
 // to a launch, and all threads of the process share it: `bytes` is the most that any launch of the kernel
 // takes, never one launch's own size, which would make another thread's larger launch fail.
 template <class K> inline cudaError_t allow_smem(K kernel, int bytes) {
+    keep_launch_error();
     return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
 }
 

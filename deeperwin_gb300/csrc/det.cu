@@ -815,7 +815,7 @@ template <class S, int NMAX, int SPLIT, bool INV>
 static void launch_slogdet_split(const float* MO, int n, int T, int nmat, double* logdet, double* sign, float* Ainv,
                                  cudaStream_t s) {
     const size_t smem = (size_t)NMAX * NMAX * 33 * sizeof(S) + (size_t)NMAX * 32;
-    cudaFuncSetAttribute(k_slogdet_split<S, NMAX, SPLIT, INV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    allow_smem(k_slogdet_split<S, NMAX, SPLIT, INV>, (int)smem);
     k_slogdet_split<S, NMAX, SPLIT, INV><<<(unsigned)((nmat + 31) / 32), 32 * SPLIT, smem, s>>>(MO, n, T, nmat, logdet,
                                                                                              sign, Ainv);
 }
@@ -824,7 +824,7 @@ template <class S, int NMAX, int TPB>
 static void launch_slogdet_inv_thread(const float* MO, int n, int T, int nmat, double* logdet, double* sign, float* Ainv,
                                       cudaStream_t s) {
     const size_t smem = (size_t)NMAX * NMAX * (TPB + 1) * sizeof(S) + (size_t)NMAX * TPB;
-    cudaFuncSetAttribute(k_slogdet_inv_thread<S, NMAX, TPB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    allow_smem(k_slogdet_inv_thread<S, NMAX, TPB>, (int)smem);
     k_slogdet_inv_thread<S, NMAX, TPB><<<(unsigned)((nmat + TPB - 1) / TPB), TPB, smem, s>>>(MO, n, T, nmat, logdet,
                                                                                           sign, Ainv);
 }
@@ -832,7 +832,7 @@ static void launch_slogdet_inv_thread(const float* MO, int n, int T, int nmat, d
 template <class S, int NMAX, int TPB>
 static void launch_slogdet_thread(const float* MO, int n, int T, int nmat, double* logdet, double* sign, cudaStream_t s) {
     const size_t smem = (size_t)NMAX * NMAX * (TPB + 1) * sizeof(S);
-    cudaFuncSetAttribute(k_slogdet_thread<S, NMAX, TPB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    allow_smem(k_slogdet_thread<S, NMAX, TPB>, (int)smem);
     k_slogdet_thread<S, NMAX, TPB><<<(unsigned)((nmat + TPB - 1) / TPB), TPB, smem, s>>>(MO, n, T, nmat, logdet, sign);
 }
 
@@ -946,7 +946,7 @@ void launch_slogdet_impl(const float* MO, const Dims& d, int B, double* logdet, 
     int wpb = (int)(96 * 1024 / per);
     wpb = wpb < 1 ? 1 : (wpb > 8 ? 8 : wpb);
     size_t sm = per * wpb;
-    if (sm > 48 * 1024) cudaFuncSetAttribute(k_slogdet<S>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    if (sm > 48 * 1024) allow_smem(k_slogdet<S>, (int)sm);
     k_slogdet<S><<<(nmat + wpb - 1) / wpb, wpb * 32, sm, s>>>(MO, n, d.T, nmat, want_inv, logdet, sign, Ainv);
     count_launch();
 }
@@ -1488,13 +1488,13 @@ void launch_det_tangents(const float* MO, const float* Ainv, const double* sign,
         const int n = d.n, G = 32 / n, wpb = 4;
         const int ais = (n * n + 1) & ~1, cgs = ((n * (n + 1) > 4 * n ? n * (n + 1) : 4 * n) + 1) & ~1;
         size_t sm = (size_t)wpb * (ais + G * cgs) * sizeof(float);
-        if (sm > 48 * 1024) cudaFuncSetAttribute(k_det_tangents_warp, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+        if (sm > 48 * 1024) allow_smem(k_det_tangents_warp, (int)sm);
         k_det_tangents_warp<<<(nmat + wpb - 1) / wpb, wpb * 32, sm, s>>>(MO, Ainv, sign, n, d.T, nmat, g, lapdet);
         count_launch();
         return;
     }
     size_t sm = 3 * (size_t)d.n * d.n * sizeof(float);
-    if (sm > 48 * 1024) cudaFuncSetAttribute(k_det_tangents, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    if (sm > 48 * 1024) allow_smem(k_det_tangents, (int)sm);
     k_det_tangents<<<nmat, 128, sm, s>>>(MO, Ainv, sign, d.n, d.T, nmat, g, lapdet);
     count_launch();
 }
@@ -1674,7 +1674,8 @@ int dw_debug_slogdet_small(const float* MO, int n, int T, int nmat, int scalar, 
     cudaStream_t s = (cudaStream_t)stream;
     if (scalar == 0) dw::launch_slogdet_small<double>(MO, n, T, nmat, logdet, sign, Ainv, want_inv != 0, s);
     else dw::launch_slogdet_small<dw::FF>(MO, n, T, nmat, logdet, sign, Ainv, want_inv != 0, s);
-    return cudaGetLastError() == cudaSuccess ? DW_OK : DW_ERR_CUDA;
+    DW_CHECK_CUDA(dw::launch_error());
+    return DW_OK;
 }
 
 // Instrumentation: determinant-tangent kernels (0: the default choice; 1: the single-buffer tile

@@ -139,7 +139,7 @@ int dw_forces(const DwArch* a, int precision, const float* params, const void* p
     k_force_mean<<<3 * N, 256, 0, s>>>(pw, B, R, Z, N, forces);
     reset_launch_count();
     count_launch((int)launches + 2);
-    DW_CHECK_CUDA(cudaGetLastError());
+    DW_CHECK_CUDA(launch_error());
     return DW_OK;
 }
 

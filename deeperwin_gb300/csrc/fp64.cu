@@ -702,7 +702,7 @@ static int run_chunk64(const Plan64& p, const Dims& d0, int Bc, const float* P, 
     Dims dc = d;
     dc.Tp = C;
     launch_combine(p.logdet, p.sign, p.g, p.lapdet, p.jas, r, R, Z, dc, Bc, lp, phase, E, grad, s, 1, nvalid);
-    DW_CHECK_CUDA(cudaGetLastError());
+    DW_CHECK_CUDA(launch_error());
     return DW_OK;
 }
 
@@ -729,7 +729,7 @@ int fp64_dets_from_f32(const float* MO, const Dims& d, int Bc, double* MO64, dou
     k64_slogdet_inv<<<nmat, 128, sm_lu, s>>>(MO64, q, logdet, sign, tang ? Ainv64 : nullptr);
     count_launch();
     if (tang) DW_CHECK(launch_tangents64(MO64, Ainv64, sign, q, nmat, g, lapdet, scratch, scratch_bytes, s));
-    DW_CHECK_CUDA(cudaGetLastError());
+    DW_CHECK_CUDA(launch_error());
     return DW_OK;
 }
 

@@ -546,7 +546,7 @@ int gemm64_tc(const double* A, int lda, const Digits& da, const Weight64& w, dou
     k64_gemm_tc<false><<<(unsigned)std::min<int64_t>(tiles, num_sms()), kThreads64, kSmem64, s>>>(ma, mb, a);
     timer_end("fp64_gemm", s, 0.0, 0.0);
     count_launch();
-    DW_CHECK_CUDA(cudaGetLastError());
+    DW_CHECK_CUDA(launch_error());
     return DW_OK;
 }
 
@@ -625,7 +625,7 @@ bool dets64_tangents(const double* MO64, const double* Ainv64, const double* sig
         count_launch();
         k64_lapdet<<<(nm + 7) / 8, 256, 0, s>>>(d.tr1, d.tr2, T - 1, rows, lapdet + m0);
         count_launch();
-        DW_CHECK_CUDA(cudaGetLastError());
+        DW_CHECK_CUDA(launch_error());
         return DW_OK;
     };
     for (int m0 = 0; m0 < nmat && *status == DW_OK; m0 += m) *status = run(m0, std::min(m, nmat - m0));

@@ -663,3 +663,17 @@ void wgrad_f32(const float* A, int lda, const float* G, int ldg, int rows, int K
 }
 
 }  // namespace dw
+
+extern "C" {
+
+// Test hook: a launch that the runtime refuses (more shared memory than an SM has), then one more call as the entry
+// points make them; returns what an entry point would.
+int dw_debug_refused_launch(void* stream) {
+    using namespace dw;
+    k_gemm_f32_tiny<<<1, 256, 512 * 1024, (cudaStream_t)stream>>>(nullptr, 0, nullptr, 0, nullptr, 0, 0, 0, 0, GemmEpi());
+    allow_smem(k_gemm_f32_tiny, kTinyK * (32 + 8) * (int)sizeof(float));
+    DW_CHECK_CUDA(launch_error());
+    return DW_OK;
+}
+
+}  // extern "C"

@@ -408,7 +408,7 @@ int launch_tc(const __nv_bfloat16* A, int lda, const __nv_bfloat16* W0, const __
     int grid = std::min(a.n_tiles, num_sms());
     kern<<<grid, kThreads, smem, s>>>(ma0, ma1, mb0, mb1, mc0, mc1, a);
     count_launch();
-    DW_CHECK_CUDA(cudaGetLastError());
+    DW_CHECK_CUDA(launch_error());
     return DW_OK;
 }
 

@@ -236,7 +236,7 @@ int tail_guard(const DwArch* a, const float* P, const void* prepared, const floa
                                                                       t.cap, E, lp, grad);
         count_launch();
     }
-    DW_CHECK_CUDA(cudaGetLastError());
+    DW_CHECK_CUDA(launch_error());
     return DW_OK;
 }
 

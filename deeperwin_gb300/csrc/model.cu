@@ -13,6 +13,17 @@ static thread_local cudaError_t g_last_cuda = cudaSuccess;
 static thread_local int64_t g_launches = 0;
 void set_last_cuda_error(cudaError_t e) { g_last_cuda = e; }
 void count_launch(int n) { g_launches += n; }
+static thread_local cudaError_t g_launch_error = cudaSuccess;
+void keep_launch_error() {
+    if (g_launch_error == cudaSuccess) g_launch_error = cudaPeekAtLastError();
+}
+cudaError_t launch_error() {
+    keep_launch_error();
+    const cudaError_t e = g_launch_error;
+    g_launch_error = cudaSuccess;
+    (void)cudaGetLastError();
+    return e;
+}
 int64_t launch_count() { return g_launches; }
 void reset_launch_count() { g_launches = 0; }
 

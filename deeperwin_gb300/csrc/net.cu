@@ -1418,8 +1418,8 @@ void launch_streams(const float* r, const float* R, const int32_t* Z, const floa
     auto blocks = [](int64_t n) { return (unsigned)((n + 127) / 128); };
     if (tang) {
         size_t sm3 = 128 * (3 * 32 + 1) * sizeof(float), sm5 = 128 * (5 * 32 + 1) * sizeof(float);
-        cudaFuncSetAttribute(k_ei_streams<5>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm5);
-        cudaFuncSetAttribute(k_pair_streams<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm3);
+        allow_smem(k_ei_streams<5>, (int)sm5);
+        allow_smem(k_pair_streams<3>, (int)sm3);
         if (d.E == 32 && d.EI == 32) {
             constexpr int EP = kRB / 3, EE = kRB / 5;
             const int64_t same_rows = (int64_t)B * (d.nu * (d.nu + 1) / 2 + d.nd * (d.nd + 1) / 2);

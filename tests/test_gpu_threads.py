@@ -97,3 +97,14 @@ def test_fp64_inverse_under_contention(cuda):
     for t in threads:
         t.join()
     assert not wrong, (len(wrong), wrong[:4], alone)
+
+
+def test_refused_launch_is_reported(cuda):
+    """A launch that fails is an error of the call that made it, whatever the call does next, and of no later call."""
+    L = _lib.lib()
+    E = torch.zeros(8, device="cuda")
+    out = torch.empty(3, dtype=torch.float64, device="cuda")
+    for _ in range(2):
+        assert L.dw_debug_refused_launch(None) == 4          # DW_ERR_CUDA
+        assert L.dw_energy_stats(api._ptr(E), 8, api._ptr(out), None) == 0
+    torch.cuda.synchronize()
