@@ -82,6 +82,9 @@ _SIGS = {
     "dw_debug_gemm_fp64": (ctypes.c_int, [_P, ctypes.c_int, _P, ctypes.c_int, _P, ctypes.c_int, ctypes.c_int,
                                           ctypes.c_int, _P, _P]),
     "dw_debug_refused_launch": (ctypes.c_int, [_P]),
+    "dw_debug_det_tangents_fp64_bytes": (ctypes.c_size_t, [ctypes.c_int, ctypes.c_int]),
+    "dw_debug_det_tangents_fp64": (ctypes.c_int, [_P, _P, _P, ctypes.c_int, ctypes.c_int, ctypes.c_int, _P, _P, _P, _P,
+                                                  ctypes.c_size_t, _P]),
     "dw_debug_gemm_jet": (ctypes.c_int, [ctypes.c_int, _P, ctypes.c_int, _P, _P, _P, ctypes.c_int]
                           + [ctypes.c_int] * 7 + [_P, _P, _P]),
     "dw_debug_tc_error_flag": (ctypes.c_int, []),

@@ -785,3 +785,25 @@ int fp64_forward_all(const DwArch* a, const float* P, const void* prepared, cons
 }
 
 }  // namespace dw
+
+extern "C" {
+
+// Test hook: FP64 determinant tangents (launch_tangents64) of nmat matrices with the 3 n + 1 derivative channels of
+// MO [mat][3 n + 2][n][n]; K determinants per walker, nvalid (device, may be null) counts walkers. A scratch below
+// dw_debug_det_tangents_fp64_bytes takes fewer matrices at a time, or the FP64 loop.
+size_t dw_debug_det_tangents_fp64_bytes(int n, int nmat) { return dw::dets64_scratch_bytes(n, 3 * n + 2, nmat); }
+int dw_debug_det_tangents_fp64(const double* MO, const double* Ainv, const double* sign, int n, int K, int nmat,
+                               const int* nvalid, double* g, double* lapdet, void* scratch, size_t scratch_bytes, void* stream) {
+    using namespace dw;
+    reset_launch_count();
+    if (!MO || !Ainv || !sign || !g || !lapdet || n < 1 || n > kMaxEl || K < 1 || nmat < 1 || nmat % K) return DW_ERR_ARG;
+    Run64 q;
+    q.d = Dims();
+    q.d.n = n; q.d.K = K;
+    q.C = 3 * n + 2; q.B = nmat / K; q.nvalid = nvalid;
+    DW_CHECK(launch_tangents64(MO, Ainv, sign, q, nmat, g, lapdet, scratch, scratch_bytes, (cudaStream_t)stream));
+    DW_CHECK_CUDA(cudaGetLastError());
+    return DW_OK;
+}
+
+}  // extern "C"

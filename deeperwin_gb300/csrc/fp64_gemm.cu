@@ -589,9 +589,11 @@ bool dets64_tangents(const double* MO64, const double* Ainv64, const double* sig
     if (!dets64_fits(n) || T < 2 || !scratch) return false;
     char* base = reinterpret_cast<char*>(((uintptr_t)scratch + 255) / 256 * 256);
     const size_t lost = (size_t)(base - static_cast<char*>(scratch)), avail = scratch_bytes > lost ? scratch_bytes - lost : 0;
-    const size_t one = carve_dets(n, T, 1, nullptr).bytes;
-    int m = (int)std::min<size_t>(nmat, avail / std::max<size_t>(one, 1));
-    while (m > 0 && carve_dets(n, T, m, nullptr).bytes > avail) --m;
+    int m = 0;                                       // the most matrices that the scratch holds
+    for (int hi = nmat; m < hi;) {
+        const int mid = m + (hi - m + 1) / 2;
+        if (carve_dets(n, T, mid, nullptr).bytes <= avail) m = mid; else hi = mid - 1;
+    }
     if (m < std::min(nmat, 32)) return false;
     const int per = (T - 1) * n;
     const DetScratch d = carve_dets(n, T, m, base);
