@@ -44,17 +44,35 @@ __device__ __forceinline__ int valid_of(const Rows64& r) { return r.nvalid ? min
 
 // Biased exponent field of x.
 __device__ __forceinline__ int exp_field(double x) { return (__double2hiint(x) >> 20) & 0x7ff; }
-// Exponent of a row from the largest exponent field: values are below 2^E.
-__device__ __forceinline__ int row_exponent(int emax) {
-    if (emax == 0) return 0;                          // zeros (and subnormals, see below)
-    return emax == 0x7ff || emax < 100 ? kFlagged : emax - 1022;
-}
-// x 2^(62 - E) rounded to an integer (E = emax - 1022), |result| <= 2^62.
-__device__ __forceinline__ long long to_fixed(double x, int emax) {
+// What a row's exponent follows from, entries taken times 2^shift: the largest exponent field, the largest
+// shift of a subnormal entry, and whether there is an infinity or NaN.
+constexpr int kNone = -(1 << 20);
+struct RowScan {
+    int emax = kNone, sub = kNone, special = 0;
+    __device__ __forceinline__ void add(double x, int shift) {
+        const long long bits = __double_as_longlong(x);
+        const int e = (int)(bits >> 52) & 0x7ff;
+        if (e == 0x7ff) special = 1;
+        else if (e) emax = max(emax, e + shift);
+        else if (bits << 1) sub = max(sub, 1 + shift);
+    }
+    __device__ __forceinline__ void merge_warp() {
+        emax = __reduce_max_sync(0xffffffffu, emax);
+        sub = __reduce_max_sync(0xffffffffu, sub);
+        special = __reduce_max_sync(0xffffffffu, special);
+    }
+    // Values are below 2^exponent(). Subnormal entries have no digits: they have to be below the last digit.
+    __device__ __forceinline__ int exponent() const {
+        if (special || (sub != kNone && sub > emax - 64)) return kFlagged;
+        return emax == kNone ? 0 : emax - 1022;
+    }
+};
+// x 2^(62 - E) rounded to an integer (E = emax - 1022), |result| <= 2^62, of an entry taken times 2^shift.
+__device__ __forceinline__ long long to_fixed(double x, int emax, int shift) {
     const long long bits = __double_as_longlong(x);
     const int e = (int)(bits >> 52) & 0x7ff;
     unsigned long long m = (bits & 0xfffffffffffffll) | (1ll << 52);
-    const int sh = emax - e - 9;                      // right shift of the 53-bit significand
+    const int sh = emax - e - shift - 9;              // right shift of the 53-bit significand
     if (e == 0 || sh > 54) return 0;
     m = sh <= 0 ? m << -sh : (m + (1ull << (sh - 1))) >> sh;
     return bits < 0 ? -(long long)m : (long long)m;
@@ -70,14 +88,14 @@ __device__ __forceinline__ uint32_t pack_digits(int a, int b) {
     return *reinterpret_cast<const uint32_t*>(&h);
 }
 
-// One row held by a warp (columns 64 u + 2 lane, + 1): common exponent and digit planes.
+// One row held by a warp (columns 64 u + 2 lane, + 1; entries taken times 2^shift): common exponent and
+// digit planes.
 template <int NU>
-__device__ __forceinline__ void slice_row(const double2 (&x)[NU], int emax, bool nonzero, int64_t m,
+__device__ __forceinline__ void slice_row(const double2 (&x)[NU], const int2 (&shift)[NU], RowScan scan, int64_t m,
                                           const Digits& d) {
     const int lane = threadIdx.x & 31, Kp = d.Kp;
-    emax = __reduce_max_sync(0xffffffffu, emax);
-    int E = row_exponent(emax);
-    if (emax == 0 && __any_sync(0xffffffffu, nonzero)) E = kFlagged;    // only subnormals
+    scan.merge_warp();
+    const int E = scan.exponent();
     if (lane == 0) d.ex[m] = E;
     __nv_bfloat16* o = d.dig + m * Kp;
     const int64_t plane = d.rows * Kp;
@@ -86,7 +104,7 @@ __device__ __forceinline__ void slice_row(const double2 (&x)[NU], int emax, bool
         const int c = u * 64 + 2 * lane;
         if (c >= Kp) continue;
         long long f0 = 0, f1 = 0;
-        if (E != kFlagged) { f0 = to_fixed(x[u].x, emax); f1 = to_fixed(x[u].y, emax); }
+        if (E != kFlagged) { f0 = to_fixed(x[u].x, scan.emax, shift[u].x); f1 = to_fixed(x[u].y, scan.emax, shift[u].y); }
         #pragma unroll
         for (int i = kDig - 1; i >= 0; --i) {
             const int d0 = i ? low_digit(f0) : (int)f0, d1 = i ? low_digit(f1) : (int)f1;
@@ -97,10 +115,12 @@ __device__ __forceinline__ void slice_row(const double2 (&x)[NU], int emax, bool
 
 // Warp per row: the largest exponent, then the digits of two neighbouring columns per lane and step.
 // HBM-bound: 8 K bytes read, 18 Kp written per row.
-// es: distance of a row's elements; NU: groups of 64 columns.
+// es: distance of a row's elements; NU: groups of 64 columns. bal (may be null): exponents [walker][K] by which
+// the columns are scaled, times 2^(sign bal).
 template <int NU>
 __global__ void __launch_bounds__(256)
-k64_slice_rows(const double* __restrict__ A, int lda, int es, int K, Rows64 rows, Digits d) {
+k64_slice_rows(const double* __restrict__ A, int lda, int es, int K, Rows64 rows, const int* __restrict__ bal, int sign,
+               Digits d) {
     const int nv = valid_of(rows), lane = threadIdx.x & 31;
     const int64_t w = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int gi = rows.ngroups > 1 && w >= (int64_t)rows.B * rows.g[0].rpw ? 1 : 0;
@@ -111,18 +131,35 @@ k64_slice_rows(const double* __restrict__ A, int lda, int es, int K, Rows64 rows
     const int64_t m = g.base + k;
     const double* src = A + (b * g.out_rpw + g.out_off + k % g.rpw) * lda;
     double2 x[NU];
-    int emax = 0;
-    bool sub = false;
+    int2 shift[NU];
+    RowScan scan;
     #pragma unroll
     for (int u = 0; u < NU; ++u) {
         const int c = u * 64 + 2 * lane;
         x[u] = make_double2(0.0, 0.0);
+        shift[u] = make_int2(0, 0);
         if (c < K) x[u].x = src[(int64_t)c * es];
         if (c + 1 < K) x[u].y = src[(int64_t)(c + 1) * es];
-        emax = max(emax, max(exp_field(x[u].x), exp_field(x[u].y)));
-        sub |= x[u].x != 0.0 || x[u].y != 0.0;
+        if (bal) {
+            if (c < K) shift[u].x = sign * bal[b * K + c];
+            if (c + 1 < K) shift[u].y = sign * bal[b * K + c + 1];
+        }
+        scan.add(x[u].x, shift[u].x);
+        scan.add(x[u].y, shift[u].y);
     }
-    slice_row(x, emax, sub, m, d);
+    slice_row(x, shift, scan, m, d);
+}
+
+// Exponents bal[matrix][o] of the rows of W (largest entry in [2^bal, 2^(bal + 1)); 0 for rows without an
+// ordinary one), warp per row.
+__global__ void __launch_bounds__(256)
+k64_balance(const double* __restrict__ W, int n, Rows64 rows, int* __restrict__ bal) {
+    const int row = (int)(((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
+    if (row / n >= valid_of(rows)) return;
+    int e = 0;
+    for (int c = lane; c < n; c += 32) e = max(e, exp_field(W[(int64_t)row * n + c]));
+    e = __reduce_max_sync(0xffffffffu, e);
+    if (lane == 0) bal[row] = e == 0 || e == 0x7ff ? 0 : e - 1023;
 }
 
 // Spin means of the hw columns of X per (walker, channel), M[(b, t)] = [mean over up electrons, mean
@@ -136,8 +173,8 @@ k64_spin_means(const double* __restrict__ X, int ldx, int hw, int n, int nu, int
     if (b >= valid_of(rows)) return;
     const int t = (int)(bt % C), lane = threadIdx.x & 31;
     double2 x[kMaxK64 / 64];
-    int emax = 0;
-    bool sub = false;
+    int2 shift[kMaxK64 / 64];
+    RowScan scan;
     #pragma unroll
     for (int u = 0; u < kMaxK64 / 64; ++u) {
         double v[2] = {0.0, 0.0};
@@ -150,12 +187,12 @@ k64_spin_means(const double* __restrict__ X, int ldx, int hw, int n, int nu, int
             for (int i = i0; i < i1; ++i) acc += X[((b * n + i) * C + t) * (int64_t)ldx + col];
             v[k] = acc / (i1 - i0);
             M[bt * 2 * hw + c] = v[k];
-            emax = max(emax, exp_field(v[k]));
-            sub |= v[k] != 0.0;
+            scan.add(v[k], 0);
         }
         x[u] = make_double2(v[0], v[1]);
+        shift[u] = make_int2(0, 0);
     }
-    slice_row(x, emax, sub, bt, d);
+    slice_row(x, shift, scan, bt, d);
 }
 
 struct WeightTable {
@@ -174,21 +211,18 @@ __global__ void __launch_bounds__(256) k64_slice_weights(WeightTable t) {
     const Weight64& w = t.w[mi];
     const int n0 = ((int)blockIdx.x - t.first[mi]) * 32, tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
     __shared__ float tile[64][33];
-    __shared__ int emax_s[8][32], sub_s[8][32];
-    int emax = 0, sub = 0;
+    __shared__ int emax_s[8][32], bad_s[8][32];
+    RowScan scan;                                     // (an FP32 value is never subnormal in FP64)
     if (n0 + tx < w.N)
-        for (int k = ty; k < w.K; k += 8) {
-            const float x = w.w[(int64_t)k * w.ldw + n0 + tx];
-            emax = max(emax, exp_field((double)x));
-            sub |= x != 0.f;
-        }
-    emax_s[ty][tx] = emax;
-    sub_s[ty][tx] = sub;
+        for (int k = ty; k < w.K; k += 8) scan.add((double)w.w[(int64_t)k * w.ldw + n0 + tx], 0);
+    emax_s[ty][tx] = scan.emax;
+    bad_s[ty][tx] = scan.special;
     __syncthreads();
     if (ty == 0) {
-        for (int k = 1; k < 8; ++k) { emax = max(emax, emax_s[k][tx]); sub |= sub_s[k][tx]; }
-        emax_s[0][tx] = emax;
-        if (n0 + tx < w.N) w.d.ex[n0 + tx] = emax == 0 && sub ? kFlagged : row_exponent(emax);
+        for (int k = 1; k < 8; ++k) { scan.emax = max(scan.emax, emax_s[k][tx]); scan.special |= bad_s[k][tx]; }
+        emax_s[0][tx] = scan.emax;
+        bad_s[0][tx] = scan.special;
+        if (n0 + tx < w.N) w.d.ex[n0 + tx] = scan.exponent();
     }
     const int64_t plane = w.d.rows * w.d.Kp;
     for (int k0 = 0; k0 < w.d.Kp; k0 += 64) {
@@ -200,8 +234,8 @@ __global__ void __launch_bounds__(256) k64_slice_weights(WeightTable t) {
         for (int n = ty; n < 32; n += 8) {
             if (n0 + n >= w.N || k >= w.d.Kp) continue;
             const int em = emax_s[0][n];
-            const bool ok = row_exponent(em) != kFlagged;
-            long long f0 = ok ? to_fixed((double)tile[2 * tx][n], em) : 0, f1 = ok ? to_fixed((double)tile[2 * tx + 1][n], em) : 0;
+            const bool ok = !bad_s[0][n];
+            long long f0 = ok ? to_fixed((double)tile[2 * tx][n], em, 0) : 0, f1 = ok ? to_fixed((double)tile[2 * tx + 1][n], em, 0) : 0;
             __nv_bfloat16* o = w.d.dig + (int64_t)(n0 + n) * w.d.Kp + k;
             #pragma unroll
             for (int i = kDig - 1; i >= 0; --i) {
@@ -493,9 +527,10 @@ __global__ void k64_lapdet(const double* __restrict__ tr1, const double* __restr
 
 }  // namespace
 
-static void slice_any(const double* A, int lda, int es, int K, const Rows64& rows, const Digits& d, int64_t n, cudaStream_t s) {
-    if (d.Kp <= 64) k64_slice_rows<1><<<(unsigned)((n + 7) / 8), 256, 0, s>>>(A, lda, es, K, rows, d);
-    else k64_slice_rows<kMaxK64 / 64><<<(unsigned)((n + 7) / 8), 256, 0, s>>>(A, lda, es, K, rows, d);
+static void slice_any(const double* A, int lda, int es, int K, const Rows64& rows, const Digits& d, int64_t n, cudaStream_t s,
+                      const int* bal = nullptr, int sign = 0) {
+    if (d.Kp <= 64) k64_slice_rows<1><<<(unsigned)((n + 7) / 8), 256, 0, s>>>(A, lda, es, K, rows, bal, sign, d);
+    else k64_slice_rows<kMaxK64 / 64><<<(unsigned)((n + 7) / 8), 256, 0, s>>>(A, lda, es, K, rows, bal, sign, d);
     count_launch();
 }
 
@@ -553,6 +588,7 @@ int gemm64_tc(const double* A, int lda, const Digits& da, const Weight64& w, dou
 // Scratch of dets64_tangents for `m` matrices at a time.
 struct DetScratch {
     Digits a, w;
+    int* bal;
     double *E, *tr1, *tr2;
     size_t bytes;
 };
@@ -563,6 +599,7 @@ static DetScratch carve_dets(int n, int T, int64_t m, void* base) {
     const int Kp = pad_k64(n);
     d.a = Digits{c.take<__nv_bfloat16>((size_t)kDig * m * per * Kp), c.take<int>(m * per), m * per, Kp};
     d.w = Digits{c.take<__nv_bfloat16>((size_t)kDig * m * n * Kp), c.take<int>(m * n), m * n, Kp};
+    d.bal = c.take<int>(m * n);
     d.E = c.take<double>(m * per * n);
     d.tr1 = c.take<double>(m);
     d.tr2 = c.take<double>(m * (T - 1));
@@ -605,8 +642,15 @@ bool dets64_tangents(const double* MO64, const double* Ainv64, const double* sig
         cols.g[0] = cols.g[1] = RowGroup{0, n, (int64_t)n * n, 0};
         const double* A = MO64 + (int64_t)m0 * T * n * n;
         const double* W = Ainv64 + (int64_t)m0 * n * n;
-        slice_any(A, n, 1, n, rows, d.a, (int64_t)nm * per, s);
-        slice_any(W, 1, n, n, cols, d.w, (int64_t)nm * n, s);
+        // The orbital index is balanced by powers of two, which leave the product as it is: an orbital that is
+        // small at every electron has a large row of A^-1, and unscaled digits would lose the one's low bits
+        // against the other orbitals (columns spread over 2^40: 2e-9 of the trace's terms, now 1e-18). The scale
+        // comes from A^-1's rows: then a row of the product is off by n 2^-56 of its largest sum |dA| |A^-1| at
+        // most, which scales by the columns of dA do not give.
+        k64_balance<<<(unsigned)(((int64_t)nm * n + 7) / 8), 256, 0, s>>>(W, n, rows, d.bal);
+        count_launch();
+        slice_any(A, n, 1, n, rows, d.a, (int64_t)nm * per, s, d.bal, 1);
+        slice_any(W, 1, n, n, cols, d.w, (int64_t)nm * n, s, d.bal, -1);
         CUtensorMap ma, mb;
         DW_CHECK(make_map3(&ma, d.a.dig, kDig, (int)d.a.rows, d.a.Kp, d.a.Kp, d.a.rows * d.a.Kp, BK, BM, kDig, false));
         DW_CHECK(make_map3(&mb, d.w.dig, kDig, (int)d.w.rows, d.w.Kp, d.w.Kp, d.w.rows * d.w.Kp, BK, BN, kDig, false));

@@ -77,7 +77,7 @@ def _reference(MO, inv):
 
 
 @pytest.mark.parametrize("n", [23, 24, 27, 40, 47, 48, 49])
-@pytest.mark.parametrize("kind", ["even"])
+@pytest.mark.parametrize("kind", ["even", "columns", "both", "envelopes", "range"])
 def test_tangents_match_extended_precision(cuda, n, kind):
     MO, inv = _matrices(n, 2, kind, n)
     for scratch in (None, 0):                # digit products where they serve, and the FP64 loop
@@ -113,6 +113,8 @@ def test_singular_and_non_finite_matrices(cuda):
     inv[1] = 0.0                                       # a singular matrix: its tangents are zeros
     MO[2, 5, 3, 4] = np.nan
     MO[3, 7, 2, 2] = np.inf
+    MO[4, :, :, 6] *= 2.0 ** -1055                     # subnormal orbital
+    inv[4, 6] *= 2.0 ** 1000
     g, lap, _ = _tangents(MO, inv, sign=sign)
     gl, ll, _ = _tangents(MO, inv, sign=sign, scratch=0)
     assert np.all(g[1] == 0.0) and lap[1] == 0.0
