@@ -567,8 +567,8 @@ static Plan64 carve64(const Dims& d, int C, int Bc, void* ws, bool digits = true
         }
         auto take = [&](int64_t r, int K) {
             const int Kp = pad_k64(K);
-            __nv_bfloat16* dig = c.take<__nv_bfloat16>((size_t)kDig * r * Kp);
-            return Digits{dig, c.take<int>(r), r, Kp};
+            __nv_bfloat16* dig = c.take<__nv_bfloat16>((size_t)planes64(false) * r * Kp);
+            return Digits{dig, c.take<int>(r), r, Kp, planes64(false)};
         };
         p.act = take(rows, std::max(kXW64, w0));
         p.mean = take((int64_t)Bc * C, 2 * std::max(d.D, d.hw[0]));

@@ -11,9 +11,16 @@
 // products with i + j = s over K <= 512 columns stays below 2^24 (for s = 8 and K = 512 the bound is
 // 2^24.2, reached only if every digit were extreme; a rounding there is 2^-56 of the last digit), so
 // the FP32 accumulators in TMEM hold every digit sum exactly, in any order. The 45 products with
-// i + j <= 8 give the result to about 2^-61 sqrt(K) max|a| max|w|, below the rounding error of an
-// FP64 sum; the nine sums are combined in integers and rounded to FP64 once. FP32 weights are
-// represented exactly down to 2^-38 of their column's maximum.
+// i + j <= 8 give the result to about 2^-61 sqrt(K) max|a| max|w| (at most K 2^-59.5); the nine sums
+// are combined in integers and rounded to FP64 once. FP32 weights are represented exactly down to
+// 2^-38 of their column's maximum.
+//
+// The error of an FP64 sum is relative to S = sum |a| |w| instead, which is far below max|a| max|w| where
+// large entries of a row meet small entries of a column. A tenth plane of each operand therefore holds the
+// magnitudes |a| 2^-Ea in BF16, whose product is S to 1 %: outputs with S below 2^-6 of both scales
+// (kTrust) are formed by an FP64 sum over the original values, so every output is within K 2^-53 S. Rows and
+// columns of zeros give zero. (Determinants, BATCH, balance their inner index instead, see dets64_tangents.)
+// Layers' rows have S near sqrt(K) of the scales, so the sum is rare; the plane costs 1 MMA in 46.
 //
 // Why: FP64 issues at about two lanes per clock and SM here (1.2 TFLOP/s), the BF16 tensor cores at
 // about 1500 times that, so even 45 products per multiplication are far cheaper: the 16 GEMMs of a
@@ -35,10 +42,12 @@ constexpr int BM = 128, BN = 48, BK = 32;            // rows, columns, K-columns
 constexpr int kStages = 2;
 constexpr int kEpi = 8;                              // epilogue warps: two per TMEM lane quarter
 constexpr int kThreads64 = 64 + 32 * kEpi;
-constexpr int kABytes = BM * BK * 2, kBBytes = BN * BK * 2;      // one digit plane of a stage
-constexpr int kStageBytes = kDig * (kABytes + kBBytes);          // 101,376
-constexpr int kSmem64 = 1024 + kStages * kStageBytes + 256;
+constexpr int kABytes = BM * BK * 2, kBBytes = BN * BK * 2;      // one plane of a stage
+constexpr int stage_bytes64(int planes) { return planes * (kABytes + kBBytes); }
+constexpr int smem64(int planes) { return 1024 + kStages * stage_bytes64(planes) + 256; }
 constexpr int kFlagged = 0x7fffffff;                 // exponent of a row that the digits do not represent
+constexpr int kZeroRow = -0x7fffffff;                // of a row of zeros
+constexpr float kTrust = 1.0f / 64;
 
 __device__ __forceinline__ int valid_of(const Rows64& r) { return r.nvalid ? min(r.B, max(0, *r.nvalid * r.mul - r.first)) : r.B; }
 
@@ -64,7 +73,7 @@ struct RowScan {
     // Values are below 2^exponent(). Subnormal entries have no digits: they have to be below the last digit.
     __device__ __forceinline__ int exponent() const {
         if (special || (sub != kNone && sub > emax - 64)) return kFlagged;
-        return emax == kNone ? 0 : emax - 1022;
+        return emax == kNone ? kZeroRow : emax - 1022;
     }
 };
 // x 2^(62 - E) rounded to an integer (E = emax - 1022), |result| <= 2^62, of an entry taken times 2^shift.
@@ -88,6 +97,12 @@ __device__ __forceinline__ uint32_t pack_digits(int a, int b) {
     return *reinterpret_cast<const uint32_t*>(&h);
 }
 
+// Magnitudes of two fixed-point values (62 fractional bits).
+__device__ __forceinline__ uint32_t pack_magnitudes(long long a, long long b) {
+    const __nv_bfloat162 h = __floats2bfloat162_rn((float)(a < 0 ? -a : a) * 0x1p-62f, (float)(b < 0 ? -b : b) * 0x1p-62f);
+    return *reinterpret_cast<const uint32_t*>(&h);
+}
+
 // One row held by a warp (columns 64 u + 2 lane, + 1; entries taken times 2^shift): common exponent and
 // digit planes.
 template <int NU>
@@ -105,6 +120,7 @@ __device__ __forceinline__ void slice_row(const double2 (&x)[NU], const int2 (&s
         if (c >= Kp) continue;
         long long f0 = 0, f1 = 0;
         if (E != kFlagged) { f0 = to_fixed(x[u].x, scan.emax, shift[u].x); f1 = to_fixed(x[u].y, scan.emax, shift[u].y); }
+        if (d.planes > kDig) *reinterpret_cast<uint32_t*>(o + kDig * plane + c) = pack_magnitudes(f0, f1);
         #pragma unroll
         for (int i = kDig - 1; i >= 0; --i) {
             const int d0 = i ? low_digit(f0) : (int)f0, d1 = i ? low_digit(f1) : (int)f1;
@@ -237,6 +253,7 @@ __global__ void __launch_bounds__(256) k64_slice_weights(WeightTable t) {
             const bool ok = !bad_s[0][n];
             long long f0 = ok ? to_fixed((double)tile[2 * tx][n], em, 0) : 0, f1 = ok ? to_fixed((double)tile[2 * tx + 1][n], em, 0) : 0;
             __nv_bfloat16* o = w.d.dig + (int64_t)(n0 + n) * w.d.Kp + k;
+            *reinterpret_cast<uint32_t*>(o + kDig * plane) = pack_magnitudes(f0, f1);
             #pragma unroll
             for (int i = kDig - 1; i >= 0; --i) {
                 const int d0 = i ? low_digit(f0) : (int)f0, d1 = i ? low_digit(f1) : (int)f1;
@@ -295,15 +312,17 @@ __device__ __forceinline__ double combine_digits(const float* acc, int stride, i
     return __longlong_as_double((long long)(q | (neg ? 1ull << 63 : 0ull)));
 }
 
-// Persistent: one CTA per SM loops over 128 x 48 output tiles. Warp 0 loads the nine digit planes of
-// 32 K-columns of both operands per stage (two TMA copies, 101 KB, two stages), warp 1 issues the 90
-// MMAs of a stage into nine TMEM accumulators (432 columns), eight warps combine and store them. Bound
-// by the MMAs' shared-memory reads of A (N = 48: 32 clocks of reads for 24 of products); nine
+// Persistent: one CTA per SM loops over 128 x 48 output tiles. Warp 0 loads the planes of 32 K-columns of
+// both operands per stage (two TMA copies, 113 KB, two stages), warp 1 issues the 92 MMAs of a stage
+// into ten TMEM accumulators (480 columns), eight warps combine and store them. Bound
+// by the MMAs' shared-memory reads of A (N = 48: 32 clocks of reads for 24 of products); the
 // accumulators leave no room for a second set, so the epilogue (about a fifth) is not overlapped.
-// BATCH: each matrix has its own weights (rows [matrix N, + N) of their digit planes) and whole tiles.
+// BATCH: each matrix has its own weights (rows [matrix N, + N) of their digit planes) and whole tiles; no
+// plane of magnitudes.
 template <bool BATCH>
 __global__ void __launch_bounds__(kThreads64, 1)
 k64_gemm_tc(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, Args64 a) {
+    constexpr int kPl = planes64(BATCH), kStageBytes = stage_bytes64(kPl);
     const int nv = valid_of(a.rows);
     int64_t tiles_of[2] = {0, 0};
     const int tpm = BATCH ? (a.per + BM - 1) / BM : 1;          // tiles per matrix
@@ -371,7 +390,7 @@ k64_gemm_tc(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
                     mbar_expect_tx(&full[s], kStageBytes);
                     uint8_t* st = smem + s * kStageBytes;
                     tma_load_3d(st, &tmA, &full[s], kt * BK, row, 0);
-                    tma_load_3d(st + kDig * kABytes, &tmB, &full[s], kt * BK, wrow, 0);
+                    tma_load_3d(st + kPl * kABytes, &tmB, &full[s], kt * BK, wrow, 0);
                     issued[s] = use + 1;
                 }
             }
@@ -394,9 +413,12 @@ k64_gemm_tc(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
                     if (!mbar_wait(&full[s], (cnt / kStages) & 1)) { err = true; break; }
                     tc_fence_after();
                     const uint64_t da = smem_desc_sw64(smem + s * kStageBytes);
-                    const uint64_t db = smem_desc_sw64(smem + s * kStageBytes + kDig * kABytes);
+                    const uint64_t db = smem_desc_sw64(smem + s * kStageBytes + kPl * kABytes);
                     const int nkk = BATCH ? min(BK / 16, (a.K - kt * BK + 15) / 16) : BK / 16;   // 16-column steps with data
                     for (int kk = 0; kk < nkk; ++kk) {
+                        if (!BATCH)
+                            umma_bf16(tmem + kDig * BN, da + (uint64_t)((kDig * kABytes + kk * 32) >> 4),
+                                      db + (uint64_t)((kDig * kBBytes + kk * 32) >> 4), idesc, (kt | kk) ? 1u : 0u);
                         #pragma unroll
                         for (int i = 0; i < kDig; ++i) {
                             #pragma unroll
@@ -435,9 +457,9 @@ k64_gemm_tc(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
             tc_fence_after();
             for (int c0 = h * 8; c0 < BN; c0 += 16) {
                 if (n0 + c0 >= a.N) break;
-                float acc[kDig * 8];
+                float acc[kPl * 8];
                 #pragma unroll
-                for (int s = 0; s < kDig; ++s) tmem_ld8(tmem + s * BN + ((uint32_t)(q * 32) << 16) + c0, acc + s * 8);
+                for (int s = 0; s < kPl; ++s) tmem_ld8(tmem + s * BN + ((uint32_t)(q * 32) << 16) + c0, acc + s * 8);
                 tmem_wait_ld();
                 if (live) {
                     #pragma unroll
@@ -447,8 +469,12 @@ k64_gemm_tc(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
                         for (int u = 0; u < 2; ++u) {
                             const int n = min(n0 + c0 + j + u, a.N - 1);
                             const int ew = a.ew[BATCH ? g * a.N + n : n];
-                            const int scale = ea + ew - 68;
-                            if (ea == kFlagged || ew == kFlagged || scale < -900 || scale > 900) {
+                            const bool flagged = ea == kFlagged || ew == kFlagged, zero = ea == kZeroRow || ew == kZeroRow;
+                            const int scale = flagged || zero ? 0 : ea + ew - 68;
+                            const bool trusted = BATCH || acc[(kPl - 1) * 8 + j + u] >= kTrust;
+                            if (zero && !flagged) {
+                                v[u] = 0.0;
+                            } else if (flagged || !trusted || scale < -900 || scale > 900) {
                                 double x = 0.0;
                                 for (int kk = 0; kk < a.K; ++kk)
                                     x = fma(a.A[row * a.lda + kk], BATCH ? a.W64[((int64_t)g * a.K + kk) * a.N + n]
@@ -563,8 +589,9 @@ int gemm64_tc(const double* A, int lda, const Digits& da, const Weight64& w, dou
               int channels, const Epi64& e, cudaStream_t s) {
     if (w.K > kMaxK64 || da.Kp < w.K || w.d.Kp < w.K) return DW_ERR_ARG;
     CUtensorMap ma, mb;
-    DW_CHECK(make_map3(&ma, da.dig, kDig, (int)da.rows, da.Kp, da.Kp, da.rows * da.Kp, BK, BM, kDig, false));
-    DW_CHECK(make_map3(&mb, w.d.dig, kDig, w.N, w.d.Kp, w.d.Kp, w.d.rows * w.d.Kp, BK, BN, kDig, false));
+    constexpr int kPl = planes64(false);
+    DW_CHECK(make_map3(&ma, da.dig, kPl, (int)da.rows, da.Kp, da.Kp, da.rows * da.Kp, BK, BM, kPl, false));
+    DW_CHECK(make_map3(&mb, w.d.dig, kPl, w.N, w.d.Kp, w.d.Kp, w.d.rows * w.d.Kp, BK, BN, kPl, false));
     Args64 a;
     a.A = A; a.lda = lda; a.W = w.w; a.ldw = w.ldw; a.C = C; a.ldc = ldc;
     a.ea = da.ex; a.ew = w.d.ex;
@@ -576,9 +603,9 @@ int gemm64_tc(const double* A, int lda, const Digits& da, const Weight64& w, dou
     if (!a.error) return DW_ERR_CUDA;
     int64_t tiles = 0;
     for (int g = 0; g < rows.ngroups; ++g) tiles += ((int64_t)rows.B * rows.g[g].rpw + BM - 1) / BM * a.ntn;
-    DW_CHECK_CUDA(allow_smem(k64_gemm_tc<false>, kSmem64));
+    DW_CHECK_CUDA(allow_smem(k64_gemm_tc<false>, smem64(kPl)));
     timer_begin("fp64_gemm", s);
-    k64_gemm_tc<false><<<(unsigned)std::min<int64_t>(tiles, num_sms()), kThreads64, kSmem64, s>>>(ma, mb, a);
+    k64_gemm_tc<false><<<(unsigned)std::min<int64_t>(tiles, num_sms()), kThreads64, smem64(kPl), s>>>(ma, mb, a);
     timer_end("fp64_gemm", s, 0.0, 0.0);
     count_launch();
     DW_CHECK_CUDA(launch_error());
@@ -597,8 +624,12 @@ static DetScratch carve_dets(int n, int T, int64_t m, void* base) {
     DetScratch d;
     const int64_t per = (int64_t)(T - 1) * n;
     const int Kp = pad_k64(n);
-    d.a = Digits{c.take<__nv_bfloat16>((size_t)kDig * m * per * Kp), c.take<int>(m * per), m * per, Kp};
-    d.w = Digits{c.take<__nv_bfloat16>((size_t)kDig * m * n * Kp), c.take<int>(m * n), m * n, Kp};
+    auto take = [&](int64_t rows) {
+        __nv_bfloat16* dig = c.take<__nv_bfloat16>((size_t)planes64(true) * rows * Kp);
+        return Digits{dig, c.take<int>(rows), rows, Kp, planes64(true)};
+    };
+    d.a = take(m * per);
+    d.w = take(m * n);
     d.bal = c.take<int>(m * n);
     d.E = c.take<double>(m * per * n);
     d.tr1 = c.take<double>(m);
@@ -662,9 +693,9 @@ bool dets64_tangents(const double* MO64, const double* Ainv64, const double* sig
         a.W64 = W; a.per = per;
         a.error = tc_error_flag();
         if (!a.error) return DW_ERR_CUDA;
-        DW_CHECK_CUDA(allow_smem(k64_gemm_tc<true>, kSmem64));
+        DW_CHECK_CUDA(allow_smem(k64_gemm_tc<true>, smem64(planes64(true))));
         const int64_t tiles = (int64_t)nm * ((per + BM - 1) / BM);
-        k64_gemm_tc<true><<<(unsigned)std::min<int64_t>(tiles, num_sms()), kThreads64, kSmem64, s>>>(ma, mb, a);
+        k64_gemm_tc<true><<<(unsigned)std::min<int64_t>(tiles, num_sms()), kThreads64, smem64(planes64(true)), s>>>(ma, mb, a);
         count_launch();
         k64_traces<<<(unsigned)((int64_t)nm * (T - 1)), 128, (size_t)n * (n + 1) * sizeof(double), s>>>(
             d.E, sign + m0, n, T - 1, rows, g + (int64_t)m0 * (T - 2), d.tr1, d.tr2);
@@ -685,7 +716,7 @@ extern "C" {
 // Test hook: C [M, N] = A [M, K] (row stride lda) @ W [K, N] (FP32, row stride ldw) by the digit products; ws
 // holds the digit planes (dw_debug_gemm_fp64_bytes).
 size_t dw_debug_gemm_fp64_bytes(int M, int N, int K) {
-    return ((size_t)M + N) * dw::kDig * dw::pad_k64(K) * 2 + ((size_t)M + N) * 4 + 4 * 256;
+    return ((size_t)M + N) * dw::planes64(false) * dw::pad_k64(K) * 2 + ((size_t)M + N) * 4 + 4 * 256;
 }
 int dw_debug_gemm_fp64(const double* A, int lda, const float* W, int ldw, double* C, int M, int N, int K, void* ws,
                        void* stream) {
@@ -694,8 +725,9 @@ int dw_debug_gemm_fp64(const double* A, int lda, const float* W, int ldw, double
     if (!A || !W || !C || !ws || M <= 0 || N <= 0 || K <= 0 || K > kMaxK64) return DW_ERR_ARG;
     cudaStream_t s = (cudaStream_t)stream;
     Carver c(ws, (size_t)-1);
-    Digits da{c.take<__nv_bfloat16>((size_t)kDig * M * pad_k64(K)), c.take<int>(M), M, pad_k64(K)};
-    Weight64 w{W, ldw, K, N, {c.take<__nv_bfloat16>((size_t)kDig * N * pad_k64(K)), c.take<int>(N), N, pad_k64(K)}};
+    constexpr int kPl = planes64(false);
+    Digits da{c.take<__nv_bfloat16>((size_t)kPl * M * pad_k64(K)), c.take<int>(M), M, pad_k64(K), kPl};
+    Weight64 w{W, ldw, K, N, {c.take<__nv_bfloat16>((size_t)kPl * N * pad_k64(K)), c.take<int>(N), N, pad_k64(K), kPl}};
     const Rows64 rows = plain_rows(M, 1, nullptr);
     slice_rows64(A, lda, K, rows, da, s);
     slice_weights64(&w, 1, nullptr, s);

@@ -8,13 +8,16 @@ constexpr int kDig = 9;            // signed 7-bit digits of a row- or column-sc
 constexpr int kMaxK64 = 512;       // widest reduction (the spin-mean rows of a 256-wide layer)
 inline int pad_k64(int K) { return round_up(K, 32); }
 
-// Digit planes of one operand: dig[plane][row][Kp] (BF16 integers in [-64, 64]), row exponents ex[row].
+// Planes of one operand: dig[plane][row][Kp], kDig of digits (BF16 integers in [-64, 64]) and, for the general
+// product, one of magnitudes; row exponents ex[row].
 struct Digits {
     __nv_bfloat16* dig;
     int* ex;
     int64_t rows;                  // rows of a plane
     int Kp;
+    int planes;
 };
+constexpr int planes64(bool batch) { return batch ? kDig : kDig + 1; }
 // Weights [K, N] row-major FP32 (stride ldw) and their digit planes (rows = columns of W).
 struct Weight64 {
     const float* w;
