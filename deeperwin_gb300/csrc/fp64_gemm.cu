@@ -53,10 +53,29 @@ __device__ __forceinline__ int valid_of(const Rows64& r) { return r.nvalid ? min
 
 // Biased exponent field of x.
 __device__ __forceinline__ int exp_field(double x) { return (__double2hiint(x) >> 20) & 0x7ff; }
-// What a row's exponent follows from, entries taken times 2^shift: the largest exponent field, the largest
-// shift of a subnormal entry, and whether there is an infinity or NaN.
-constexpr int kNone = -(1 << 20);
+// What a row's exponent E follows from (values are below 2^E): the largest exponent field, here of unscaled
+// entries. Subnormal entries have no digits, so the largest has to be far above them.
 struct RowScan {
+    int emax = 0;
+    uint32_t any = 0;
+    __device__ __forceinline__ void add(double x) {
+        emax = max(emax, exp_field(x));
+        any |= (uint32_t)__double2loint(x) | ((uint32_t)__double2hiint(x) << 1);
+    }
+    __device__ __forceinline__ int exponent() const {
+        if (emax == 0) return any ? kFlagged : kZeroRow;
+        return emax == 0x7ff || emax < 100 ? kFlagged : emax - 1022;
+    }
+    __device__ __forceinline__ int merge_warp() {
+        emax = __reduce_max_sync(0xffffffffu, emax);
+        any = __any_sync(0xffffffffu, any != 0);
+        return exponent();
+    }
+};
+// The same of entries taken times 2^shift: the field may leave its range, subnormal entries and infinities are
+// kept apart.
+struct ScaledRowScan {
+    static constexpr int kNone = -(1 << 20);
     int emax = kNone, sub = kNone, special = 0;
     __device__ __forceinline__ void add(double x, int shift) {
         const long long bits = __double_as_longlong(x);
@@ -65,23 +84,20 @@ struct RowScan {
         else if (e) emax = max(emax, e + shift);
         else if (bits << 1) sub = max(sub, 1 + shift);
     }
-    __device__ __forceinline__ void merge_warp() {
+    __device__ __forceinline__ int merge_warp() {
         emax = __reduce_max_sync(0xffffffffu, emax);
         sub = __reduce_max_sync(0xffffffffu, sub);
         special = __reduce_max_sync(0xffffffffu, special);
-    }
-    // Values are below 2^exponent(). Subnormal entries have no digits: they have to be below the last digit.
-    __device__ __forceinline__ int exponent() const {
         if (special || (sub != kNone && sub > emax - 64)) return kFlagged;
         return emax == kNone ? kZeroRow : emax - 1022;
     }
 };
-// x 2^(62 - E) rounded to an integer (E = emax - 1022), |result| <= 2^62, of an entry taken times 2^shift.
-__device__ __forceinline__ long long to_fixed(double x, int emax, int shift) {
+// x 2^(62 - E) rounded to an integer (E = emax - 1022), |result| <= 2^62.
+__device__ __forceinline__ long long to_fixed(double x, int emax) {
     const long long bits = __double_as_longlong(x);
     const int e = (int)(bits >> 52) & 0x7ff;
     unsigned long long m = (bits & 0xfffffffffffffll) | (1ll << 52);
-    const int sh = emax - e - shift - 9;              // right shift of the 53-bit significand
+    const int sh = emax - e - 9;             // right shift of the 53-bit significand
     if (e == 0 || sh > 54) return 0;
     m = sh <= 0 ? m << -sh : (m + (1ull << (sh - 1))) >> sh;
     return bits < 0 ? -(long long)m : (long long)m;
@@ -103,14 +119,11 @@ __device__ __forceinline__ uint32_t pack_magnitudes(long long a, long long b) {
     return *reinterpret_cast<const uint32_t*>(&h);
 }
 
-// One row held by a warp (columns 64 u + 2 lane, + 1; entries taken times 2^shift): common exponent and
-// digit planes.
-template <int NU>
-__device__ __forceinline__ void slice_row(const double2 (&x)[NU], const int2 (&shift)[NU], RowScan scan, int64_t m,
-                                          const Digits& d) {
+// One row held by a warp (columns 64 u + 2 lane, + 1) of exponent E: its planes. emax(u, k): largest exponent field
+// of the row less the shift of column 64 u + 2 lane + k.
+template <int NU, class EMax>
+__device__ __forceinline__ void slice_row(const double2 (&x)[NU], int E, EMax emax, int64_t m, const Digits& d) {
     const int lane = threadIdx.x & 31, Kp = d.Kp;
-    scan.merge_warp();
-    const int E = scan.exponent();
     if (lane == 0) d.ex[m] = E;
     __nv_bfloat16* o = d.dig + m * Kp;
     const int64_t plane = d.rows * Kp;
@@ -119,7 +132,7 @@ __device__ __forceinline__ void slice_row(const double2 (&x)[NU], const int2 (&s
         const int c = u * 64 + 2 * lane;
         if (c >= Kp) continue;
         long long f0 = 0, f1 = 0;
-        if (E != kFlagged) { f0 = to_fixed(x[u].x, scan.emax, shift[u].x); f1 = to_fixed(x[u].y, scan.emax, shift[u].y); }
+        if (E != kFlagged) { f0 = to_fixed(x[u].x, emax(u, 0)); f1 = to_fixed(x[u].y, emax(u, 1)); }
         if (d.planes > kDig) *reinterpret_cast<uint32_t*>(o + kDig * plane + c) = pack_magnitudes(f0, f1);
         #pragma unroll
         for (int i = kDig - 1; i >= 0; --i) {
@@ -130,10 +143,10 @@ __device__ __forceinline__ void slice_row(const double2 (&x)[NU], const int2 (&s
 }
 
 // Warp per row: the largest exponent, then the digits of two neighbouring columns per lane and step.
-// HBM-bound: 8 K bytes read, 18 Kp written per row.
-// es: distance of a row's elements; NU: groups of 64 columns. bal (may be null): exponents [walker][K] by which
-// the columns are scaled, times 2^(sign bal).
-template <int NU>
+// HBM-bound: 8 K bytes read, 20 Kp (BATCH: 18 Kp) written per row.
+// es: distance of a row's elements; NU: groups of 64 columns. bal (BATCH): exponents [matrix][K] by which the
+// columns are scaled, times 2^(sign bal).
+template <int NU, bool BATCH>
 __global__ void __launch_bounds__(256)
 k64_slice_rows(const double* __restrict__ A, int lda, int es, int K, Rows64 rows, const int* __restrict__ bal, int sign,
                Digits d) {
@@ -147,23 +160,33 @@ k64_slice_rows(const double* __restrict__ A, int lda, int es, int K, Rows64 rows
     const int64_t m = g.base + k;
     const double* src = A + (b * g.out_rpw + g.out_off + k % g.rpw) * lda;
     double2 x[NU];
-    int2 shift[NU];
-    RowScan scan;
     #pragma unroll
     for (int u = 0; u < NU; ++u) {
         const int c = u * 64 + 2 * lane;
         x[u] = make_double2(0.0, 0.0);
-        shift[u] = make_int2(0, 0);
         if (c < K) x[u].x = src[(int64_t)c * es];
         if (c + 1 < K) x[u].y = src[(int64_t)(c + 1) * es];
-        if (bal) {
-            if (c < K) shift[u].x = sign * bal[b * K + c];
-            if (c + 1 < K) shift[u].y = sign * bal[b * K + c + 1];
-        }
-        scan.add(x[u].x, shift[u].x);
-        scan.add(x[u].y, shift[u].y);
     }
-    slice_row(x, shift, scan, m, d);
+    if constexpr (BATCH) {
+        int shift[NU][2];
+        ScaledRowScan scan;
+        #pragma unroll
+        for (int u = 0; u < NU; ++u)
+            #pragma unroll
+            for (int v = 0; v < 2; ++v) {
+                const int c = u * 64 + 2 * lane + v;
+                shift[u][v] = c < K ? sign * bal[b * K + c] : 0;
+                scan.add(v ? x[u].y : x[u].x, shift[u][v]);
+            }
+        const int E = scan.merge_warp();
+        slice_row(x, E, [&](int u, int v) { return scan.emax - shift[u][v]; }, m, d);
+    } else {
+        RowScan scan;
+        #pragma unroll
+        for (int u = 0; u < NU; ++u) { scan.add(x[u].x); scan.add(x[u].y); }
+        const int E = scan.merge_warp();
+        slice_row(x, E, [&](int, int) { return scan.emax; }, m, d);
+    }
 }
 
 // Exponents bal[matrix][o] of the rows of W (largest entry in [2^bal, 2^(bal + 1)); 0 for rows without an
@@ -189,7 +212,6 @@ k64_spin_means(const double* __restrict__ X, int ldx, int hw, int n, int nu, int
     if (b >= valid_of(rows)) return;
     const int t = (int)(bt % C), lane = threadIdx.x & 31;
     double2 x[kMaxK64 / 64];
-    int2 shift[kMaxK64 / 64];
     RowScan scan;
     #pragma unroll
     for (int u = 0; u < kMaxK64 / 64; ++u) {
@@ -203,12 +225,12 @@ k64_spin_means(const double* __restrict__ X, int ldx, int hw, int n, int nu, int
             for (int i = i0; i < i1; ++i) acc += X[((b * n + i) * C + t) * (int64_t)ldx + col];
             v[k] = acc / (i1 - i0);
             M[bt * 2 * hw + c] = v[k];
-            scan.add(v[k], 0);
+            scan.add(v[k]);
         }
         x[u] = make_double2(v[0], v[1]);
-        shift[u] = make_int2(0, 0);
     }
-    slice_row(x, shift, scan, bt, d);
+    const int E = scan.merge_warp();
+    slice_row(x, E, [&](int, int) { return scan.emax; }, bt, d);
 }
 
 struct WeightTable {
@@ -227,17 +249,16 @@ __global__ void __launch_bounds__(256) k64_slice_weights(WeightTable t) {
     const Weight64& w = t.w[mi];
     const int n0 = ((int)blockIdx.x - t.first[mi]) * 32, tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
     __shared__ float tile[64][33];
-    __shared__ int emax_s[8][32], bad_s[8][32];
+    __shared__ int emax_s[8][32];
     RowScan scan;                                     // (an FP32 value is never subnormal in FP64)
     if (n0 + tx < w.N)
-        for (int k = ty; k < w.K; k += 8) scan.add((double)w.w[(int64_t)k * w.ldw + n0 + tx], 0);
+        for (int k = ty; k < w.K; k += 8) scan.add((double)w.w[(int64_t)k * w.ldw + n0 + tx]);
     emax_s[ty][tx] = scan.emax;
-    bad_s[ty][tx] = scan.special;
     __syncthreads();
     if (ty == 0) {
-        for (int k = 1; k < 8; ++k) { scan.emax = max(scan.emax, emax_s[k][tx]); scan.special |= bad_s[k][tx]; }
+        for (int k = 1; k < 8; ++k) scan.emax = max(scan.emax, emax_s[k][tx]);
         emax_s[0][tx] = scan.emax;
-        bad_s[0][tx] = scan.special;
+        scan.any = 0;                                 // no field: a column of zeros
         if (n0 + tx < w.N) w.d.ex[n0 + tx] = scan.exponent();
     }
     const int64_t plane = w.d.rows * w.d.Kp;
@@ -250,8 +271,8 @@ __global__ void __launch_bounds__(256) k64_slice_weights(WeightTable t) {
         for (int n = ty; n < 32; n += 8) {
             if (n0 + n >= w.N || k >= w.d.Kp) continue;
             const int em = emax_s[0][n];
-            const bool ok = !bad_s[0][n];
-            long long f0 = ok ? to_fixed((double)tile[2 * tx][n], em, 0) : 0, f1 = ok ? to_fixed((double)tile[2 * tx + 1][n], em, 0) : 0;
+            const bool ok = em != 0x7ff;
+            long long f0 = ok ? to_fixed((double)tile[2 * tx][n], em) : 0, f1 = ok ? to_fixed((double)tile[2 * tx + 1][n], em) : 0;
             __nv_bfloat16* o = w.d.dig + (int64_t)(n0 + n) * w.d.Kp + k;
             *reinterpret_cast<uint32_t*>(o + kDig * plane) = pack_magnitudes(f0, f1);
             #pragma unroll
@@ -553,17 +574,13 @@ __global__ void k64_lapdet(const double* __restrict__ tr1, const double* __restr
 
 }  // namespace
 
-static void slice_any(const double* A, int lda, int es, int K, const Rows64& rows, const Digits& d, int64_t n, cudaStream_t s,
-                      const int* bal = nullptr, int sign = 0) {
-    if (d.Kp <= 64) k64_slice_rows<1><<<(unsigned)((n + 7) / 8), 256, 0, s>>>(A, lda, es, K, rows, bal, sign, d);
-    else k64_slice_rows<kMaxK64 / 64><<<(unsigned)((n + 7) / 8), 256, 0, s>>>(A, lda, es, K, rows, bal, sign, d);
-    count_launch();
-}
-
 void slice_rows64(const double* A, int lda, int K, const Rows64& rows, const Digits& d, cudaStream_t s) {
     int64_t n = 0;
     for (int g = 0; g < rows.ngroups; ++g) n += (int64_t)rows.B * rows.g[g].rpw;
-    slice_any(A, lda, 1, K, rows, d, n, s);
+    const unsigned grid = (unsigned)((n + 7) / 8);
+    if (d.Kp <= 64) k64_slice_rows<1, false><<<grid, 256, 0, s>>>(A, lda, 1, K, rows, nullptr, 0, d);
+    else k64_slice_rows<kMaxK64 / 64, false><<<grid, 256, 0, s>>>(A, lda, 1, K, rows, nullptr, 0, d);
+    count_launch();
 }
 
 void spin_means64(const double* X, int ldx, int hw, int n, int nu, int C, const Rows64& rows, double* M, const Digits& d,
@@ -680,8 +697,10 @@ bool dets64_tangents(const double* MO64, const double* Ainv64, const double* sig
         // most, which scales by the columns of dA do not give.
         k64_balance<<<(unsigned)(((int64_t)nm * n + 7) / 8), 256, 0, s>>>(W, n, rows, d.bal);
         count_launch();
-        slice_any(A, n, 1, n, rows, d.a, (int64_t)nm * per, s, d.bal, 1);
-        slice_any(W, 1, n, n, cols, d.w, (int64_t)nm * n, s, d.bal, -1);
+        k64_slice_rows<1, true><<<(unsigned)(((int64_t)nm * per + 7) / 8), 256, 0, s>>>(A, n, 1, n, rows, d.bal, 1, d.a);
+        count_launch();
+        k64_slice_rows<1, true><<<(unsigned)(((int64_t)nm * n + 7) / 8), 256, 0, s>>>(W, 1, n, n, cols, d.bal, -1, d.w);
+        count_launch();
         CUtensorMap ma, mb;
         DW_CHECK(make_map3(&ma, d.a.dig, kDig, (int)d.a.rows, d.a.Kp, d.a.Kp, d.a.rows * d.a.Kp, BK, BM, kDig, false));
         DW_CHECK(make_map3(&mb, d.w.dig, kDig, (int)d.w.rows, d.w.Kp, d.w.Kp, d.w.rows * d.w.Kp, BK, BN, kDig, false));
