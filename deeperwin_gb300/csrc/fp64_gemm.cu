@@ -481,7 +481,7 @@ k64_gemm_tc(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
                 float acc[kPl * 8];
                 #pragma unroll
                 for (int s = 0; s < kPl; ++s) tmem_ld8(tmem + s * BN + ((uint32_t)(q * 32) << 16) + c0, acc + s * 8);
-                tmem_wait_ld();
+                tmem_wait_ld(acc);
                 if (live) {
                     #pragma unroll
                     for (int j = 0; j < 8; j += 2) {

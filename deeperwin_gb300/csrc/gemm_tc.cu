@@ -296,7 +296,7 @@ k_gemm_tc(const __grid_constant__ CUtensorMap tmA0, const __grid_constant__ CUte
                 const uint32_t base = tmem + acc * (uint32_t)BN + ((uint32_t)(q * 32) << 16) + (uint32_t)c0;
                 #pragma unroll
                 for (int j = 0; j < CW; j += 16) tmem_ld16(base + j, v + j);
-                tmem_wait_ld();
+                tmem_wait_ld(v);
                 #pragma unroll
                 for (int j = 0; j < CW; ++j) v[j] += rbv[j];
                 // double-buffered staging: the store issued from this buffer two chunks ago has

@@ -171,6 +171,10 @@ __device__ __forceinline__ void tmem_wait_ld16(float (&v)[16]) {
                    "+f"(v[8]), "+f"(v[9]), "+f"(v[10]), "+f"(v[11]), "+f"(v[12]), "+f"(v[13]), "+f"(v[14]), "+f"(v[15])
                  :: "memory");
 }
-__device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+template <int N> __device__ __forceinline__ void tmem_wait_ld(float (&v)[N]) {
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+    #pragma unroll
+    for (int j = 0; j < N; ++j) asm volatile("" : "+f"(v[j]));
+}
 
 }  // namespace dw
