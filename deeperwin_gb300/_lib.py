@@ -81,6 +81,7 @@ _SIGS = {
     "dw_debug_gemm_fp64_bytes": (ctypes.c_size_t, [ctypes.c_int, ctypes.c_int, ctypes.c_int]),
     "dw_debug_gemm_fp64": (ctypes.c_int, [_P, ctypes.c_int, _P, ctypes.c_int, _P, ctypes.c_int, ctypes.c_int,
                                           ctypes.c_int, _P, _P]),
+    "dw_debug_workspace_least_bytes": (ctypes.c_size_t, [ctypes.POINTER(DwArch), ctypes.c_int, ctypes.c_int, ctypes.c_int]),
     "dw_debug_refused_launch": (ctypes.c_int, [_P]),
     "dw_debug_det_tangents_fp64_bytes": (ctypes.c_size_t, [ctypes.c_int, ctypes.c_int]),
     "dw_debug_det_tangents_fp64": (ctypes.c_int, [_P, _P, _P, ctypes.c_int, ctypes.c_int, ctypes.c_int, _P, _P, _P, _P,

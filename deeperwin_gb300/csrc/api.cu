@@ -147,7 +147,7 @@ struct Plan {
     double* logdet; double* sign; float* Ainv; double* g; double* lapdet;
     Act* J1; Act* J2; double* jas;
     size_t bytes;
-    void* scratch = nullptr; size_t scratch_bytes = 0;     // what the caller's region holds beyond the plan
+    void* scratch = nullptr; size_t scratch_bytes = 0;     // FP64 determinant tangents by digit products (0: none)
 };
 
 static const int kXW = 320;   // row width of the layer-1..3 inputs: 256 (h) + 32 (conv_ee) + 32 (conv_ei)
@@ -407,33 +407,54 @@ static size_t plan_bytes(const DwArch* a, int B, bool tang, size_t budget = kChu
     Dims d = make_dims(a, tang);
     return (carve_plan<Act>(d, choose_chunk<Act>(d, std::max(B, 1), budget), nullptr).bytes + 4096 + 255) / 256 * 256;
 }
+// Bytes that a forward takes at least: those of the plan, or of one whose channel rows are padded to a power of two, as
+// they once were (its chunk at the budget can take less than the chunk of unpadded rows).
+template <class Act>
+static size_t least_plan_bytes(const DwArch* a, int B, bool tang, size_t budget) {
+    Dims d = make_dims(a, tang);
+    const size_t now = carve_plan<Act>(d, choose_chunk<Act>(d, std::max(B, 1), budget), nullptr).bytes;
+    if (!tang) return now;
+    d.Tp = next_pow2(d.T);
+    return std::min(now, carve_plan<Act>(d, choose_chunk<Act>(d, std::max(B, 1), budget), nullptr).bytes);
+}
 
 // Mixed-form local energies: the forward's plan (or the tail re-evaluation, which reuses that
 // region once the forward is done) followed by the per-walker error scales.
-static size_t guarded_bytes(const DwArch* a, int B, size_t plan) {
-    return (std::max(plan, guard_bytes(a, B)) + 255) / 256 * 256 + (size_t)3 * B * sizeof(float) + 256;
+static size_t guarded_region(const DwArch* a, int B, size_t plan, bool least) {
+    return (std::max(plan, guard_bytes(a, B, least)) + 255) / 256 * 256;
 }
 
-// Workspace of one forward (value or tangent) and the forward itself, for every precision form.
+// Region of one forward (value or tangent), for every precision form: what it runs best in, or the least that it
+// takes (the FP64 form without digit planes, FP64 determinant tangents without scratch for them). The least is
+// what such a region held before there were digit products; regions of that size are still taken.
 template <class Act>
-static size_t plan_bytes_any(const DwArch* a, int B, bool tang) {
-    if constexpr (std::is_same<Act, double>::value) return fp64_plan_bytes(a, B, tang);
+static size_t plan_bytes_any(const DwArch* a, int precision, int B, bool tang, bool least = false) {
+    if constexpr (std::is_same<Act, double>::value) return least ? fp64_least_bytes(a, B, tang) : fp64_plan_bytes(a, B, tang);
+    else if (det64_form(precision) && tang) return least ? det64_least_bytes(a, precision, B) : det64_plan_bytes(a, precision, B);
+    else if (least) return (least_plan_bytes<Act>(a, B, tang, kChunkBudget) + 4096 + 255) / 256 * 256;
     else return plan_bytes<Act>(a, B, tang);
 }
+// The region that a workspace of wsb bytes leaves in front of `rest` bytes: `full`, or less down to `least` (0: too small).
+static size_t region_of(size_t full, size_t least, size_t rest, size_t wsb) {
+    if (wsb < rest) return 0;
+    const size_t room = (wsb - rest) / 256 * 256;
+    return room >= full ? full : (room >= least ? room : 0);
+}
 
 template <class Act>
-static size_t ws_bytes_t(const DwArch* a, int n_walkers, int mode) {
+static size_t ws_bytes_t(const DwArch* a, int precision, int n_walkers, int mode, bool least = false) {
     if (mode == 3) return bwd_bytes(a, n_walkers, nullptr);
     if (mode == 2) {
-        size_t b = plan_bytes_any<Act>(a, n_walkers, false);
+        size_t b = plan_bytes_any<Act>(a, precision, n_walkers, false, least);
         b += (size_t)n_walkers * a->n_el * 3 * sizeof(float) + 256;      // proposals
         b += (size_t)n_walkers * sizeof(float) + 256;                    // proposal log psi^2
         b += (size_t)n_walkers * sizeof(float) + 256;                    // log proposal ratios
         b += (size_t)mh_counts_needed(kMaxSeg) * sizeof(int) + 256;
         return b;
     }
-    size_t b = plan_bytes_any<Act>(a, n_walkers, mode == 1);
-    if (mode == 1 && std::is_same<Act, Split>::value) b = guarded_bytes(a, n_walkers, b);
+    size_t b = plan_bytes_any<Act>(a, precision, n_walkers, mode == 1, least);
+    if (mode == 1 && precision == DW_PRECISION_MIXED)
+        b = guarded_region(a, n_walkers, b, least) + (size_t)3 * n_walkers * sizeof(float) + 256;
     if (mode == 1) b += (size_t)n_walkers * sizeof(float) + 256;         // log psi^2 when not requested
     return b;
 }
@@ -450,11 +471,15 @@ static int forward_all(const DwArch* a, int precision, const float* P, const voi
     ParamLayout L;
     make_layout(a, &L);
     Prepared pre = carve_prepared(a, precision, const_cast<void*>(prepared));
+    if (least_plan_bytes<Act>(a, B, tang, budget) > ws_bytes) return DW_ERR_WORKSPACE;
     int bc = choose_chunk<Act>(d, B, budget);
+    while (bc > 1 && carve_plan<Act>(d, bc, nullptr).bytes > ws_bytes) bc -= std::max(1, bc / 32);
     Plan<Act> p = carve_plan<Act>(d, bc, ws);
     if (p.bytes > ws_bytes) return DW_ERR_WORKSPACE;
-    p.scratch = static_cast<char*>(ws) + p.bytes;
-    p.scratch_bytes = ws_bytes - p.bytes;
+    if (det64_form(precision) && tang) {
+        const size_t need = dets64_scratch_bytes(d.n, d.T, (int64_t)bc * d.K);
+        if (ws_bytes - p.bytes >= need) { p.scratch = static_cast<char*>(ws) + p.bytes; p.scratch_bytes = need; }
+    }
     d.nseg = nseg;
     p.d.nseg = nseg;      // the chunks index geometries through the plan's dims
     launch_ion_maps(P, L, d, Z, p.him, s);
@@ -487,18 +512,21 @@ static int local_energy_impl(const DwArch* a, int precision, const float* params
                              float* grad, void* ws, size_t wsb, cudaStream_t s) {
     return with_act(precision, true, [&](auto tag) {
         using Act = act_of<decltype(tag)>;
-        const size_t pb = plan_bytes_any<Act>(a, B, true);
         const bool guarded = std::is_same<Act, Split>::value && precision == DW_PRECISION_MIXED;
-        const size_t region = guarded ? (std::max(pb, guard_bytes(a, B)) + 255) / 256 * 256 : pb;
+        const size_t lp_bytes = ((size_t)B * sizeof(float) + 255) / 256 * 256, esc_bytes = (size_t)3 * B * sizeof(float);
+        auto region_bytes = [&](bool least) {
+            const size_t pb = plan_bytes_any<Act>(a, precision, B, true, least);
+            return guarded ? guarded_region(a, B, pb, least) : pb;
+        };
+        const size_t region = region_of(region_bytes(false), region_bytes(true), (lp ? 0 : lp_bytes) + (guarded ? esc_bytes : 0), wsb);
+        if (region == 0) return (int)DW_ERR_WORKSPACE;
         char* tail = static_cast<char*>(ws) + region;
         float* lpo = lp;
         if (!lpo) {   // log psi^2 output is optional; it then lives after the plan
             lpo = reinterpret_cast<float*>(tail);
-            tail += ((size_t)B * sizeof(float) + 255) / 256 * 256;
+            tail += lp_bytes;
         }
         float* esc = guarded ? reinterpret_cast<float*>(tail) : nullptr;
-        if (guarded) tail += (size_t)3 * B * sizeof(float);
-        if ((size_t)(tail - static_cast<char*>(ws)) > wsb) return (int)DW_ERR_WORKSPACE;
         if constexpr (std::is_same<Act, double>::value) {
             return fp64_forward_all(a, params, prepared, r, B, R, Z, lpo, nullptr, E, grad, true, ws, region, s, seg, nseg,
                                     nullptr);
@@ -517,14 +545,17 @@ static int local_energy_impl(const DwArch* a, int precision, const float* params
 // Local energy with FP64 determinant algebra on a caller region (DW_PRECISION_FP32_DET64: plain
 // FP32 network, DW_PRECISION_MIXED_DET64: split-BF16 network): the mixed form's re-evaluation of
 // flagged walkers (guard.cu).
+size_t det64_least_bytes(const DwArch* a, int precision, int B) {
+    return ((precision == DW_PRECISION_MIXED_DET64 ? least_plan_bytes<Split>(a, B, true, kChunkBudget)
+                                                   : least_plan_bytes<float>(a, B, true, kChunkBudget)) + 4096 + 255) / 256 * 256;
+}
 size_t det64_plan_bytes(const DwArch* a, int precision, int B) {
     const Dims d = make_dims(a, true);
+    const int bc = precision == DW_PRECISION_MIXED_DET64 ? choose_chunk<Split>(d, std::max(B, 1)) : choose_chunk<float>(d, std::max(B, 1));
     // and the scratch of the FP64 determinant tangents of a chunk
-    auto bytes = [&](auto tag) {
-        using Act = act_of<decltype(tag)>;
-        return plan_bytes<Act>(a, B, true) + dets64_scratch_bytes(d.n, d.T, (int64_t)choose_chunk<Act>(d, std::max(B, 1)) * d.K);
-    };
-    return precision == DW_PRECISION_MIXED_DET64 ? bytes((Split*)nullptr) : bytes((float*)nullptr);
+    const size_t scratch = dets64_scratch_bytes(d.n, d.T, (int64_t)bc * d.K);
+    return (precision == DW_PRECISION_MIXED_DET64 ? plan_bytes<Split>(a, B, true) : plan_bytes<float>(a, B, true)) +
+           (scratch + 255) / 256 * 256;
 }
 int det64_local_energy(const DwArch* a, int precision, const float* P, const void* prepared, const float* r, int B,
                        const float* R, const int32_t* Z, const int32_t* seg, int nseg, float* E, float* lp, float* grad,
@@ -534,6 +565,13 @@ int det64_local_energy(const DwArch* a, int precision, const float* P, const voi
                                   nseg);
     return forward_all<float>(a, DW_PRECISION_FP32_DET64, P, prepared, r, B, R, Z, lp, nullptr, E, grad, true, ws, wsb,
                               s, seg, nseg);
+}
+
+size_t workspace_least_bytes(const DwArch* a, int precision, int n_walkers, int mode) {
+    if (check_arch(a) != DW_OK || n_walkers <= 0) return 0;
+    size_t out = 0;
+    with_act(precision, false, [&](auto tag) { out = ws_bytes_t<act_of<decltype(tag)>>(a, precision, n_walkers, mode, true); return 0; });
+    return out;
 }
 
 // FP32 row-gathered layer weights of a prepared buffer (the same offsets in every precision form).
@@ -589,8 +627,13 @@ int dw_prepare_params(const DwArch* a, int precision, const float* params, void*
 size_t dw_workspace_bytes(const DwArch* a, int precision, int n_walkers, int mode) {
     if (check_arch(a) != DW_OK || n_walkers <= 0) return 0;
     size_t out = 0;
-    with_act(precision, false, [&](auto tag) { out = ws_bytes_t<act_of<decltype(tag)>>(a, n_walkers, mode); return 0; });
+    with_act(precision, false, [&](auto tag) { out = ws_bytes_t<act_of<decltype(tag)>>(a, precision, n_walkers, mode); return 0; });
     return out;
+}
+
+// Test hook: the least workspace that the entry points take.
+size_t dw_debug_workspace_least_bytes(const DwArch* a, int precision, int n_walkers, int mode) {
+    return workspace_least_bytes(a, precision, n_walkers, mode);
 }
 
 int dw_log_psi_sqr(const DwArch* a, int precision, const float* params, const void* prepared, const float* r,
@@ -643,8 +686,9 @@ static int mcmc_impl(const DwArch* a, int precision, const float* params, const 
                      void* ws, size_t wsb, cudaStream_t s) {
     return with_act(precision, true, [&](auto tag) {
         using Act = act_of<decltype(tag)>;
-        if (wsb < ws_bytes_t<Act>(a, B, 2)) return (int)DW_ERR_WORKSPACE;
-        size_t fwd = plan_bytes_any<Act>(a, B, false);
+        const size_t full = plan_bytes_any<Act>(a, precision, B, false), least = plan_bytes_any<Act>(a, precision, B, false, true);
+        const size_t fwd = region_of(full, least, ws_bytes_t<Act>(a, precision, B, 2) - full, wsb);
+        if (fwd == 0) return (int)DW_ERR_WORKSPACE;
         Carver c(static_cast<char*>(ws) + fwd, wsb - fwd);
         float* r_prop = c.take<float>((size_t)B * a->n_el * 3);
         float* lp_prop = c.take<float>((size_t)B);

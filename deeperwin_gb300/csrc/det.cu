@@ -1575,9 +1575,9 @@ __global__ void k_combine(const double* __restrict__ logdet, const double* __res
                           const double* __restrict__ jas, const float* __restrict__ r, const float* __restrict__ R,
                           const int32_t* __restrict__ Z, Dims d, int B, float* __restrict__ log_psi_sqr,
                           float* __restrict__ phase, float* __restrict__ E_loc, float* __restrict__ grad_out,
-                          int coul64, const int* __restrict__ nvalid, float* __restrict__ esc) {
+                          int coul64, const int* __restrict__ nvalid, int first, float* __restrict__ esc) {
     int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-    if (warp >= B || (nvalid && warp >= *nvalid)) return;
+    if (warp >= B || (nvalid && first + warp >= *nvalid)) return;
     const int b = warp, K = d.K, n3 = 3 * d.n;
     const double* ld = logdet + (int64_t)b * K;
     const double* sg = sign + (int64_t)b * K;
@@ -1654,9 +1654,9 @@ __global__ void k_combine(const double* __restrict__ logdet, const double* __res
 void launch_combine(const double* logdet, const double* sign, const double* g, const double* lapdet, const double* jas,
                     const float* r, const float* R, const int32_t* Z, const Dims& d, int B,
                     float* log_psi_sqr, float* phase, float* E_loc, float* grad_out, cudaStream_t s, int coul64,
-                    const int* nvalid, float* esc) {
+                    const int* nvalid, float* esc, int first) {
     k_combine<<<(B * 32 + 255) / 256, 256, 0, s>>>(logdet, sign, g, lapdet, jas, r, R, Z, d, B, log_psi_sqr, phase,
-                                                   E_loc, grad_out, coul64, nvalid, esc);
+                                                   E_loc, grad_out, coul64, nvalid, first, esc);
     count_launch();
 }
 

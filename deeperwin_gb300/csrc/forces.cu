@@ -120,8 +120,10 @@ int dw_forces(const DwArch* a, int precision, const float* params, const void* p
     if (antithetic && (!params || !prepared)) return DW_ERR_ARG;
     cudaStream_t s = (cudaStream_t)stream;
     const int n = a->n_el, N = a->n_ions;
-    const size_t fwd = dw_workspace_bytes(a, precision, B, 0);
+    size_t fwd = dw_workspace_bytes(a, precision, B, 0);
     if (fwd == 0) return DW_ERR_ARG;
+    const size_t need = dw_forces_workspace_bytes(a, precision, B), rest = need - fwd;
+    if (wsb < need) fwd = std::max(workspace_least_bytes(a, precision, B, 0), wsb > rest ? (wsb - rest) / 256 * 256 : 0);
     Carver c(static_cast<char*>(ws) + fwd, wsb > fwd ? wsb - fwd : 0);
     float* rm = c.take<float>((size_t)B * n * 3);
     float* lpm = c.take<float>((size_t)B);

@@ -26,9 +26,10 @@ struct Run64 {
     int C;          // channels per electron
     int B;          // walkers in the chunk
     const int* nvalid;
+    int first = 0;  // the chunk's first walker in that count
 };
 __device__ __forceinline__ int valid_walkers(const Run64& q) {
-    return q.nvalid ? min(q.B, max(0, *q.nvalid)) : q.B;
+    return q.nvalid ? min(q.B, max(0, *q.nvalid - q.first)) : q.B;
 }
 __device__ __forceinline__ double softplus_d(double x) { return fmax(x, 0.0) + log1p(exp(-fabs(x))); }
 
@@ -489,7 +490,7 @@ static int launch_tangents64(const double* MO, const double* Ainv, const double*
                              double* lapdet, void* scratch, size_t scratch_bytes, cudaStream_t s) {
     const int n = q.d.n;
     int status = DW_OK;
-    if (dets64_tangents(MO, Ainv, sign, n, q.C, q.d.K, nmat, q.nvalid, g, lapdet, scratch, scratch_bytes, s, &status)) return status;
+    if (dets64_tangents(MO, Ainv, sign, n, q.C, q.d.K, nmat, q.nvalid, q.first, g, lapdet, scratch, scratch_bytes, s, &status)) return status;
     const size_t sm = (size_t)3 * n * n * sizeof(double);
     if (sm > 48 * 1024) allow_smem(k64_det_tangents, 3 * kMaxEl * kMaxEl * (int)sizeof(double));
     k64_det_tangents<<<nmat, 128, sm, s>>>(MO, Ainv, sign, q, g, lapdet);
@@ -528,7 +529,7 @@ struct Plan64 {
 };
 static const int kXW64 = 320;    // layer 1..3 input [h (256) | conv_ee (32) | conv_ei (32)]
 
-// Buffers of a chunk of Bc walkers; without `digits` only those that the chunk size is chosen by.
+// Buffers of a chunk of Bc walkers, with the digit planes and the tangents' scratch or without.
 static Plan64 carve64(const Dims& d, int C, int Bc, void* ws, bool digits = true) {
     Carver c(ws, (size_t)-1);
     Plan64 p;
@@ -560,32 +561,41 @@ static Plan64 carve64(const Dims& d, int C, int Bc, void* ws, bool digits = true
     p.jas = c.take<double>((int64_t)Bc * C);
     p.scratch = nullptr;
     p.scratch_bytes = 0;
-    if (digits) {
-        if (C > 1) {
-            p.scratch_bytes = dets64_scratch_bytes(d.n, C, (int64_t)Bc * d.K);
-            p.scratch = c.take<unsigned char>(p.scratch_bytes);
-        }
-        auto take = [&](int64_t r, int K) {
-            const int Kp = pad_k64(K);
-            __nv_bfloat16* dig = c.take<__nv_bfloat16>((size_t)planes64(false) * r * Kp);
-            return Digits{dig, c.take<int>(r), r, Kp, planes64(false)};
-        };
-        p.act = take(rows, std::max(kXW64, w0));
-        p.mean = take((int64_t)Bc * C, 2 * std::max(d.D, d.hw[0]));
-        const int J[2] = {d.J0, d.J1}, JK[2] = {d.D, d.J0};
-        for (int k = 0; k < kMaxW64; ++k) {
-            const int l = k % 4;
-            const int K = k < 4 ? d.hw[l] : k < 8 ? 2 * d.hw[l] : k < 12 ? d.hw[l] + d.E + d.eiw[l] : k < 14 ? d.D : JK[k - 14];
-            const int N = k < 4 ? d.E : k < 12 ? d.D : k < 14 ? d.KN : J[k - 14];
-            p.w[k] = Weight64{nullptr, N, K, N, take(N, K)};
-        }
+    if (digits && C > 1) {
+        p.scratch_bytes = dets64_scratch_bytes(d.n, C, (int64_t)Bc * d.K);
+        p.scratch = c.take<unsigned char>(p.scratch_bytes);
+    }
+    auto take = [&](int64_t r, int K) {
+        const int Kp = pad_k64(K);
+        if (!digits) return Digits{nullptr, nullptr, r, Kp, 0};
+        __nv_bfloat16* dig = c.take<__nv_bfloat16>((size_t)planes64(false) * r * Kp);
+        return Digits{dig, c.take<int>(r), r, Kp, planes64(false)};
+    };
+    p.act = take(rows, std::max(kXW64, w0));
+    p.mean = take((int64_t)Bc * C, 2 * std::max(d.D, d.hw[0]));
+    const int J[2] = {d.J0, d.J1}, JK[2] = {d.D, d.J0};
+    for (int k = 0; k < kMaxW64; ++k) {
+        const int l = k % 4;
+        const int K = k < 4 ? d.hw[l] : k < 8 ? 2 * d.hw[l] : k < 12 ? d.hw[l] + d.E + d.eiw[l] : k < 14 ? d.D : JK[k - 14];
+        const int N = k < 4 ? d.E : k < 12 ? d.D : k < 14 ? d.KN : J[k - 14];
+        p.w[k] = Weight64{nullptr, N, K, N, take(N, K)};
     }
     p.bytes = c.used;
     return p;
 }
 
-static const size_t kChunkBudget64 = (size_t)6 << 30;    // without the digit planes (about half as much again)
+static const size_t kChunkBudget64 = (size_t)6 << 30;
 
+// Walkers of a chunk with the digit planes: the most whose buffers take `budget` bytes (0: not one).
+static int choose_chunk64_digits(const Dims& d, int C, int B, size_t budget) {
+    int lo = 0;
+    for (int hi = std::min(B, 32768); lo < hi;) {
+        const int mid = lo + (hi - lo + 1) / 2;
+        if (carve64(d, C, mid, nullptr).bytes <= budget) lo = mid; else hi = mid - 1;
+    }
+    return lo;
+}
+// Walkers of a chunk without them.
 static int choose_chunk64(const Dims& d, int C, int B, size_t budget) {
     const size_t one = carve64(d, C, 1, nullptr, false).bytes, two = carve64(d, C, 2, nullptr, false).bytes;
     const size_t per = std::max<size_t>(two > one ? two - one : one, 1);
@@ -600,21 +610,30 @@ static inline unsigned blocks_for(int64_t n, int tpb) { return (unsigned)((n + t
 
 // The FP64 forward (value or tangent) of one chunk of walkers.
 static int run_chunk64(const Plan64& p, const Dims& d0, int Bc, const float* P, const ParamLayout& L, const float* r,
-                       const float* R, const int32_t* Z, const int32_t* seg, const int* nvalid, float* lp, float* phase,
-                       float* E, float* grad, cudaStream_t s) {
+                       const float* R, const int32_t* Z, const int32_t* seg, const int* nvalid, int first, float* lp,
+                       float* phase, float* E, float* grad, cudaStream_t s) {
     Dims d = d0;
     d.seg = seg;
     Run64 q;
-    q.d = d; q.C = p.C; q.B = Bc; q.nvalid = nvalid;
+    q.d = d; q.C = p.C; q.B = Bc; q.nvalid = nvalid; q.first = first;
     const int C = p.C, n = d.n;
+    const bool digits = p.act.dig != nullptr;
     const int64_t rows = (int64_t)Bc * n * C;
     const bool tang = C > 1;
     const int w0 = d.hw[0] + d.E + d.eiw[0];
-    const Rows64 all = plain_rows(Bc, n * C, nvalid), chan = plain_rows(Bc, C, nvalid);
+    Rows64 all = plain_rows(Bc, n * C, nvalid), chan = plain_rows(Bc, C, nvalid);
+    all.first = chan.first = first;
     // digit planes of the first K columns, reusing the plan's buffer at that width
     auto planes = [](Digits x, int K) { x.Kp = pad_k64(K); return x; };
+    auto slice = [&](const double* A, int lda, int K, const Rows64& rr) {
+        const Digits x = planes(p.act, K);
+        if (digits) slice_rows64(A, lda, K, rr, x, s);
+        return x;
+    };
     auto gemm = [&](const double* A, int lda, const Digits& da, const Weight64& w, double* Cm, int ldc, const Rows64& rr,
-                    const Epi64& e) { return gemm64_tc(A, lda, da, w, Cm, ldc, rr, C, e, s); };
+                    const Epi64& e) {
+        return digits ? gemm64_tc(A, lda, da, w, Cm, ldc, rr, C, e, s) : gemm64_pipe(A, lda, w, Cm, ldc, rr, C, e, s);
+    };
     // layer-0 input [features | conv_ee | conv_ei] in XB (free until layer 1 writes it)
     timer_begin("fp64_streams", s);
     k64_features<<<blocks_for(rows * d.N, 256), 256, 0, s>>>(r, R, Z, q, p.XB, w0);
@@ -631,8 +650,7 @@ static int run_chunk64(const Plan64& p, const Dims& d0, int Bc, const float* P, 
         const int hw = d.hw[l];
         // h_map = tanh(h W + b) -> HM
         Epi64 em; em.bias = P + L.h_map_b[l];
-        const Digits dh = planes(p.act, hw);
-        slice_rows64(xin, ldin, hw, all, dh, s);
+        const Digits dh = slice(xin, ldin, hw, all);
         DW_CHECK(gemm(xin, ldin, dh, p.w[l], p.Zt, d.E, all, em));
         jet_tanh(p.Zt, d.E, d.E, q, p.HM, 32, s);
         // convolutions into columns [hw, hw + E + eiw)
@@ -649,8 +667,7 @@ static int run_chunk64(const Plan64& p, const Dims& d0, int Bc, const float* P, 
         DW_CHECK(gemm(p.M, 2 * hw, dm, p.w[4 + l], p.WB, d.D, chan, eb));
         // h_el = tanh([h | conv_ee | conv_ei] W_main + mean term) (ferminet_embedding.py:233-241)
         Epi64 e3; e3.rowbias = p.WB; e3.ldrb = d.D;
-        const Digits dx = planes(p.act, p.w[8 + l].K);
-        slice_rows64(xin, ldin, p.w[8 + l].K, all, dx, s);
+        const Digits dx = slice(xin, ldin, p.w[8 + l].K, all);
         DW_CHECK(gemm(xin, ldin, dx, p.w[8 + l], p.Zt, d.D, all, e3));
         jet_tanh(p.Zt, d.D, d.D, q, xout, kXW64, s);
         xin = xout;
@@ -663,8 +680,7 @@ static int run_chunk64(const Plan64& p, const Dims& d0, int Bc, const float* P, 
     spins.ngroups = 2;
     spins.g[0] = RowGroup{0, d.nu * C, (int64_t)n * C, 0};
     spins.g[1] = RowGroup{(int64_t)Bc * d.nu * C, d.nd * C, (int64_t)n * C, (int64_t)d.nu * C};
-    const Digits dH = planes(p.act, d.D);
-    slice_rows64(H, kXW64, d.D, spins, dH, s);
+    const Digits dH = slice(H, kXW64, d.D, spins);
     for (int spin = 0; spin < 2; ++spin) {
         Rows64 one = spins;
         one.ngroups = 1;
@@ -692,8 +708,7 @@ static int run_chunk64(const Plan64& p, const Dims& d0, int Bc, const float* P, 
     DW_CHECK(gemm(H, kXW64, dH, p.w[14], p.Zt, d.J0, spins, j0));
     jet_tanh(p.Zt, d.J0, d.J0, q, p.J1, d.J0, s);
     Epi64 j1; j1.bias = P + L.jas_b[1];
-    const Digits dj = planes(p.act, d.J0);
-    slice_rows64(p.J1, d.J0, d.J0, all, dj, s);
+    const Digits dj = slice(p.J1, d.J0, d.J0, all);
     DW_CHECK(gemm(p.J1, d.J0, dj, p.w[15], p.Zt, d.J1, all, j1));
     jet_tanh(p.Zt, d.J1, d.J1, q, p.J2, d.J1, s);
     k64_jastrow_out<<<blocks_for((int64_t)Bc * C * 32, 256), 256, 0, s>>>(p.J2, d.J1, P + L.jas_w[2], q, p.jas);
@@ -701,7 +716,7 @@ static int run_chunk64(const Plan64& p, const Dims& d0, int Bc, const float* P, 
     // log-sum-exp over determinants, derivatives of log psi^2, kinetic + FP64 Coulomb energy
     Dims dc = d;
     dc.Tp = C;
-    launch_combine(p.logdet, p.sign, p.g, p.lapdet, p.jas, r, R, Z, dc, Bc, lp, phase, E, grad, s, 1, nvalid);
+    launch_combine(p.logdet, p.sign, p.g, p.lapdet, p.jas, r, R, Z, dc, Bc, lp, phase, E, grad, s, 1, nvalid, nullptr, first);
     DW_CHECK_CUDA(launch_error());
     return DW_OK;
 }
@@ -739,10 +754,16 @@ int fp64_max_chunk(const DwArch* a, bool tang) {
     return choose_chunk64(d, C, 1 << 30, kChunkBudget64);
 }
 
+size_t fp64_least_bytes(const DwArch* a, int B, bool tang) {
+    Dims d = make_dims(a, tang);
+    const int C = tang ? 3 * d.n + 2 : 1;
+    return (carve64(d, C, choose_chunk64(d, C, std::max(B, 1), kChunkBudget64), nullptr, false).bytes + 4096 + 255) / 256 * 256;
+}
 size_t fp64_plan_bytes(const DwArch* a, int B, bool tang) {
     Dims d = make_dims(a, tang);
     const int C = tang ? 3 * d.n + 2 : 1;
-    return (carve64(d, C, choose_chunk64(d, C, std::max(B, 1), kChunkBudget64), nullptr).bytes + 4096 + 255) / 256 * 256;
+    const int bc = std::max(1, choose_chunk64_digits(d, C, std::max(B, 1), kChunkBudget64));
+    return std::max((carve64(d, C, bc, nullptr).bytes + 4096 + 255) / 256 * 256, fp64_least_bytes(a, B, tang));
 }
 
 int fp64_forward_all(const DwArch* a, const float* P, const void* prepared, const float* r, int B, const float* R,
@@ -758,10 +779,16 @@ int fp64_forward_all(const DwArch* a, const float* P, const void* prepared, cons
     const float* main_w[4];
     const float* mean_w[4];
     prepared_fp32_layers(a, prepared, main_w, mean_w);
-    const int bc = choose_chunk64(d, C, B, kChunkBudget64);
-    if (nvalid && bc < B) return DW_ERR_ARG;       // a device-side walker count needs one chunk
-    Plan64 p = carve64(d, C, bc, ws);
-    if (p.bytes > ws_bytes) return DW_ERR_WORKSPACE;
+    // With the digit planes in the largest chunk that the region holds (its base rounded up to 256 bytes: the
+    // planes are read by TMA), or, in a region sized without them that holds not one walker's, without.
+    int bc = choose_chunk64(d, C, B, kChunkBudget64);
+    if (carve64(d, C, bc, nullptr, false).bytes > ws_bytes) return DW_ERR_WORKSPACE;
+    char* base = reinterpret_cast<char*>(((uintptr_t)ws + 255) / 256 * 256);
+    const size_t lost = (size_t)(base - static_cast<char*>(ws)), room = ws_bytes > lost ? ws_bytes - lost : 0;
+    const size_t one = carve64(d, C, 1, nullptr).bytes;      // one walker may take more than the budget
+    const int bd = one > room ? 0 : std::max(1, choose_chunk64_digits(d, C, B, std::min(room, kChunkBudget64)));
+    if (bd > 0) bc = bd;
+    Plan64 p = bd > 0 ? carve64(d, C, bc, base) : carve64(d, C, bc, ws, false);
     for (int l = 0; l < 4; ++l) {
         p.w[l].w = P + L.h_map_w[l];
         p.w[4 + l].w = mean_w[l];
@@ -771,14 +798,14 @@ int fp64_forward_all(const DwArch* a, const float* P, const void* prepared, cons
     p.w[13].w = P + L.bf_dn;
     p.w[14].w = P + L.jas_w[0];
     p.w[15].w = P + L.jas_w[1];
-    slice_weights64(p.w, kMaxW64, nvalid, s);
+    if (p.act.dig) slice_weights64(p.w, kMaxW64, nvalid, s);
     const int total = nseg * 4 * d.N * 32;
     k64_ion_maps<<<(total + 255) / 256, 256, 0, s>>>(P, L, d, Z, p.him);
     count_launch();
     for (int b0 = 0; b0 < B; b0 += bc) {
         const int nb = std::min(bc, B - b0);
         DW_CHECK(run_chunk64(p, d, nb, P, L, r + (int64_t)b0 * d.n * 3, R, Z, seg ? seg + b0 : nullptr,
-                             nvalid, lp + b0, phase ? phase + b0 : nullptr, E ? E + b0 : nullptr,
+                             nvalid, b0, lp + b0, phase ? phase + b0 : nullptr, E ? E + b0 : nullptr,
                              grad ? grad + (int64_t)b0 * 3 * d.n : nullptr, s));
     }
     return DW_OK;

@@ -25,8 +25,8 @@
 // Why: FP64 issues at about two lanes per clock and SM here (1.2 TFLOP/s), the BF16 tensor cores at
 // about 1500 times that, so even 45 products per multiplication are far cheaper: the 16 GEMMs of a
 // C2H4-shaped local energy (16 electrons, 32 determinants, 64 walkers) took 46.0 ms on the FP64 pipe
-// (64 x 64 tiles, 0.97 TFLOP/s) and take 4.6 ms here; a single tile of the FP64 loop took longer than
-// the smallest launch of this kernel, so no size keeps it.
+// (64 x 64 tiles, 0.97 TFLOP/s) and take 4.7 ms here; a single tile of the FP64 loop takes longer than
+// the smallest launch of this kernel, so no size keeps it. It serves workspaces without room for the planes.
 //
 // Rows and columns whose scale is not an ordinary one (infinities, NaN, below 2^-922) are computed
 // from the original FP64 values in the epilogue.
@@ -229,6 +229,7 @@ k64_spin_means(const double* __restrict__ X, int ldx, int hw, int n, int nu, int
         }
         x[u] = make_double2(v[0], v[1]);
     }
+    if (!d.dig) return;
     const int E = scan.merge_warp();
     slice_row(x, E, [&](int, int) { return scan.emax; }, bt, d);
 }
@@ -529,6 +530,72 @@ k64_gemm_tc(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
     if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem) : "memory");
 }
 
+// The same product on the FP64 pipe: 64 x 64 tiles, 16-deep K slices, 256 threads with a 4 x 4 patch each
+// (rows tr + 16 i, columns tc + 16 j: a warp's shared reads of W are 16 consecutive doubles, those of A two
+// broadcasts). Bound by the pipe, two lanes per clock and SM. blockIdx.z: row group.
+__global__ void __launch_bounds__(256) k64_gemm_pipe(Args64 a) {
+    constexpr int PM = 64, PN = 64, PK = 16;
+    const RowGroup& g = a.rows.g[blockIdx.z];
+    const int64_t total = (int64_t)valid_of(a.rows) * g.rpw, m0 = (int64_t)blockIdx.y * PM;
+    if (m0 >= total) return;
+    __shared__ double As[PK][PM + 1];
+    __shared__ double Ws[PK][PN];
+    __shared__ int64_t row_of[PM];
+    const int tid = threadIdx.x, tr = tid / 16, tc = tid % 16, n0 = blockIdx.x * PN;
+    if (tid < PM) {
+        const int64_t k = m0 + tid, b = k / g.rpw;
+        row_of[tid] = k < total ? b * g.out_rpw + g.out_off + k % g.rpw : -1;
+    }
+    __syncthreads();
+    double acc[4][4];
+    #pragma unroll
+    for (int i = 0; i < 4; ++i)
+        #pragma unroll
+        for (int j = 0; j < 4; ++j) acc[i][j] = 0.0;
+    for (int k0 = 0; k0 < a.K; k0 += PK) {
+        #pragma unroll
+        for (int u = 0; u < PM * PK / 256; ++u) {
+            const int e = tid + u * 256, r = e / PK, k = e % PK;
+            As[k][r] = row_of[r] >= 0 && k0 + k < a.K ? a.A[row_of[r] * a.lda + k0 + k] : 0.0;
+        }
+        #pragma unroll
+        for (int u = 0; u < PK * PN / 256; ++u) {
+            const int e = tid + u * 256, k = e / PN, c = e % PN;
+            Ws[k][c] = k0 + k < a.K && n0 + c < a.N ? (double)a.W[(int64_t)(k0 + k) * a.ldw + n0 + c] : 0.0;
+        }
+        __syncthreads();
+        #pragma unroll
+        for (int k = 0; k < PK; ++k) {
+            double x[4], w[4];
+            #pragma unroll
+            for (int i = 0; i < 4; ++i) x[i] = As[k][tr + 16 * i];
+            #pragma unroll
+            for (int j = 0; j < 4; ++j) w[j] = Ws[k][tc + 16 * j];
+            #pragma unroll
+            for (int i = 0; i < 4; ++i)
+                #pragma unroll
+                for (int j = 0; j < 4; ++j) acc[i][j] = fma(x[i], w[j], acc[i][j]);
+        }
+        __syncthreads();
+    }
+    #pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int64_t row = row_of[tr + 16 * i];
+        if (row < 0) continue;
+        const int t = (int)(row % a.channels);
+        const double* rb = a.e.rowbias ? a.e.rowbias + ((m0 + tr + 16 * i) / g.rpw * a.channels + t) * a.e.ldrb : nullptr;
+        #pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const int n = n0 + tc + 16 * j;
+            if (n >= a.N) continue;
+            double v = acc[i][j];
+            if (a.e.bias && t == 0) v += (double)a.e.bias[n];
+            if (rb) v += rb[n];
+            a.C[row * a.ldc + n] = v;
+        }
+    }
+}
+
 // Traces of E = dA_t A^-1 (cyclic: those of A^-1 dA_t), block per (matrix, channel): tr E to g (tr1 for the
 // Laplacian channel), tr E^2 to tr2.
 __global__ void __launch_bounds__(128)
@@ -629,6 +696,24 @@ int gemm64_tc(const double* A, int lda, const Digits& da, const Weight64& w, dou
     return DW_OK;
 }
 
+int gemm64_pipe(const double* A, int lda, const Weight64& w, double* C, int ldc, const Rows64& rows, int channels,
+                const Epi64& e, cudaStream_t s) {
+    Args64 a;
+    a.A = A; a.lda = lda; a.W = w.w; a.ldw = w.ldw; a.C = C; a.ldc = ldc;
+    a.ea = nullptr; a.ew = nullptr;
+    a.rows = rows; a.e = e;
+    a.N = w.N; a.K = w.K; a.channels = channels; a.ntn = 0;
+    a.W64 = nullptr; a.per = 0; a.error = nullptr;
+    int64_t most = 0;
+    for (int g = 0; g < rows.ngroups; ++g) most = std::max(most, (int64_t)rows.B * rows.g[g].rpw);
+    timer_begin("fp64_gemm", s);
+    k64_gemm_pipe<<<dim3((w.N + 63) / 64, (unsigned)((most + 63) / 64), rows.ngroups), 256, 0, s>>>(a);
+    timer_end("fp64_gemm", s, 0.0, 0.0);
+    count_launch();
+    DW_CHECK_CUDA(launch_error());
+    return DW_OK;
+}
+
 // Scratch of dets64_tangents for `m` matrices at a time.
 struct DetScratch {
     Digits a, w;
@@ -668,7 +753,7 @@ size_t dets64_scratch_bytes(int n, int T, int64_t nmat) {
 }
 
 bool dets64_tangents(const double* MO64, const double* Ainv64, const double* sign, int n, int T, int K, int nmat,
-                     const int* nvalid, double* g, double* lapdet, void* scratch, size_t scratch_bytes, cudaStream_t s,
+                     const int* nvalid, int first, double* g, double* lapdet, void* scratch, size_t scratch_bytes, cudaStream_t s,
                      int* status) {
     *status = DW_OK;
     if (!dets64_fits(n) || T < 2 || !scratch) return false;
@@ -684,7 +769,7 @@ bool dets64_tangents(const double* MO64, const double* Ainv64, const double* sig
     const DetScratch d = carve_dets(n, T, m, base);
     auto run = [&](int m0, int nm) -> int {
         Rows64 rows;                                 // the matrices' derivative channels: rows of n
-        rows.ngroups = 1; rows.B = nm; rows.nvalid = nvalid; rows.mul = K; rows.first = m0;
+        rows.ngroups = 1; rows.B = nm; rows.nvalid = nvalid; rows.mul = K; rows.first = first * K + m0;
         rows.g[0] = rows.g[1] = RowGroup{0, per, (int64_t)T * n, n};
         Rows64 cols = rows;                          // the inverses' columns
         cols.g[0] = cols.g[1] = RowGroup{0, n, (int64_t)n * n, 0};

@@ -48,7 +48,8 @@ inline Rows64 plain_rows(int B, int rpw, const int* nvalid) {
 
 // Digit planes of the rows of A [.., K] (row stride lda); skips walkers beyond nvalid.
 void slice_rows64(const double* A, int lda, int K, const Rows64& rows, const Digits& d, cudaStream_t s);
-// Spin means M [(b, t)][2 hw] of X's first hw columns over the nu up and n - nu down electrons, and their digit planes.
+// Spin means M [(b, t)][2 hw] of X's first hw columns over the nu up and n - nu down electrons, and their digit planes
+// (none if d.dig is null).
 void spin_means64(const double* X, int ldx, int hw, int n, int nu, int C, const Rows64& rows, double* M, const Digits& d,
                   cudaStream_t s);
 // Digit planes of `count` weight matrices in one launch (nothing when *nvalid == 0).
@@ -64,14 +65,18 @@ struct Epi64 {
 };
 // FP64 determinant tangents of nmat matrices with T - 1 derivative channels (MO64 [mat][T][n][n], Ainv64
 // [mat][n][n], sign): g[mat][3 n] = tr(A^-1 dA_t), lapdet[mat] = tr(A^-1 Lap A) - sum_t tr((A^-1 dA_t)^2), as
-// digit products. K determinants per walker (nvalid counts walkers). Returns false, having done nothing,
+// digit products. K determinants per walker (nvalid counts walkers, these start at `first`). Returns false, having done nothing,
 // where the FP64 loop is as fast (n < 24), for n > 48, or with scratch for less than 32 matrices at a time.
 size_t dets64_scratch_bytes(int n, int T, int64_t nmat);
 bool dets64_tangents(const double* MO64, const double* Ainv64, const double* sign, int n, int T, int K, int nmat,
-                     const int* nvalid, double* g, double* lapdet, void* scratch, size_t scratch_bytes, cudaStream_t s,
+                     const int* nvalid, int first, double* g, double* lapdet, void* scratch, size_t scratch_bytes, cudaStream_t s,
                      int* status);
 
+// The product by digits (A's planes da, w.d).
 int gemm64_tc(const double* A, int lda, const Digits& da, const Weight64& w, double* C, int ldc, const Rows64& rows,
               int channels, const Epi64& e, cudaStream_t s);
+// The product on the FP64 pipe, for workspaces without room for the planes.
+int gemm64_pipe(const double* A, int lda, const Weight64& w, double* C, int ldc, const Rows64& rows, int channels,
+                const Epi64& e, cudaStream_t s);
 
 }  // namespace dw

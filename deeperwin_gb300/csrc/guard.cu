@@ -163,7 +163,7 @@ int guard_capacity(const DwArch* a, int B) {
     return std::min(B, std::max(16, (B + 31) / 32));
 }
 
-// second tier: up to 1 / 128 of the batch (at least 8) in one FP64 chunk; its kernels skip the
+// second tier: up to 1 / 128 of the batch (at least 8), at most an FP64 chunk; its kernels skip the
 // unused capacity through the device-side count, so it costs FP64 work only for the walkers
 // flagged (0.14 ms per C2H4-shaped walker)
 static int guard64_capacity(const DwArch* a, int B) {
@@ -181,7 +181,8 @@ struct GuardPlan {
     size_t bytes;
 };
 
-static GuardPlan carve_guard(const DwArch* a, int B, void* ws) {
+// Least: the region sized for forwards without digit products (what the re-evaluation then runs as).
+static GuardPlan carve_guard(const DwArch* a, int B, void* ws, bool least) {
     GuardPlan g;
     const int n3 = 3 * a->n_el;
     Carver c(ws, (size_t)-1);
@@ -196,21 +197,25 @@ static GuardPlan carve_guard(const DwArch* a, int B, void* ws) {
         t.lp_sub = c.take<float>((size_t)t.cap);
         t.g_sub = c.take<float>((size_t)t.cap * n3);
     }
-    g.region_bytes = std::max({det64_plan_bytes(a, DW_PRECISION_FP32_DET64, g.t[0].cap),
-                               det64_plan_bytes(a, DW_PRECISION_MIXED_DET64, g.t[0].cap),
-                               fp64_plan_bytes(a, g.t[1].cap, true)});
+    auto det64 = [&](int form) { return least ? det64_least_bytes(a, form, g.t[0].cap) : det64_plan_bytes(a, form, g.t[0].cap); };
+    g.region_bytes = std::max({det64(DW_PRECISION_FP32_DET64), det64(DW_PRECISION_MIXED_DET64),
+                               least ? fp64_least_bytes(a, g.t[1].cap, true) : fp64_plan_bytes(a, g.t[1].cap, true)});
     g.region = c.take<unsigned char>(g.region_bytes);
     g.bytes = c.used + 256;
     return g;
 }
 
-size_t guard_bytes(const DwArch* a, int B) { return carve_guard(a, B, nullptr).bytes; }
+size_t guard_bytes(const DwArch* a, int B, bool least) { return carve_guard(a, B, nullptr, least).bytes; }
 
 int tail_guard(const DwArch* a, const float* P, const void* prepared, const float* r, int B, const float* R,
                const int32_t* Z, const int32_t* seg, int nseg, const float* esc, float* E, float* lp, float* grad,
                void* ws, size_t wsb, cudaStream_t s) {
-    GuardPlan g = carve_guard(a, B, ws);
-    if (g.bytes > wsb) return DW_ERR_WORKSPACE;
+    GuardPlan g = carve_guard(a, B, ws, false);
+    if (g.bytes > wsb) {
+        const size_t full = g.bytes;
+        if (guard_bytes(a, B, true) > wsb) return DW_ERR_WORKSPACE;
+        g.region_bytes -= (full - wsb + 255) / 256 * 256;
+    }
     const int n3 = 3 * a->n_el;
     for (int k = 0; k < 2; ++k) {
         const GuardTier& t = g.t[k];

@@ -120,7 +120,7 @@ void launch_det_tangents(const float* MO, const float* Ainv, const double* sign,
 void launch_combine(const double* logdet, const double* sign, const double* g, const double* lapdet, const double* jas,
                     const float* r, const float* R, const int32_t* Z, const Dims& d, int B,
                     float* log_psi_sqr, float* phase, float* E_loc, float* grad_out, cudaStream_t s,
-                    int coul64 = 0, const int* nvalid = nullptr, float* esc = nullptr);
+                    int coul64 = 0, const int* nvalid = nullptr, float* esc = nullptr, int first = 0);
 void launch_coulomb(const float* r, int B, int n, const float* R, const int32_t* Z, int N, float* E, cudaStream_t s);
 // FP64 Gauss-Jordan log|det| and inverse of the value-channel Slater matrices (any Dims mode).
 void launch_slogdet_inv(const float* MO, const Dims& d, int B, double* logdet, double* sign, float* Ainv, cudaStream_t s);
@@ -135,9 +135,11 @@ int value_forward(const DwArch* a, int precision, const float* params, const voi
 void prepared_fp32_layers(const DwArch* a, const void* prepared, const float* main[4], const float* mean[4]);
 
 // fp64.cu: FP64 form (DW_PRECISION_FP64). nvalid (device int, may be null): walkers at or beyond
-// *nvalid are skipped; it requires the walkers to fit one chunk.
+// *nvalid are skipped.
 size_t fp64_plan_bytes(const DwArch* a, int B, bool tang);
-int fp64_max_chunk(const DwArch* a, bool tang);     // walkers of one FP64 chunk
+// The least region that fp64_forward_all takes: no digit planes, the GEMMs run on the FP64 pipe.
+size_t fp64_least_bytes(const DwArch* a, int B, bool tang);
+int fp64_max_chunk(const DwArch* a, bool tang);     // walkers of one chunk without digit planes
 // FP64 LU, inverse and determinant tangents of float32 Slater channels (MO layout of the forward
 // plans, d.T channels); MO64 holds Bc K T n^2 doubles, Ainv64 Bc K n^2.
 // scratch (may be null): dets64_scratch_bytes for the digit products of the tangents.
@@ -153,6 +155,9 @@ inline bool det64_form(int precision) {
     return precision == DW_PRECISION_FP32_DET64 || precision == DW_PRECISION_MIXED_DET64;
 }
 size_t det64_plan_bytes(const DwArch* a, int precision, int B);
+size_t det64_least_bytes(const DwArch* a, int precision, int B);     // without the tangents' scratch
+// api.cu: least bytes that the entry points take for dw_workspace_bytes' arguments
+size_t workspace_least_bytes(const DwArch* a, int precision, int n_walkers, int mode);
 int det64_local_energy(const DwArch* a, int precision, const float* P, const void* prepared, const float* r, int B,
                        const float* R, const int32_t* Z, const int32_t* seg, int nseg, float* E, float* lp, float* grad,
                        void* ws, size_t wsb, cudaStream_t s);
@@ -160,7 +165,7 @@ int det64_local_energy(const DwArch* a, int precision, const float* P, const voi
 // guard.cu: FP64 re-evaluation of the mixed form's flagged walkers (esc: per-walker error scales
 // written by the combine kernel, 3 floats per walker)
 int guard_capacity(const DwArch* a, int B);
-size_t guard_bytes(const DwArch* a, int B);
+size_t guard_bytes(const DwArch* a, int B, bool least = false);    // least: without room for digit products
 int tail_guard(const DwArch* a, const float* P, const void* prepared, const float* r, int B, const float* R,
                const int32_t* Z, const int32_t* seg, int nseg, const float* esc, float* E, float* lp, float* grad,
                void* ws, size_t wsb, cudaStream_t s);
