@@ -669,6 +669,13 @@ void slice_weights64(const Weight64* w, int count, const int* nvalid, cudaStream
     count_launch();
 }
 
+// Multiply-adds (two operations each) of the rows' walkers, as the timers count them.
+static double flops_of(const Rows64& rows, const Weight64& w) {
+    double m = 0.0;
+    for (int g = 0; g < rows.ngroups; ++g) m += (double)rows.B * rows.g[g].rpw;
+    return 2.0 * m * w.N * w.K;
+}
+
 int gemm64_tc(const double* A, int lda, const Digits& da, const Weight64& w, double* C, int ldc, const Rows64& rows,
               int channels, const Epi64& e, cudaStream_t s) {
     if (w.K > kMaxK64 || da.Kp < w.K || w.d.Kp < w.K) return DW_ERR_ARG;
@@ -690,7 +697,7 @@ int gemm64_tc(const double* A, int lda, const Digits& da, const Weight64& w, dou
     DW_CHECK_CUDA(allow_smem(k64_gemm_tc<false>, smem64(kPl)));
     timer_begin("fp64_gemm", s);
     k64_gemm_tc<false><<<(unsigned)std::min<int64_t>(tiles, num_sms()), kThreads64, smem64(kPl), s>>>(ma, mb, a);
-    timer_end("fp64_gemm", s, 0.0, 0.0);
+    timer_end("fp64_gemm", s, flops_of(rows, w), 0.0);
     count_launch();
     DW_CHECK_CUDA(launch_error());
     return DW_OK;
@@ -708,7 +715,7 @@ int gemm64_pipe(const double* A, int lda, const Weight64& w, double* C, int ldc,
     for (int g = 0; g < rows.ngroups; ++g) most = std::max(most, (int64_t)rows.B * rows.g[g].rpw);
     timer_begin("fp64_gemm", s);
     k64_gemm_pipe<<<dim3((w.N + 63) / 64, (unsigned)((most + 63) / 64), rows.ngroups), 256, 0, s>>>(a);
-    timer_end("fp64_gemm", s, 0.0, 0.0);
+    timer_end("fp64_gemm", s, flops_of(rows, w), 0.0);
     count_launch();
     DW_CHECK_CUDA(launch_error());
     return DW_OK;
