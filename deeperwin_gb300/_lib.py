@@ -88,6 +88,13 @@ _SIGS = {
                                                   ctypes.c_size_t, _P]),
     "dw_debug_gemm_jet": (ctypes.c_int, [ctypes.c_int, _P, ctypes.c_int, _P, _P, _P, ctypes.c_int]
                           + [ctypes.c_int] * 7 + [_P, _P, _P]),
+    "dw_debug_gemm_jet_bf16": (ctypes.c_int, [ctypes.c_int, _P, ctypes.c_int, _P, _P, ctypes.c_int]
+                               + [ctypes.c_int] * 7 + [_P, _P, _P]),
+    "dw_debug_gemm_jet_env": (ctypes.c_int, [ctypes.c_int, _P, ctypes.c_int] + [_P] * 6 + [ctypes.c_int] + [_P] * 3
+                              + [ctypes.c_int] * 7 + [_P]),
+    "dw_debug_det_tangents": (ctypes.c_int, [_P, _P, _P, ctypes.c_int, ctypes.c_int, _P, _P, _P]),
+    "dw_debug_gemm_f32": (ctypes.c_int, [_P, ctypes.c_int, _P, ctypes.c_int, _P] + [ctypes.c_int] * 4
+                          + [_P, _P, ctypes.c_int, ctypes.c_int, _P]),
     "dw_debug_tc_error_flag": (ctypes.c_int, []),
     "dw_debug_set_gemm_bk": (ctypes.c_int, [ctypes.c_int]),
     "dw_debug_set_guard_form": (ctypes.c_int, [ctypes.c_int]),

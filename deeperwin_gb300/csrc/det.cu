@@ -1678,6 +1678,17 @@ int dw_debug_slogdet_small(const float* MO, int n, int T, int nmat, int scalar, 
     return DW_OK;
 }
 
+// Test hook: launch_det_tangents of nmat matrices MO [mat][3 n + 2][n][n] with inverses Ainv [mat][n][n].
+int dw_debug_det_tangents(const float* MO, const float* Ainv, const double* sign, int n, int nmat, double* g, double* lapdet,
+                          void* stream) {
+    if (!MO || !Ainv || !sign || !g || !lapdet || n < 2 || n > dw::kMaxEl || nmat < 1) return DW_ERR_ARG;
+    dw::Dims d = dw::Dims();
+    d.n = n; d.K = 1; d.T = d.Tp = 3 * n + 2; d.lap = d.T - 1;
+    dw::launch_det_tangents(MO, Ainv, sign, d, nmat, g, lapdet, (cudaStream_t)stream);
+    DW_CHECK_CUDA(dw::launch_error());
+    return DW_OK;
+}
+
 // Instrumentation: determinant-tangent kernels (0: the default choice; 1: the single-buffer tile
 // kernel for n <= 32 and the general kernel for n = 33..40, in place of the pipelined and the
 // 8 x 8 ones). Returns the previous choice.

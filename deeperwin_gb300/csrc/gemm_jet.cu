@@ -639,4 +639,30 @@ int dw_debug_gemm_jet(int out, const void* A, int lda, const void* W0, const voi
                     JetRows{nw, n, T, ns, i0}, NF, K, e, (cudaStream_t)stream);
 }
 
+// The same on BF16 rows (np = 1); out 0 (fp32) or 1 (bf16).
+int dw_debug_gemm_jet_bf16(int out, const void* A, int lda, const void* W, void* C, int ldc, int nw, int n, int T, int ns,
+                           int i0, int NF, int K, const float* bias, const float* rowbias, void* stream) {
+    using namespace dw;
+    if (!tc_available()) return DW_ERR_UNSUPPORTED;
+    GemmEpi e;
+    e.bias = bias; e.rowbias = rowbias; e.ldrb = 256; e.Tp = T;
+    return gemm_jet(1, out, A, lda, (const __nv_bfloat16*)W, nullptr, C, ldc, JetRows{nw, n, T, ns, i0}, NF, K, e,
+                    (cudaStream_t)stream);
+}
+
+// Test hook: gemm_jet_env, the backflow of electrons [i0, i0 + ns) of nw walkers of n electrons and N ions (geometry
+// seg[b] of nseg, seg may be null) times the envelope, into MO [walker][dets][3 n + 2][n][n].
+int dw_debug_gemm_jet_env(int np, const void* A, int lda, const void* W0, const void* W1, const float* r, const float* R,
+                          const int32_t* Z, const int32_t* seg, int nseg, const float* alpha, const float* weights, float* MO,
+                          int nw, int n, int N, int dets, int ns, int i0, int K, void* stream) {
+    using namespace dw;
+    if (!tc_available()) return DW_ERR_UNSUPPORTED;
+    if (n < 1 || n > kMaxEl || N < 1 || N > kMaxIons || dets < 1 || i0 < 0 || i0 + ns > n || nseg < 1) return DW_ERR_ARG;
+    EnvEpi env{r, R, Z, alpha, weights, MO, Dims()};
+    env.d.n = n; env.d.N = N; env.d.K = dets; env.d.KN = dets * n; env.d.T = env.d.Tp = 3 * n + 2;
+    env.d.seg = seg; env.d.nseg = nseg;
+    return gemm_jet_env(np, A, lda, (const __nv_bfloat16*)W0, (const __nv_bfloat16*)W1, JetRows{nw, n, env.d.T, ns, i0}, K, env,
+                        (cudaStream_t)stream);
+}
+
 }  // extern "C"

@@ -666,6 +666,17 @@ void wgrad_f32(const float* A, int lda, const float* G, int ldg, int rows, int K
 
 extern "C" {
 
+// Test hook: gemm_f32 with bias, row bias (one row per walker) and tanh.
+int dw_debug_gemm_f32(const float* A, int lda, const float* W, int ldw, float* C, int ldc, int M, int N, int K, const float* bias,
+                      const float* rowbias, int rows_per_walker, int act, void* stream) {
+    using namespace dw;
+    GemmEpi e;
+    e.bias = bias; e.rowbias = rowbias; e.ldrb = N; e.rows_per_walker = rows_per_walker; e.act = act;
+    gemm_f32(A, lda, W, ldw, C, ldc, M, N, K, e, 1, 0, 0, (cudaStream_t)stream);
+    DW_CHECK_CUDA(launch_error());
+    return DW_OK;
+}
+
 // Test hook: a launch that the runtime refuses (more shared memory than an SM has), then one more call as the entry
 // points make them; returns what an entry point would.
 int dw_debug_refused_launch(void* stream) {
