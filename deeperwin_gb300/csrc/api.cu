@@ -472,6 +472,7 @@ static int forward_all(const DwArch* a, int precision, const float* P, const voi
     make_layout(a, &L);
     Prepared pre = carve_prepared(a, precision, const_cast<void*>(prepared));
     if (least_plan_bytes<Act>(a, B, tang, budget) > ws_bytes) return DW_ERR_WORKSPACE;
+    if ((uintptr_t)ws & 15) return DW_ERR_WORKSPACE;       // 16-byte loads and stores, TMA
     int bc = choose_chunk<Act>(d, B, budget);
     while (bc > 1 && carve_plan<Act>(d, bc, nullptr).bytes > ws_bytes) bc -= std::max(1, bc / 32);
     Plan<Act> p = carve_plan<Act>(d, bc, ws);

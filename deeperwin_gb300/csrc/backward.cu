@@ -610,7 +610,7 @@ int backward_all(const DwArch* a, const float* P, const float* const main[4], co
     make_layout(a, &L);
     int bc = 0;
     size_t need = bwd_bytes(a, B, &bc);
-    if (need > wsb) return DW_ERR_WORKSPACE;
+    if (need > wsb || ((uintptr_t)ws & 15)) return DW_ERR_WORKSPACE;
     Bwd w = carve_bwd(d, bc, ws);
     const float* m4[4] = {main[0], main[1], main[2], main[3]};
     const float* n4[4] = {mean[0], mean[1], mean[2], mean[3]};

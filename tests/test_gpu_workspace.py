@@ -105,3 +105,26 @@ def test_mixed_form_with_re_evaluated_walkers(cuda, name, K, B):
         assert st == 0
         assert np.all(np.abs(lp2 - lp) <= DIGITS_RTOL * np.abs(lp))
         assert np.all(np.abs(E2 - E) <= DIGITS_RTOL * np.abs(E) + 1e-9 * S), np.abs(E2 - E).max()
+
+
+@pytest.mark.parametrize("prec", ["fp32", "mixed", "bf16", "fp32_det64", "mixed_det64"])
+def test_misaligned_workspace_is_refused(cuda, prec):
+    """Below 16 bytes (the FP64 form takes 8) nothing is launched on a workspace that vector stores would fault on."""
+    L = _lib.lib()
+    params, r, R, Z = _setup(A.lih(), 2, prec, 3)
+    for mode in (0, 1):
+        full = _sizes(params, 3, mode)[0]
+        for offset in (4, 8):
+            st, E, lp, _, launches = _call(params, r, R, Z, full, offset, mode)
+            assert st == 3 and launches == 0 and np.all(lp == -7.0)
+        assert _call(params, r, R, Z, full, 16, mode)[0] == 0
+    if prec in ("fp32", "mixed"):
+        nb = L.dw_workspace_bytes(ctypes.byref(params.c_arch), params.prec, 3, 3)
+        ws, grad = torch.empty(nb + 256, dtype=torch.uint8, device="cuda"), torch.zeros_like(params.flat)
+        base = (ws.data_ptr() + 255) // 256 * 256
+        for offset, status in ((4, 3), (8, 3), (16, 0)):
+            assert L.dw_log_psi_sqr_backward(ctypes.byref(params.c_arch), params.prec, api._ptr(params.flat),
+                                             api._ptr(params.prepared), api._ptr(r), 3, api._ptr(R), api._ptr(Z),
+                                             api._ptr(torch.ones(3, device="cuda")), api._ptr(grad),
+                                             ctypes.c_void_p(base + offset), nb, None) == status
+        torch.cuda.synchronize()
