@@ -316,7 +316,7 @@ void gemm_f32(const float* A, int lda, const float* W, int ldw, float* C, int ld
     // Tile by the grid: a few rows (a single walker's launches are load latency and one FMA chain); 64 x 64
     // (64 x 32 for N <= 32) where 128-row tiles give less than two blocks per SM (2,048 LiH walkers: the
     // layers' 8,192 x 256 are 128 blocks, the spin means' 2,048 x 256 only 32); larger tiles reuse more
-    // per shared load. Measured: log psi^2 of one LiH walker 579 -> 229 us; 2,048 walkers, per launch: spin
+    // per shared load. Measured: log psi^2 of one LiH walker 567 -> 192 us; 2,048 walkers, per launch: spin
     // means 62 -> 27 us, layers 45 -> 43 us, h_map 24 -> 16 us, Jastrow 62 -> 35 us.
     if (batch == 1 && M <= kTinyM && K <= kTinyK) {
         const size_t sm = (size_t)K * (32 + 8) * sizeof(float);

@@ -811,7 +811,7 @@ k_ei_streams(const float* __restrict__ r, const float* __restrict__ R, const int
 // (SymmetricFeatures, ferminet_embedding.py:60-72). Row width mw (>= 2hw, zero padded).
 // Thread per (walker, channel, V columns): the loads of V columns of all electrons are what bounds it, so
 // every walker's channels are spread over the grid (a block per walker left most SMs idle where a chunk
-// holds few walkers: 40 electrons, 36 walkers per chunk, 14.5 -> 1.9 ms per 512-walker local energy).
+// holds few walkers: 40 electrons, 36 walkers per chunk, 14.7 -> 2.0 ms per 512-walker local energy).
 template <class Act, int V> struct MeanIO;
 template <int V> struct MeanIO<Split, V> {
     __device__ static __forceinline__ void add(const Split* X, int64_t row, int ldx, int f, float (&v)[V]) {
@@ -1523,7 +1523,8 @@ void launch_conv(const float* r, const float* WPl, const float* HM, const float*
 // shared memory (negative: a padding ion of a packed geometry), rows of an ion side by side, so that
 // one 16-byte load serves an ion's four exponentials in flight. Same mathematics as k_envelope.
 // NI bounds the ions held in registers; with NI = 8 four blocks fit an SM, which doubles the loads
-// in flight of this memory-bound kernel. ENV_NUMBERS
+// in flight of this memory-bound kernel. Per forward: C2H4, 4,096 walkers 189 -> 141 us, H10, 8,192 walkers
+// 156 -> 94 us against a scalar shared load and a branch per exponential.
 constexpr int kEnvWG = 4;
 constexpr int kEnvMaxIons = 16;
 template <int NI>

@@ -99,7 +99,10 @@ int dw_prepare_params(const DwArch* arch, int precision, const float* params,
                       void* prepared, size_t prepared_bytes, void* stream);
 
 /* Workspace bytes for n_walkers walkers. mode: 0 = log psi^2 only, 1 = local energy,
- * 2 = MCMC steps, 3 = parameter gradient. */
+ * 2 = MCMC steps, 3 = parameter gradient. The workspace starts at a multiple of 16 bytes (8 for
+ * DW_PRECISION_FP64), else DW_ERR_WORKSPACE. Forms with FP64 network or determinant algebra also
+ * take less, down to what they need without the buffers of the tensor-core digit products: fewer
+ * walkers per chunk then, or the same sums on the FP64 pipe. */
 size_t dw_workspace_bytes(const DwArch* arch, int precision, int n_walkers, int mode);
 
 /* log psi^2 and phase for all walkers.
@@ -269,9 +272,8 @@ int dw_guard_tier_stats(int tier, int64_t* walkers, int64_t* flagged, int64_t* o
 int dw_guard_stats(int64_t* walkers, int64_t* flagged, int64_t* overflow, int reset);
 
 /* Instrumentation: determinant-tangent kernels. 0 = the default choice; 1 = the single-buffer
- * tile kernel instead of the pipelined one for n_el in {4, 8, 16} and the general kernel instead
- * of the tile kernel for n_el in 33..40. Returns the previous choice, or -DW_ERR_ARG. No
- * reference counterpart. */
+ * tile kernel for n_el <= 32 and the general kernel for n_el in 33..40, in place of the pipelined
+ * and the 8 x 8 ones. Returns the previous choice, or -DW_ERR_ARG. No reference counterpart. */
 int dw_debug_set_det_tangents_kernel(int which);
 
 /* Instrumentation: network of the tier-0 re-evaluation, DW_PRECISION_FP32_DET64 (default) or
