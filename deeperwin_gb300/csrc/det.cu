@@ -1493,8 +1493,9 @@ void launch_det_tangents(const float* MO, const float* Ainv, const double* sign,
         count_launch();
         return;
     }
-    size_t sm = 3 * (size_t)d.n * d.n * sizeof(float);
-    if (sm > 48 * 1024) allow_smem(k_det_tangents, (int)sm);
+    const size_t sm = 3 * (size_t)d.n * d.n * sizeof(float);
+    // 48 KB at n = 64, more than a launch may take by default beside the kernel's own shared memory
+    allow_smem(k_det_tangents, 3 * kMaxEl * kMaxEl * (int)sizeof(float));
     k_det_tangents<<<nmat, 128, sm, s>>>(MO, Ainv, sign, d.n, d.T, nmat, g, lapdet);
     count_launch();
 }
